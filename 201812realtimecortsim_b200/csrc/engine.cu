@@ -14,8 +14,8 @@
 //   spike ring    80 slots x N: ids u32, te f64 (one slot per step)
 //   events        per target neuron `cap` slots of {u32 key, f32 weight};
 //                 overflow list of {target, key, weight}
-//   bath          per rank: 64-entry ran3 history, draw ring of LUT index
-//                 (u8) and lapse (f32); per step per-neuron event lists
+//   bath          per rank: the last 256 ran3 draws; per step per-neuron
+//                 event lists
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -100,7 +100,6 @@ struct NetConst {
   float stdp_drift, stdp_tauDecay;
   uint32_t ev_cap, ovf_cap;
   uint32_t light_max;   // neurons with more synaptic events take the heavy path
-  uint32_t bath_need;  // largest maxExternCurrentCount
   uint32_t delay_exp;  // getRandomDelay_EXP instead of _UNI
   float inv_log_tn;    // (float)(1.0 / log(0.05)), the EXP tail constant
 };
@@ -461,22 +460,19 @@ struct Dev {
   uint32_t *heavy_list, *heavy_cnt;   // [4N]: neuron, event count of the warp path, then of
                                       // the block path; heavy_cnt[0..1]: their lengths
   // bath
-  uint32_t *bath_hist;      // [P][64] ran3 history ring
-  uint64_t *bath_produced, *bath_pos;  // [P]
-  uint8_t *draw_idx;        // [P][BATH_RING] converted draws kept between steps
-  float *draw_lapse;        // [P][BATH_RING]
+  uint32_t *bath_hist;      // [P][BATH_HIST] the draws before each rank's next one
   uint64_t *bath_rank_base; // [P+1]
   uint32_t *bath_off;       // [N]
   uint16_t *bath_cnt;       // [N]
   double *bath_time;
   uint8_t *bath_lut;
-  logf_fixup_t fix;
   const uint32_t *fix_bitmap; // one bit per float in [0x30000000, 0x3F800000]: key has a fix-up
-  const float *fix_near;      // [256] by the result's exponent: a fix-up input's exact log lies at most
-                              // this many ulps from a rounding midpoint (-1: none in that binade)
+  const double *fix_near;     // [256] by the result's exponent: a fix-up input's exact log lies at least
+                              // this far from the float it rounds to
+  const double2 *log_tab;     // [LOG_TAB_N] i = LOG_TAB_0 + k: 64/i, log(i/64)
   // control
   uint32_t *t;              // current step
-  uint32_t *bath_t;         // step of the next bath launch (the bath runs one step ahead)
+  uint32_t *bath_t;         // [P] step of the rank's next bath (the bath runs one step ahead)
   uint32_t *flags;
   unsigned long long *events;  // synaptic events delivered
 };
@@ -733,844 +729,579 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
 // Step 3: the Poisson bath (regularDynamicTimeStep, DPSNN_neuron_sim.c:604-640,
 // getPoissonLapse :844-865).  Each rank owns one serial ran3 stream that its
 // neurons consume in index order: a neuron whose next bath time is before
-// t+1 takes one pair of draws (LUT index, lapse) per event.  One block per
-// rank runs a shared-memory pipeline:
-//   warp 1     extends the lagged Fibonacci sequence 24 values per round
-//              (x[n] = x[n-55] - x[n-24] mod 1e9) into a ring of raw draws;
-//   warps 2, 3 convert groups of four rounds into the LUT index (uint32)(u*256)
-//              and the lapse factor -logf((float)(1-u)), and extend q[], the
-//              running sum over draws of one parity of the lapses in 2^-20
-//              units (q[n] = q[n-2] + round(lap[n] * 2^20), integers mod 2^32);
-//   warps 5-7, 9-15 (builders) tabulate the event counts of the chunk of 32
-//              neurons two chunks ahead of the walk.  The number of events c
-//              of a neuron is the first c at which nextBath + sum of c lapses
-//              * invNuExt reaches t+1; it depends on where in the stream the
-//              neuron starts, which is known only once every earlier neuron
-//              of the rank is decided.  Each neuron's budget (t+1 -
-//              nextBath)/invNuExt becomes two integer bounds that enclose
-//              every rounding of the reference's sequential sum; its start is
-//              predicted from the latest known chunk start and the expected
-//              counts (1 + budget each); for the BATH_NC candidate starts
-//              around the prediction (a warp per neuron, two candidates per
-//              lane) a binary search of q[] finds c (c - 1 sums below the
-//              lower bound, the c-th at or above the upper one); a candidate
-//              the bounds do not decide is marked undecided.  A builder
-//              takes whole quads of neurons (the rank's quads in turn) and
-//              composes their tables itself: for every candidate start of
-//              neuron 2p the events of neurons 2p and 2p+1 together, then of
-//              4k .. 4k+3 together;
-//   warp 0     (walk) follows the chain: one lookup per four neurons, at the
-//              quad's actual start, gives the next quad's start.  A quad the
-//              tables do not decide goes neuron by neuron, and an undecided
-//              neuron (or one at the maxExternCurrentCount cap) runs the
-//              reference's sequential loop.  The lanes then recover every
-//              neuron's start and count from the pair and single tables in
-//              parallel and hand the chunk to
-//   warp 4     (emitter), whose lanes write the chunk's events, each
-//              replaying its neuron in the reference's exact arithmetic;
-//   warp 8     stays idle: warps go to the SM's four schedulers by index, so
-//              the walk shares its scheduler with the emitter only.
-// Rounds are published in order with a flag; every wait is bounded and
-// raises F_BATH_DRAWS when its limit is reached.
-#define BATH_THREADS 512       // 16 warps: roles in bath_kernel
-#define BATH_RING 8192         // draws resident in shared memory
-#define BATH_ROUNDS 512        // round flags tracked (BATH_ROUNDS*24 > BATH_RING)
-#define BATH_MAX_EXT 2048      // largest maxExternCurrentCount supported
-#define BATH_SPIN_LIMIT (1u << 26)
-#define BATH_FAST_LANES 32     // events decided by one count table entry
-#define BATH_WINDOW (2 * BATH_FAST_LANES + 2)   // draws a count decision reads past its start
-#define BATH_NC 64             // candidate start positions tabulated per neuron
-#define BATH_BUILDERS 10       // table-building warps: 5, 6, 7, 9 .. 15
-#define BATH_AHEAD 2           // chunks the count tables are built ahead of the consumer (the code below
-                               // predicts from chunk c-2's start)
-#define BATH_TABS (BATH_AHEAD + 1)
-#define BATH_CG 4              // generator rounds a converter takes at once: 96 draws, 3 per lane
-#define BATH_TROW (BATH_NC + 4)  // bytes per neuron in a count table: BATH_NC candidates, then the sentinel
+// t+1 takes one pair of draws (LUT index, lapse) per event, the first c pairs
+// at which nextBath + sum of c lapses * invNuExt reaches t+1.  Where a
+// neuron's pairs start is known only once every earlier neuron of the rank is
+// decided: a chain over the rank's neurons, which bounds the kernel.
+//
+// One block per rank.  The block meets at one barrier per round; in a round
+//   mappers     (warps 0-7) decide up to 128 neurons, 16 each: a mapper walks
+//               its 16 neurons from each of 32 candidate starts around the
+//               predicted one, a candidate per lane (bath_map).  The chain is
+//               then eight lookups (bath_compose, warp 0): each segment's
+//               end for its actual start.  A start outside a segment's window
+//               ends the round there;
+//   preparers   (8, 13) read the next neurons, turn each one's budget (t+1 -
+//               nextBath)/invNuExt into integer bounds, and queue those with
+//               an event this step (the others pass at once);
+//   converters  (9-11) turn 192 pairs of raw draws at a time into (LUT index,
+//               lapse) and extend q[], the running sum of the lapses in
+//               2^-20 units (integers mod 2^32);
+//   emitters    (12, 14) write the events of the neurons decided in the round
+//               before, a lane per neuron, each replaying its neuron in the
+//               reference's arithmetic;
+//   generator   (15) extends the stream's raw draws, 96 at a time.
+// Warps go to the SM's four schedulers by index: the roles are spread so that
+// each scheduler has two mappers and about the same instructions beside them.
+// Starts are predicted in time, not in pairs: a neuron's last event
+// overshoots its budget by a lapse of mean and deviation 1, so after n
+// neurons the start's q is the sum of the budgets and n, to within sqrt(n).
+// The pairs' parity is that of the launch's first draw (only draws past a
+// neuron's maxExternCurrentCount cap are single; after one the pairs start
+// afresh at the new position), so only every other draw becomes a lapse.
+// What bounds it: the latency of a round (a mapper's 16 dependent steps, then
+// the chain), not issue slots (a third used).  Segments of 16: a round costs
+// about 3000 cycles beside its steps, and at more neurons per segment the last
+// windows miss too often.  Measured per step (one B200), against the form
+// before, in which ten warps built tables of 64 candidate starts for every
+// neuron and every draw of both parities was converted: 62 us from 173 for one
+// rank of 1600 neurons, 99 from 300 for 11 ranks of 2743, 194 from 679 for 192
+// ranks of 3750, 16 from 67 for one of 100.  One warp deciding neuron by
+// neuron (a shared read, a vote and a count each) took 85 cycles per neuron
+// alone and 215 beside the other warps; this takes about 75.
+#define BATH_THREADS 512       // 16 warps: roles above
+#define BATH_SEG 16            // neurons per mapper
+#define BATH_SEGS 8            // mappers
+#define BATH_SB (BATH_SEG * BATH_SEGS)
+#define BATH_NC 32             // candidate starts of a segment: 4 deviations on either side of the second
+                               // one's, 1.5 of the last one's (a third of the rounds lose a segment or two)
+#define BATH_PAIRS 2048        // pairs resident: two rounds behind (the emitters' and the walk's own), and ahead
+#define BATH_MIRROR 1024       // the ring's first words again past its end: a round's reads do not wrap
+#define BATH_RAW (2 * BATH_PAIRS)   // raw draws resident
+#define BATH_HIST 256          // raw draws kept between launches (the generator reads 220 back)
+#define BATH_ACT 512           // queued neurons: those being emitted, decided and prepared
+#define BATH_CONV 192          // pairs converted at a time: 2 per lane of three warps
+#define BATH_AHEAD 960         // pairs converted ahead of the decided ones, at most
+#define BATH_MAX_EXT 121       // largest maxExternCurrentCount supported
+#define BATH_UNDECIDED 0xFFFFu // a segment's entry: to be walked
+#define BATH_NOT_YET 0xFFFEu   // or to be mapped in the next round
+static_assert(BATH_AHEAD + BATH_CONV + BATH_MAX_EXT + 64 < BATH_PAIRS,
+              "the walk always finds its next neuron's pairs converted or room for them");
+static_assert(BATH_SEG == 16 && BATH_NC == 32, "packed counts are 16 nibbles; a candidate per lane");
+static_assert(3 * BATH_SB + 64 <= BATH_ACT, "room to queue 64 neurons while two rounds' are held and one is ahead");
 
-static_assert(BATH_NC == 64, "a builder lane takes two candidate starts");
-static_assert(24 * BATH_CG == 96 && BATH_ROUNDS % BATH_CG == 0, "a converter group is 3 draws per lane");
-
-// q[] keeps the two parities apart: draws n, n+2, n+4, .. sit in consecutive
-// words, so the 32 lanes of a builder, each on its own candidate start two
-// draws from the next, read 32 different banks.
-__device__ __forceinline__ uint32_t bath_qi(unsigned long long n) {
-  return (((uint32_t)n & 1u) * (BATH_RING / 2)) | (((uint32_t)n & (BATH_RING - 1)) >> 1);
-}
-
-struct BathSmem {
-  uint32_t lap[BATH_RING];          // raw draw until converted, then the lapse (float bits)
-  uint32_t q[BATH_RING];            // per-parity prefix of the lapses, 2^-20 units, at bath_qi(n)
-  uint8_t idx[BATH_RING];
-  // count tables of chunk c in buffer c % BATH_TABS.  Neuron j: its events
-  // when it starts at bp_base[j] + 2o, 0xFF = undecided; entries BATH_NC..
-  // answer a start outside the window (0xFF; 0 for a neuron with no event
-  // this step, whose every entry is 0).  Pair p, quad k: the events of
-  // neurons 2p, 2p+1 (4k .. 4k+3) when 2p (4k) starts at bp_base[2p] + 2o.
-  uint8_t tab[BATH_TABS][32][BATH_TROW];
-  uint8_t tab2[BATH_TABS][16][BATH_TROW];
-  uint8_t tab4[BATH_TABS][8][BATH_TROW];
-  uint32_t bp_base[BATH_TABS][32];  // position (low 32 bits) of candidate 0 of neuron j
-  uint32_t tab_cnt[BATH_TABS];      // quads whose tables of this buffer are complete
-  uint32_t c_start[32], c_cnt[32];  // the walk's record: quad starts, and neurons walked one by one
-  uint32_t e_start[2][32], e_cnt[2][32];  // chunk c, handed to the emitter in buffer c & 1
-  unsigned long long e_end[2];      // its end position
-  uint32_t e_out[2];                // its first event slot
-  uint32_t e_seq, emit_done;        // chunks handed over, chunks emitted
-  unsigned long long emit_pos;      // ring slots before this position may be reused
-  unsigned long long chunk_start[BATH_TABS];  // exact start of chunk c (walk, as it begins chunk c)
-  uint32_t chunk_seq;               // chunks whose start is published
-  uint32_t flag[BATH_ROUNDS];       // round r converted <=> flag[r % BATH_ROUNDS] == r + 1
-  float near[256];                  // the logf fix-up filter's distances (Dev::fix_near)
-  uint32_t hist[64];
-  unsigned long long pos;           // walk position (draws)
-  unsigned long long raw_end;       // draws generated
-  unsigned long long conv_base;     // first draw of round 0 of this launch
-  uint32_t next_round;              // next group of BATH_CG rounds a converter claims
-  uint32_t published;               // rounds 0 .. published-1 are converted (raised after their flags)
-  uint32_t done, err;
+// What a round starts from; each field is written during the round before by
+// one warp, into the other copy.
+struct BathCtl {
+  uint32_t m, a;        // walk: next pair, next queued neuron
+  uint32_t rebase;      // walk: the pairs start afresh at this draw after this round (0: no)
+  uint32_t done;        // walk: nothing is left to decide or to emit
+  uint32_t act_end;     // preparers: queued neurons
+  uint32_t prep_done;   // preparers: every neuron of the rank seen
+  uint32_t conv_end;    // converters: pairs [0, conv_end) converted, from draw `base`
+  uint32_t raw_end;     // generator: raw draws [.., raw_end)
+  uint32_t sb_a, sb_n;  // walk: the neurons to emit
+  uint32_t slow;        // walk: its segments walked neuron by neuron (bits)
+  uint32_t keep;        // walk: first pair of the neurons being emitted
+  uint32_t base, out;   // walk: first draw of pair 0, events before it
 };
 
-// The table entry for a start dl draws after candidate 0: dl / 2 for an
-// even dl inside the window, else BATH_NC (an odd dl rotates into the top
-// bit).
-__device__ __forceinline__ uint32_t bath_row(uint32_t dl) {
-  return min(__funnelshift_r(dl, dl, 1), (uint32_t)BATH_NC);
+#define LOG_TAB_0 48
+#define LOG_TAB_N 49
+struct BathSmem {
+  uint32_t raw[BATH_RAW];           // draw n at n % BATH_RAW
+  uint32_t q[BATH_PAIRS + BATH_MIRROR];   // sum of the lapses of the pairs before k, at k % BATH_PAIRS
+  float lap[BATH_PAIRS];
+  uint8_t idx[BATH_PAIRS];
+  double a_nb[BATH_ACT], a_inv[BATH_ACT];   // queued neuron a at a % BATH_ACT
+  uint4 a_b[BATH_ACT];              // bounds lo and hi - lo, min(cap, 16), cap
+  uint32_t a_id[BATH_ACT];
+  uint32_t a_t[BATH_ACT];           // expected q advance of the queued neurons before a (2^-20 units)
+  uint2 pack[BATH_SEGS][BATH_NC];   // a segment's counts less one, a nibble per neuron, by candidate
+  uint16_t end[BATH_SEGS][BATH_NC + 2];   // its end, from win[], or BATH_UNDECIDED, BATH_NOT_YET
+  uint4 win[BATH_SEGS / 4];         // pair of candidate 0
+  uint2 e_pack[2][BATH_SEGS];       // decided segments by round parity: counts, first pairs
+  uint32_t e_start[2][BATH_SEGS];
+  uint32_t prep_n[2], prep_t[2];    // preparers: each one's queued neurons and their expected advance
+  uint32_t start[2][BATH_SB + 1];   // first pairs of the neurons of the slow segments, then their end
+  double near[256];                 // Dev::fix_near
+  double2 log_tab[LOG_TAB_N];       // Dev::log_tab
+  uint32_t conv_tot[3];             // converters: lapse sums of the warps' pairs
+  BathCtl ctl[2];
+};
+
+// The correctly rounded float log in the rare case that the double one does
+// not decide it; out of line, since inlined it takes the registers of the
+// whole kernel.
+__device__ __noinline__ static float logf_cr_undecided(float x) { return (float)log_cr((double)x); }
+
+// The double of a normal float's bits (no conversion instruction: those have a
+// quarter of the rate).
+__device__ __forceinline__ double double_of_bits(uint32_t fb) {
+  return __hiloint2double((int)((fb & 0x80000000u) | (((fb & 0x7FFFFFFFu) >> 3) + 0x38000000u)), (int)(fb << 29));
 }
 
-// The fix-up value of input key (when it has one), else f: a binary search of
-// the keys of its block of 4096 floats.
-__device__ static inline float logf_fixup_search(const logf_fixup_t &fx, uint32_t key, float f) {
-  const uint32_t bk = (key >> 12) - LOGF_FIX_BASE;
-  uint32_t lo = __ldg(&fx.bucket[bk]), hi = __ldg(&fx.bucket[bk + 1]);
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(&fx.keys[mid]) < key) lo = mid + 1; else hi = mid;
-  }
-  return (lo < fx.n && __ldg(&fx.keys[lo]) == key) ? __ldg(&fx.vals[lo]) : f;
-}
-
-// logf of the host C library on (0,1].  The inputs where it differs from
-// the correctly rounded float all have an exact logarithm close to a
-// rounding midpoint; an input whose logarithm lies farther from one than any
-// fix-up input of the same result binade returns the correctly rounded value
-// at once.  Otherwise a one-bit-per-float filter, then a binary search of
-// the fix-up keys of its block of 4096 floats.
-__device__ static inline float logf_ref_dev(const logf_fixup_t &fx, const uint32_t *__restrict__ bitmap,
-                                            const float *__restrict__ near, float x) {
-  const double y = log((double)x);
-  const float f = logf_cr_from(x, y);
-  union { float f; uint32_t u; } b;
-  b.f = x;
-  const uint32_t key = b.u;
-  if (key < 0x30000000u || key > 0x3F800000u) return f;
-  const uint32_t fb = __float_as_uint(f), E = (fb >> 23) & 0xFFu;
-  if ((fb & 0x7FFFFFu) != 0 && E > 24) {   // not a power of two: one ulp on either side
-    const double inv_ulp = __longlong_as_double((long long)(150 - E + 1023) << 52);   // 2^(150-E)
-    const double dist = 0.5 - fabs(y - (double)f) * inv_ulp;
-    if (dist > (double)__ldg(&near[E])) return f;
-  }
-  const uint32_t bit = key - 0x30000000u;
-  if (!((__ldg(&bitmap[bit >> 5]) >> (bit & 31)) & 1u)) return f;
-  return logf_fixup_search(fx, key, f);
-}
-
-// Converts raw draw mj into (LUT index, lapse) (getPoissonLapse, :844-865,
-// and the LUT index draw at :617-619).
-__device__ static inline float bath_lapse(const Dev &d, uint32_t mj, uint8_t &idx) {
-  const double u = mj * (1.0 / (double)MBIG);
-  idx = (uint8_t)(uint32_t)(u * 256);
-  double temp = (double)1.0 - u;
-  if (temp < 0) temp = 0;
-  return -logf_ref_dev(d.fix, d.fix_bitmap, d.fix_near, (float)temp);
-}
-
-// bath_lapse for three draws at once, each step for all three before the
-// next: their filter-table loads are in flight together.  near is the
-// per-binade distance table (logf_ref_dev), here from shared memory.
-__device__ static inline void bath_lapse3(const Dev &d, const float *near, const uint32_t (&mj)[3], float (&lap)[3],
-                                          uint8_t (&idx)[3]) {
-  float f[3];
-  uint32_t key[3], bw[3];
-  bool chk[3];
+// Lapses of K raw draws (getPoissonLapse, DPSNN_neuron_sim.c:844-865): -logf
+// of the host C library on (0,1].
+//  - The double log: x = 2^e m, m in [0.75,1.5), i = round(64 m), log x =
+//    e ln 2 + log(i/64) + log1p(r), r = m (64/i) - 1 in one rounding, |r| <=
+//    1/96, by the series through r^8; an error below 2^-49 of the result (for
+//    x near 1, i = 64 and the first two terms are zero).
+//  - Inputs where the C library differs from the correctly rounded float all
+//    have a logarithm close to a rounding midpoint: nearer than the furthest
+//    of them in the result's binade (near) a bit per float says whether x is
+//    one.  Its value is then the float on the midpoint's other side (checked
+//    when the table is loaded; a search of the table here took up to eight
+//    dependent loads, in half of a warp's conversions).
+// Each step is done for all K draws before the next, so that their loads are
+// in flight together.
+template <int K>
+__device__ static inline void bath_lapse(const Dev &d, const BathSmem &s, const uint32_t (&mj)[K], float (&lap)[K]) {
+  uint32_t fb[K], key[K], bw[K];
+  double r[K];
 #pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const double u = mj[i] * (1.0 / (double)MBIG);
-    idx[i] = (uint8_t)(uint32_t)(u * 256);
-    double temp = (double)1.0 - u;
-    if (temp < 0) temp = 0;
-    const float x = (float)temp;
-    const double y = log((double)x);
-    f[i] = logf_cr_from(x, y);
-    key[i] = __float_as_uint(x);
-    chk[i] = key[i] >= 0x30000000u && key[i] <= 0x3F800000u;
-    const uint32_t fb = __float_as_uint(f[i]), E = (fb >> 23) & 0xFFu;
-    if (chk[i] && (fb & 0x7FFFFFu) != 0 && E > 24) {
-      const double inv_ulp = __longlong_as_double((long long)(150 - E + 1023) << 52);   // 2^(150-E)
-      chk[i] = 0.5 - fabs(y - (double)f[i]) * inv_ulp <= (double)near[E];
+  for (int i = 0; i < K; i++) {
+    // u = mj / MBIG as the reference rounds it; x = (float)(1 - u)
+    const double u = (__hiloint2double(0x43300000, (int)mj[i]) - 0x1p52) * (1.0 / (double)MBIG);
+    key[i] = __float_as_uint((float)(1.0 - u));
+    const int e = (int)(key[i] - 0x3F400000u) >> 23;
+    const uint32_t mb = key[i] - ((uint32_t)e << 23);
+    const double2 c = s.log_tab[(int)(__uint_as_float(mb) * 64.0f + 0.5f) - LOG_TAB_0];
+    const double z = fma(double_of_bits(mb), c.x, -1.0);
+    double q = fma(z, -1.0 / 8, 1.0 / 7);
+    q = fma(z, q, -1.0 / 6);
+    q = fma(z, q, 1.0 / 5);
+    q = fma(z, q, -1.0 / 4);
+    q = fma(z, q, 1.0 / 3);
+    q = fma(z, q, -1.0 / 2);
+    const double ef = __hiloint2double(0x43300000, (int)(0x80000000u + (uint32_t)e)) - (0x1p52 + 0x1p31);
+    const double y = fma(ef, 0x1.62e42fefa39efp-1, c.y) + fma(z * z, q, z);
+    fb[i] = __float_as_uint((float)y);
+    r[i] = y - double_of_bits(fb[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < K; i++) {
+    bw[i] = 0;
+    if (fabs(r[i]) >= s.near[(fb[i] >> 23) & 0xFFu] || (fb[i] & 0x7FFFFFu) == 0)
+      bw[i] = __ldg(&d.fix_bitmap[(key[i] - 0x30000000u) >> 5]);   // 1e-9 <= x <= 1
+  }
+#pragma unroll
+  for (int i = 0; i < K; i++) {
+    // within 2^-18 of a midpoint (2^-24 of the binade, or 2^-25 below a power
+    // of two): the rounding needs more digits
+    const uint32_t E = (fb[i] >> 23) & 0xFFu;
+    const double half = __hiloint2double((int)((E - 24 + 896) << 20), 0);
+    if (fabs(r[i]) > half * (1.0 - 0x1p-18) ||
+        ((fb[i] & 0x7FFFFFu) == 0 && fabs(r[i]) > 0.5 * half * (1.0 - 0x1p-18))) {
+      if (E) {
+        const float f = logf_cr_undecided(__uint_as_float(key[i]));
+        r[i] += double_of_bits(fb[i]) - double_of_bits(__float_as_uint(f));
+        fb[i] = __float_as_uint(f);
+      }
     }
-  }
-#pragma unroll
-  for (int i = 0; i < 3; i++) bw[i] = chk[i] ? __ldg(&d.fix_bitmap[(key[i] - 0x30000000u) >> 5]) : 0u;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    if ((bw[i] >> ((key[i] - 0x30000000u) & 31)) & 1u) f[i] = logf_fixup_search(d.fix, key[i], f[i]);
-    lap[i] = -f[i];
+    // f < 0: the next float below has the next bit pattern
+    if ((bw[i] >> ((key[i] - 0x30000000u) & 31)) & 1u) fb[i] += r[i] < 0 ? 1u : 0xFFFFFFFFu;
+    lap[i] = -__uint_as_float(fb[i]);
   }
 }
 
 __device__ static inline uint32_t lap_fixed(float lap) {
-  return __double2uint_rn((double)lap * 0x1p20);   // lap < 2^11: no overflow
+  return __float2uint_rn(lap * 0x1p20f);   // an exact product; lap < 2^11: no overflow
 }
 
-// Integer bounds on the lapse sum, in 2^-20 units, for one neuron: a
-// fixed-point sum F of c lapses below lo means the reference's sequential
-// nextBath after c events is certainly < t+1, at or above hi1 certainly
-// >= t+1.  E1 bounds the rounding of that sequential sum (c <= 32
-// additions, |values| < |T1| + 42 invNuExt, and t+1 - nextBath); 2^-16
-// bounds the rounding of F (32 terms of at most 2^-21); the 2^-30 relative
-// margin covers the bound's own arithmetic.  Both are clamped to 32 bits
-// (F < 2^30).  misc: 0 = no bath event this step; else 0x100 |
-// min(32, maxExternCurrentCount).
-__device__ static inline void bath_bounds(double T1, double nb, double inv, uint32_t mx, uint32_t &lo,
-                                          uint32_t &hi1, uint32_t &misc) {
-  lo = hi1 = misc = 0;
-  if (inv > 0 && nb < T1) {
-    const double E1 = 0x1p-44 * (fabs(T1) + fabs(nb) + 1.0 + 32.0 * inv);
-    double blo = ((T1 - nb) - E1) / inv - 0x1p-16;
-    double bhi = ((T1 - nb) + E1) / inv + 0x1p-16;
-    const double mg = 0x1p-30 * (fabs(bhi) + 1.0);
-    blo = fmin(fmax(floor((blo - mg) * 0x1p20), 0.0), 4294967295.0);
-    bhi = fmin(fmax(ceil((bhi + mg) * 0x1p20) + 1.0, 0.0), 4294967295.0);
-    lo = (uint32_t)blo;
-    hi1 = (uint32_t)bhi;
-    misc = 0x100u | min(32u, mx);
+// Integer bounds on the lapse sum, in 2^-20 units, for one neuron with an
+// event this step (inv > 0, nb < T1): a fixed-point sum F of c lapses below
+// lo means the reference's sequential nextBath after c events is certainly <
+// t+1, at or above hi1 certainly >= t+1.  E1 bounds the rounding of that
+// sequential sum (c <= 32 additions, |values| < |T1| + 42 invNuExt, and t+1 -
+// nextBath); 2^-16 bounds the rounding of F (32 terms of at most 2^-21); the
+// 2^-30 relative margin covers the bound's own arithmetic.  Both are clamped
+// to 32 bits (F < 2^30).
+__device__ static inline void bath_bounds(double T1, double nb, double inv, uint32_t &lo, uint32_t &hi1) {
+  const double E1 = 0x1p-44 * (fabs(T1) + fabs(nb) + 1.0 + 32.0 * inv);
+  const double bud = (T1 - nb) / inv;
+  const double mg = 1.001 * (double)((float)E1 / (float)inv) + 0x1p-16 + 0x1p-30 * (bud + 1.0);
+  lo = __double2uint_rd(fmax((bud - mg) * 0x1p20, 0.0));   // the conversions clamp at 2^32 - 1
+  hi1 = __double2uint_ru((bud + mg) * 0x1p20);
+  hi1 += hi1 != 0xFFFFFFFFu;
+}
+
+// Draws past a neuron's cap, single ones (rare): from draw n on, until
+// nextBath reaches T1; returns the position after them, 0 when a draw that
+// is not generated yet is needed.
+__device__ static inline uint32_t bath_singles(const Dev &d, const BathSmem &s, uint32_t n, uint32_t raw_end,
+                                               double inv, double T1, double &v) {
+  do {
+    if (n >= raw_end) return 0;
+    const uint32_t mj[1] = {s.raw[n % BATH_RAW]};
+    float lp[1];
+    bath_lapse<1>(d, s, mj, lp);
+    v += (double)lp[0] * inv;
+    n++;
+  } while (v < T1);
+  return n;
+}
+
+// Mapper w: its segment's end and counts from every candidate start.
+__device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t w, uint32_t lane) {
+  const uint32_t A = BATH_ACT - 1, a0 = cur.a + BATH_SEG * w;
+  if (a0 >= cur.act_end || cur.rebase) return;
+  const uint32_t n = min(cur.act_end - a0, (uint32_t)BATH_SEG);
+  const uint32_t b = cur.m & (BATH_PAIRS - 1), lim = cur.conv_end - cur.m;   // q[b + i]: pair m + i; stale past lim
+  uint32_t win = 0;   // candidate 0, from m
+  if (w) {
+    // the pair at the predicted time, to within two: pairs have density 1, so
+    // it lies within a few sqrt(dt) of dt pairs on
+    const uint32_t dt = s.a_t[a0 & A] - s.a_t[cur.a & A], T = s.q[b] + dt;
+    const uint32_t first = max(min(dt >> 20, 600u), 64u) - 64, at = first + 4 * lane;
+    const uint32_t pred =
+        first + 4 * __popc(__ballot_sync(0xffffffffu, at <= lim && (int32_t)(s.q[b + at] - T) < 0)) - 2;
+    win = max(pred, (uint32_t)BATH_NC / 2) - BATH_NC / 2;
   }
-}
-
-// The reference's loop for one neuron from stream position pos
-// (regularDynamicTimeStep, DPSNN_neuron_sim.c:604-640): the events go to c,
-// the position after the neuron's draws is returned.  Waits (bounded) until
-// the draws it reads are converted; sets fail when a wait gives up.
-__device__ static inline unsigned long long bath_exact(BathSmem &s, double nbv, double inv, uint32_t mx, double T1,
-                                                       unsigned long long pos, unsigned long long &lim, uint32_t &rr,
-                                                       uint32_t &spins, bool &fail, uint32_t &c) {
-  volatile BathSmem &vs = s;
-  const uint32_t M = BATH_RING - 1;
-  c = 0;
-  while (lim < pos + 2ull * mx + 4) {
-    const uint32_t pb = vs.published;
-    if (pb > rr) {
-      rr = pb;
-      lim = s.conv_base + (unsigned long long)rr * 24;
-      __threadfence_block();
-    } else if (++spins > BATH_SPIN_LIMIT) {
-      fail = true;
-      return pos;
+  uint32_t p = b + win + lane, qm = s.q[p];
+  uint32_t pk = 0, pk0 = 0;
+  bool bad = false;
+  uint4 nb = s.a_b[a0 & A];
+#pragma unroll 1
+  for (uint32_t j = 0; j < n; j++) {
+    // the neuron's count: 1 + the number of sums of 1..16 lapses below lo,
+    // by fours, then within the four
+    const uint4 k = nb;
+    nb = s.a_b[(a0 + j + 1) & A];
+    const uint32_t T = qm + k.x;
+    const uint32_t n4 = ((s.q[p + 4] - T) >> 31) + ((s.q[p + 8] - T) >> 31) + ((s.q[p + 12] - T) >> 31);
+    const uint32_t x = p + 4 * n4;
+    const uint32_t y1 = s.q[x + 1] - T, y2 = s.q[x + 2] - T, y3 = s.q[x + 3] - T, y4 = s.q[x + 4] - T;
+    const uint32_t e = x + (y1 >> 31) + (y2 >> 31) + (y3 >> 31) + (y4 >> 31), c = e - p;
+    // the first sum not below lo, less lo: the negative ones are large unsigned
+    const uint32_t over = min(min(y1, y2), min(y3, y4));
+    // undecided: the sum lies between lo and hi, or the count is beyond
+    // sixteen or the neuron's cap
+    bad |= c >= k.z || over < k.y;
+    qm = T + over;
+    p = e + 1;
+    pk |= c << (4 * (j & 7));
+    if (j == 7) {
+      pk0 = pk;
+      pk = 0;
     }
   }
-  float ln = __uint_as_float(s.lap[(pos + 1) & M]);
-  do {
-    c++;
-    const double step = (double)ln * inv;
-    pos += 2;
-    ln = __uint_as_float(s.lap[(pos + 1) & M]);
-    nbv += step;
-  } while ((nbv < T1) && (c < mx));
-  if (c >= mx && nbv < T1) {
-    do {   // single draws past the cap (rare)
-      while (lim <= pos) {
-        const uint32_t pb = vs.published;
-        if (pb > rr) {
-          rr = pb;
-          lim = s.conv_base + (unsigned long long)rr * 24;
-          __threadfence_block();
-        } else if (++spins > BATH_SPIN_LIMIT) {
-          fail = true;
-          return pos;
-        }
-      }
-      nbv += (double)__uint_as_float(s.lap[pos & M]) * inv;
-      pos += 1;
-    } while (nbv < T1);
+  // an end within 16 pairs of the converted ones may rest on stale words
+  const uint32_t e = p - b;
+  s.end[w][lane] = (uint16_t)(e + 16 > lim ? BATH_NOT_YET : bad ? BATH_UNDECIDED : e - win);
+  s.pack[w][lane] = n > 7 ? make_uint2(pk0, pk) : make_uint2(pk, 0u);
+  if (lane == 0) {
+    reinterpret_cast<uint32_t *>(s.win)[w] = cur.m + win;
+    s.end[w][BATH_NC] = BATH_NOT_YET;
   }
-  return pos;
 }
 
-__device__ static inline int bath_builder_index(uint32_t warp) {
-  return (warp >= 5 && warp <= 7) ? (int)warp - 5 : (warp >= 9 && warp <= 15) ? (int)warp - 6 : -1;
+// Warp 0, the segments mapped: the chain over them, and the next round's
+// start.  A segment with no decided entry at its start runs neuron by
+// neuron: the sums of 1..32 lapses by lane and a vote, or the reference's
+// loop.
+__device__ static inline void bath_compose(const Dev &d, BathSmem &s, const BathCtl &cur, BathCtl &nxt, uint32_t par,
+                                           double T1, uint32_t lane) {
+  const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1, lim = cur.conv_end;
+  const uint32_t left = cur.rebase ? 0u : min(cur.act_end - cur.a, (uint32_t)BATH_SB);
+  const uint32_t nseg = (left + BATH_SEG - 1) / BATH_SEG;
+  uint32_t m = cur.m, n_done = 0, rebase = 0, slow = 0;
+  const uint4 wa = s.win[0], wb = s.win[1];
+  const uint32_t win[BATH_SEGS] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+  for (uint32_t g0 = 0; g0 < nseg;) {
+    // the chain over the segments from g0 on (a start outside the window
+    // finds the sentinel); lane g keeps segment g's start
+    uint32_t my_m = 0, my_w = 0, P = m;
+#pragma unroll
+    for (uint32_t g = 0; g < BATH_SEGS; g++) {
+      const uint32_t e = win[g] + s.end[g][min(P - win[g], (uint32_t)BATH_NC)];
+      my_m = lane == g ? P : my_m;
+      my_w = lane == g ? win[g] : my_w;
+      P = g >= g0 && g < nseg ? e : P;
+    }
+    const bool mine = lane >= g0 && lane < nseg;
+    const uint32_t my_o = min(my_m - my_w, (uint32_t)BATH_NC), my_e = mine ? s.end[lane][my_o] : 0u;
+    const uint32_t g1 = min((uint32_t)__ffs(__ballot_sync(0xffffffffu, my_e >= BATH_NOT_YET)) - 1u, nseg);
+    if (mine && lane < g1) {
+      s.e_start[par][lane] = my_m;
+      s.e_pack[par][lane] = s.pack[lane][my_o];
+    }
+    n_done = min(g1 * BATH_SEG, left);
+    if (g1 == nseg) {
+      m = P;
+      break;
+    }
+    m = __shfl_sync(0xffffffffu, my_m, g1);
+    if (__shfl_sync(0xffffffffu, my_e, g1) == BATH_NOT_YET) break;
+    slow |= 1u << g1;
+    const uint32_t n_end = min(n_done + BATH_SEG, left);
+    bool stop = false;
+    while (n_done < n_end && !stop) {
+      const uint32_t a = (cur.a + n_done) & A, mx = s.a_b[a].w, lo = s.a_b[a].x;
+      if (m + max(33u, mx + 1) > lim) {   // its pairs are not converted yet
+        stop = true;
+        break;
+      }
+      uint32_t c = 0;
+      const uint32_t F = s.q[(m + 1 + lane) & M] - s.q[m & M];
+      const uint32_t mm = __popc(__ballot_sync(0xffffffffu, F < lo));
+      if (mm < min(32u, mx) && __shfl_sync(0xffffffffu, F, mm) - lo >= s.a_b[a].y) c = mm + 1;
+      if (!c) {   // the reference's loop (DPSNN_neuron_sim.c:604-640)
+        const double inv = s.a_inv[a];
+        double v = s.a_nb[a];
+        do {
+          v += (double)s.lap[(m + c) & M] * inv;
+          c++;
+        } while (v < T1 && c < mx);
+        if (v < T1) {
+          rebase = bath_singles(d, s, cur.base + 2 * (m + c), cur.raw_end, inv, T1, v);
+          stop = true;
+          if (!rebase) break;   // draws not generated yet
+        }
+      }
+      if (lane == 0) {
+        s.start[par][n_done] = m;
+        s.start[par][n_done + 1] = m + c;
+      }
+      m += c;
+      n_done++;
+    }
+    if (stop) break;
+    g0 = g1 + 1;
+  }
+  const uint32_t a = cur.a + n_done;
+  if (lane == 0) {
+    nxt.sb_a = cur.a;
+    nxt.sb_n = a - cur.a;
+    nxt.slow = slow;
+    nxt.a = a;
+    nxt.rebase = rebase;
+    nxt.done = cur.prep_done && a == cur.act_end && n_done == 0 && !cur.rebase;
+    if (cur.rebase) {   // the neurons before it are emitted in this round
+      nxt.m = nxt.keep = 0;
+      nxt.base = cur.rebase;
+      nxt.out = cur.out + cur.m;
+    } else {
+      nxt.m = m;
+      nxt.keep = cur.m;
+      nxt.base = cur.base;
+      nxt.out = cur.out;
+    }
+  }
+}
+
+// Sum of the nibbles of x (at most 8 x 15).
+__device__ static inline uint32_t nibble_sum(uint32_t x) {
+  return (((x & 0x0F0F0F0Fu) + ((x >> 4) & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
 }
 
 __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
-  const uint32_t t = *d.bath_t;
   extern __shared__ __align__(16) unsigned char bath_smem_raw[];
   BathSmem &s = *reinterpret_cast<BathSmem *>(bath_smem_raw);
-  volatile BathSmem &vs = s;
   const NetConst *net = d.net;
   const uint32_t h = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t M = BATH_RING - 1;
-  // restore: generator history, consumer position, draws converted last launch
-  const unsigned long long p0 = d.bath_pos[h], q0 = d.bath_produced[h];
-  if (tid < 64) s.hist[tid] = d.bath_hist[h * 64 + tid];
-  for (unsigned long long n = p0 + tid; n < q0; n += blockDim.x) {
-    const uint32_t k = (uint32_t)n & M;
-    s.lap[k] = __float_as_uint(d.draw_lapse[(size_t)h * BATH_RING + k]);
-    s.idx[k] = d.draw_idx[(size_t)h * BATH_RING + k];
-  }
-  for (uint32_t r = tid; r < BATH_ROUNDS; r += blockDim.x) s.flag[r] = 0;
-  for (uint32_t r = tid; r < 256; r += blockDim.x) s.near[r] = d.fix_near[r];
-  if (tid == 0) {
-    s.pos = p0;
-    s.raw_end = q0;
-    s.conv_base = q0;
-    s.next_round = 0;
-    s.published = 0;
-    s.done = 0;
-    s.err = 0;
-    s.chunk_seq = 0;
-    s.e_seq = 0;
-    s.emit_done = 0;
-    s.emit_pos = p0;
-    for (int b = 0; b < BATH_TABS; b++) s.tab_cnt[b] = 0;
-    s.q[bath_qi(p0 - 2)] = 0;   // the prefix starts at p0 in each launch
-    s.q[bath_qi(p0 - 1)] = 0;
-  }
-  __syncthreads();
-  if (warp == 0) {   // prefix of the restored draws [p0, q0)
-    for (unsigned long long n0 = p0; n0 < q0; n0 += 32) {
-      const unsigned long long n = n0 + lane;
-      uint32_t v = (n < q0) ? lap_fixed(__uint_as_float(s.lap[n & M])) : 0u;
-      for (int o = 2; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= (uint32_t)o) v += y;
-      }
-      v += s.q[bath_qi(n0 - 2 + (lane & 1))];
-      __syncwarp();
-      if (n < q0) s.q[bath_qi(n)] = v;
-      __syncwarp();
-    }
-  }
-  __syncthreads();
+  const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1;
+  const uint32_t t = d.bath_t[h], locN = net->locN, i0 = h * locN;
   const double T1 = (double)((double)t + 1.0);
-  const uint32_t locN = net->locN, i0 = h * locN;
   const uint64_t ev_base = d.bath_rank_base[h];
-
-  if (warp == 1) {
-    // ---- generator
-    uint32_t r = 0;
-    while (true) {
-      const unsigned long long n0 = s.conv_base + (unsigned long long)r * 24;
-      uint32_t spins = 0;
-      while (!vs.done && n0 + 24 > vs.emit_pos + BATH_RING - 64) {
-        if (++spins > BATH_SPIN_LIMIT) { vs.err = 1; vs.done = 1; break; }
-        __nanosleep(64);   // leave the issue slots to the consumer
-      }
-      if (vs.done) break;
-      const uint32_t nn = (uint32_t)(n0 + lane);
-      int32_t x = 0;
-      if (lane < 24) {
-        x = (int32_t)s.hist[(nn - 55) & 63] - (int32_t)s.hist[(nn - 24) & 63];
-        if (x < 0) x += MBIG;
-      }
-      __syncwarp();
-      if (lane < 24) {
-        s.hist[nn & 63] = (uint32_t)x;
-        s.lap[nn & M] = (uint32_t)x;
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) vs.raw_end = n0 + 24;
-      r++;
-    }
-  } else if (bath_builder_index(warp) >= 0) {
-    // ---- count tables, two chunks ahead of the walk
-    const uint32_t bw = (uint32_t)bath_builder_index(warp);
-    unsigned long long pred = p0;   // predicted start of chunk c
-    uint32_t exp1 = 0, exp2 = 0;    // expected events of chunks c-1 and c-2
-    unsigned long long lim = s.raw_end;
-    uint32_t rr = 0, spins = 0;
-    bool fail = false;
-    // What does not depend on where a chunk starts -- each lane's neuron,
-    // its bounds and expected events, their prefix over the chunk -- is
-    // prepared a chunk early: the next chunk's loads are in flight while
-    // this chunk's candidates are evaluated.
-    uint32_t n_lo = 0, n_hi1 = 0, n_misc = 0, n_ec = 0, n_incl = 0;
-    double x_nb = 0, x_inv = 0;
-    uint32_t x_mx = 0;
-    auto prepare = [&](uint32_t cc0) {
-      const uint32_t ccn = min(32u, locN - cc0);
-      n_lo = n_hi1 = n_misc = n_ec = 0;
-      if (lane < ccn) {
-        bath_bounds(T1, x_nb, x_inv, x_mx, n_lo, n_hi1, n_misc);
-        if (n_misc) n_ec = 1u + (uint32_t)fmin(rint((T1 - x_nb) / x_inv), 64.0);   // expected events: 1 + budget
-      }
-      n_incl = n_ec;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, n_incl, o);
-        if (lane >= (uint32_t)o) n_incl += y;
-      }
-    };
-    if (lane < min(32u, locN)) {
-      x_nb = d.nb_prev[i0 + lane];
-      x_inv = d.inv_nu[i0 + lane];
-      x_mx = d.max_ext[i0 + lane];
-    }
-    prepare(0);
-    for (uint32_t c = 0, c0 = 0; c0 < locN; c++, c0 += 32) {
-      const uint32_t cn = min(32u, locN - c0), b = c % BATH_TABS;
-      const uint32_t lo = n_lo, hi1 = n_hi1, misc = n_misc, ec = n_ec, incl = n_incl;
-      if (c0 + 32 < locN && lane < min(32u, locN - c0 - 32)) {   // the next chunk's neurons
-        x_nb = d.nb_prev[i0 + c0 + 32 + lane];
-        x_inv = d.inv_nu[i0 + c0 + 32 + lane];
-        x_mx = d.max_ext[i0 + c0 + 32 + lane];
-      }
-      // the prediction starts from the latest chunk start known for sure,
-      // chunk c-2's (BATH_AHEAD = 2), published by the consumer as it begins
-      // that chunk (so it is also done with this buffer's previous tables),
-      // plus the expected events of chunks c-2 and c-1; chunk 0 starts at p0
-      unsigned long long floor_pos = p0;
-      if (c >= 3) {
-        while (vs.chunk_seq < c - 1) {
-          if (vs.done) { fail = true; break; }
-          if (++spins > BATH_SPIN_LIMIT) { vs.err = 1; vs.done = 1; fail = true; break; }
-          __nanosleep(32);
-        }
-        if (fail) break;
-        __threadfence_block();
-        floor_pos = vs.chunk_start[(c - 2) % BATH_TABS];
-      }
-      pred = floor_pos + 2ull * ((c >= 2 ? exp2 : 0u) + (c >= 1 ? exp1 : 0u));
-      exp2 = exp1;
-      exp1 = __shfl_sync(0xffffffffu, incl, 31);
-      // candidate o of this lane's neuron starts at base + 2o, the
-      // prediction in the middle of the window
-      const unsigned long long base = pred + 2ull * (incl - ec) - BATH_NC;
-      // the draws every candidate of the chunk reads are converted; never
-      // beyond what the generator may produce ahead of the walk (once the
-      // emitter is done with the chunks before c-2, at least floor_pos +
-      // BATH_RING - 64): candidates past that stay undecided
-      const unsigned long long reach = floor_pos + BATH_RING - 512;
-      const unsigned long long need =
-          min(__shfl_sync(0xffffffffu, base, 31) + 2ull * BATH_NC + BATH_WINDOW, reach);
-      while (lim < need) {
-        const uint32_t pb = vs.published;
-        if (pb > rr) {
-          rr = pb;
-          lim = s.conv_base + (unsigned long long)rr * 24;
-          __threadfence_block();
-        } else if (vs.done) {
-          fail = true;
-          break;
-        } else if (++spins > BATH_SPIN_LIMIT) {
-          vs.err = 1;
-          vs.done = 1;
-          fail = true;
-          break;
-        } else {
-          __nanosleep(32);
-        }
-      }
-      if (fail) break;
-      const uint32_t b32 = (uint32_t)base, f32 = (uint32_t)floor_pos;
-      const uint32_t r32 = (uint32_t)reach - BATH_WINDOW;
-      // this warp's quads of the chunk: the rank's quads go to the builders
-      // in turn (quad 8c + k to builder (8c + k) mod BATH_BUILDERS), so the
-      // builders share the quads evenly and need no other warp
-      for (uint32_t k = (bw + BATH_BUILDERS - (8 * c) % BATH_BUILDERS) % BATH_BUILDERS; k < 8; k += BATH_BUILDERS) {
-        // stage 1: the quad's neurons j = 4k .. 4k+3, two at a time (a half
-        // warp each); for neuron j the half's lanes take the candidates
-        // o = hl, hl + 16, hl + 32, hl + 48.  For a start P the count is
-        // m + 1, m the number of i < 32 whose sum of the i+1 lapses at P+1,
-        // P+3, .., P+1+2i is below lo (the sums grow with i), when the
-        // (m+1)-th sum reaches hi1.  Positions are taken modulo 2^32 (a step
-        // reads far fewer draws); the four candidates' binary searches run
-        // in lockstep.
-        for (uint32_t jp = 4 * k; jp < 4 * k + 4; jp += 2) {
-          const uint32_t hl = lane & 15u, j = jp + (lane >> 4);
-          const uint32_t mj = __shfl_sync(0xffffffffu, misc, j);
-          const uint32_t loj = __shfl_sync(0xffffffffu, lo, j), hij = __shfl_sync(0xffffffffu, hi1, j);
-          const uint32_t bj = __shfl_sync(0xffffffffu, b32, j);
-          uint8_t *row = s.tab[b][j];
-          if (!mj) {   // no bath event this step (or past the rank's last neuron): 0 from any start
-#pragma unroll
-            for (int v = 0; v < 4; v++) row[hl + 16 * v] = 0;
-          } else {
-            const uint32_t cap = mj & 0xFFu;
-            // draw P+1+2i of a candidate sits at word hv | ((w0 + i) mod 4096) of q[]
-            const uint32_t hv = ((bj + 1) & 1u) * (BATH_RING / 2);
-            uint32_t w0[4], qb[4], m[4];
-            bool ok[4];
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-              const uint32_t P = bj + 2u * (hl + 16u * v);
-              ok[v] = (int32_t)(P - f32) >= 0 && (int32_t)(r32 - P) >= 0;
-              w0[v] = (P + 1) >> 1;
-              qb[v] = s.q[hv | ((w0[v] - 1) & (BATH_RING / 2 - 1))];
-              m[v] = 0;
-            }
-#pragma unroll
-            for (uint32_t st = 16; st > 0; st >>= 1) {
-              uint32_t f[4];
-#pragma unroll
-              for (int v = 0; v < 4; v++) f[v] = s.q[hv | ((w0[v] + m[v] + st - 1) & (BATH_RING / 2 - 1))];
-#pragma unroll
-              for (int v = 0; v < 4; v++) m[v] += (f[v] - qb[v] < loj) ? st : 0u;
-            }
-#pragma unroll
-            for (int v = 0; v < 4; v++) {
-              const uint32_t F = s.q[hv | ((w0[v] + m[v]) & (BATH_RING / 2 - 1))] - qb[v];
-              const uint32_t mm = (m[v] == 31 && F < loj) ? 32u : m[v];
-              row[hl + 16 * v] = (ok[v] && mm < cap && F >= hij) ? (uint8_t)(mm + 1) : (uint8_t)0xFF;
-            }
-          }
-        }
-        // the quad's window bases, and each table's answer outside its
-        // window: 0 when none of its neurons has an event, else undecided
-        const uint32_t mq = __shfl_sync(0xffffffffu, misc, 4 * k + (lane & 3));
-        const uint32_t bq = __shfl_sync(0xffffffffu, b32, 4 * k + (lane & 3));
-        const uint32_t B0 = __shfl_sync(0xffffffffu, b32, 4 * k), B1 = __shfl_sync(0xffffffffu, b32, 4 * k + 1);
-        const uint32_t B2 = __shfl_sync(0xffffffffu, b32, 4 * k + 2), B3 = __shfl_sync(0xffffffffu, b32, 4 * k + 3);
-        const uint32_t m2a = __shfl_sync(0xffffffffu, mq, 0) | __shfl_sync(0xffffffffu, mq, 1);
-        const uint32_t m2b = __shfl_sync(0xffffffffu, mq, 2) | __shfl_sync(0xffffffffu, mq, 3);
-        if (lane < 4) {
-          s.bp_base[b][4 * k + lane] = bq;
-          *reinterpret_cast<uint32_t *>(&s.tab[b][4 * k + lane][BATH_NC]) = mq ? 0xFFFFFFFFu : 0u;
-        }
-        if (lane == 0) {
-          *reinterpret_cast<uint32_t *>(&s.tab2[b][2 * k][BATH_NC]) = m2a ? 0xFFFFFFFFu : 0u;
-          *reinterpret_cast<uint32_t *>(&s.tab2[b][2 * k + 1][BATH_NC]) = m2b ? 0xFFFFFFFFu : 0u;
-          *reinterpret_cast<uint32_t *>(&s.tab4[b][k][BATH_NC]) = (m2a | m2b) ? 0xFFFFFFFFu : 0u;
-        }
-        __syncwarp();
-        // stage 2: the two pairs, from each candidate start of neuron 2p through 2p+1
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const uint32_t pp = 2 * k + (v >> 1), o = lane + 32u * (v & 1), a = 2 * pp;
-          const uint32_t ba = (v >> 1) ? B2 : B0, bn = (v >> 1) ? B3 : B1;
-          const uint32_t ca = s.tab[b][a][o];
-          uint32_t val = 0xFFu;
-          if (ca != 0xFFu) {
-            const uint32_t cb = s.tab[b][a + 1][bath_row(ba + 2 * (o + ca) - bn)];
-            if (cb != 0xFFu) val = ca + cb;
-          }
-          s.tab2[b][pp][o] = (uint8_t)val;
-        }
-        __syncwarp();
-        // stage 3: the quad, from each candidate start of neuron 4k through its two pairs
-#pragma unroll
-        for (int v = 0; v < 2; v++) {
-          const uint32_t o = lane + 32u * v;
-          const uint32_t va = s.tab2[b][2 * k][o];
-          uint32_t val = 0xFFu;
-          if (va != 0xFFu) {
-            const uint32_t vb = s.tab2[b][2 * k + 1][bath_row(B0 + 2 * (o + va) - B2)];
-            if (vb != 0xFFu) val = va + vb;   // at most 4 x 32
-          }
-          s.tab4[b][k][o] = (uint8_t)val;
-        }
-        __syncwarp();
-        __threadfence_block();
-        if (lane == 0) atomicAdd(&s.tab_cnt[b], 1u);
-      }
-      if (c0 + 32 < locN) prepare(c0 + 32);
-    }
-  } else if (warp == 2 || warp == 3) {
-    // ---- converters: groups of BATH_CG rounds (3 draws per lane) are
-    // claimed in order and published in order
-    while (true) {
-      uint32_t g = 0;
-      if (lane == 0) g = atomicAdd(&s.next_round, 1u);
-      g = __shfl_sync(0xffffffffu, g, 0);
-      const uint32_t r0 = g * BATH_CG;
-      const unsigned long long n0 = s.conv_base + (unsigned long long)r0 * 24;
-      uint32_t spins = 0;
-      bool quit = false;
-      while (true) {
-        if (vs.raw_end >= n0 + 24 * BATH_CG) break;
-        if (vs.done) { quit = true; break; }
-        if (++spins > BATH_SPIN_LIMIT) { vs.err = 1; vs.done = 1; quit = true; break; }
-        __nanosleep(64);
-      }
-      if (quit) break;
-      __threadfence_block();
-      uint8_t ix[3];
-      float lp[3];
-      uint32_t v[3];
-      {
-        uint32_t raw[3];
-#pragma unroll
-        for (int i = 0; i < 3; i++) raw[i] = vs.lap[(n0 + lane + 32 * i) & M];
-        bath_lapse3(d, s.near, raw, lp, ix);
-      }
-#pragma unroll
-      for (int i = 0; i < 3; i++) v[i] = lap_fixed(lp[i]);
-      // per-parity prefix over the 96 draws: within each 32, then the
-      // totals of the earlier 32s (lanes 30, 31) carried
-      for (int o = 2; o < 32; o <<= 1) {
-#pragma unroll
-        for (int i = 0; i < 3; i++) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, v[i], o);
-          if (lane >= (uint32_t)o) v[i] += y;
-        }
-      }
-      const uint32_t c0 = __shfl_sync(0xffffffffu, v[0], 30 + (lane & 1));
-      const uint32_t c1 = __shfl_sync(0xffffffffu, v[1], 30 + (lane & 1));
-      v[1] += c0;
-      v[2] += c0 + c1;
-      // the previous group's prefix is final once its last flag is set
-      if (r0 > 0) {
-        spins = 0;
-        while (true) {
-          if (vs.flag[(r0 - 1) % BATH_ROUNDS] == r0) break;
-          if (vs.done) { quit = true; break; }
-          if (++spins > BATH_SPIN_LIMIT) { vs.err = 1; vs.done = 1; quit = true; break; }
-          __nanosleep(32);
-        }
-        if (quit) break;   // nothing of this group was written
-        __threadfence_block();
-      }
-      const uint32_t qb = vs.q[bath_qi(n0 - 2 + (lane & 1))];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        const unsigned long long n = n0 + lane + 32 * i;
-        s.lap[n & M] = __float_as_uint(lp[i]);
-        s.idx[n & M] = ix[i];
-        s.q[bath_qi(n)] = v[i] + qb;
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane < BATH_CG) vs.flag[(r0 + lane) % BATH_ROUNDS] = r0 + lane + 1;
-      if (lane == 0) atomicMax(&s.published, r0 + BATH_CG);   // groups finish in order, their stores need not
-    }
-  } else if (warp == 0) {
-    // ---- walk (warp 0)
-    unsigned long long pos = s.pos;
-    unsigned long long lim = s.raw_end;   // converted draws available (prefix)
-    uint32_t rr = 0;                      // rounds known converted
-    uint32_t out = 0, spins = 0;
-    bool fail = false;
-    double nx_nb = 0, nx_inv = 0;
-    uint32_t nx_mx = 0;
-    if (lane < min(32u, locN)) {
-      nx_nb = d.nb_prev[i0 + lane];
-      nx_inv = d.inv_nu[i0 + lane];
-      nx_mx = d.max_ext[i0 + lane];
-    }
-    for (uint32_t c0 = 0, ck = 0; c0 < locN && !fail; c0 += 32, ck++) {
-      const uint32_t cn = min(32u, locN - c0), tb = ck % BATH_TABS, eb = ck & 1u;
-      const double my_nb = nx_nb, my_inv = nx_inv;
-      const uint32_t my_mx = nx_mx;
-      // this chunk's count tables, then its start for the builders
-      {
-        uint32_t sp = 0;
-        while (vs.tab_cnt[tb] < 8u * (ck / BATH_TABS + 1)) {
-          if (vs.done || ++sp > BATH_SPIN_LIMIT) { fail = true; break; }
-          __nanosleep(20);   // leave the shared-memory pipe to the builders
-        }
-        if (fail) break;
-        __threadfence_block();
-        if (lane == 0) {
-          vs.chunk_start[ck % BATH_TABS] = pos;
-          __threadfence_block();
-          vs.chunk_seq = ck + 1;
-        }
-      }
-      if (c0 + 32 < locN && lane < min(32u, locN - c0 - 32)) {   // prefetch the next chunk
-        nx_nb = d.nb_prev[i0 + c0 + 32 + lane];
-        nx_inv = d.inv_nu[i0 + c0 + 32 + lane];
-        nx_mx = d.max_ext[i0 + c0 + 32 + lane];
-      }
-      // the serial chain: one lookup per quad at its actual start; a run
-      // has no branch on the chain (an out-of-window start reads the
-      // sentinel); the first undecided quad is walked neuron by neuron
-      // below and the run goes on after it
-      const unsigned long long base = pos;
-      const uint32_t *bb = s.bp_base[tb];
-      const uint8_t *t1 = &s.tab[tb][0][0], *t2 = &s.tab2[tb][0][0], *t4 = &s.tab4[tb][0][0];
-      uint32_t P = (uint32_t)base, slow = 0;
-      for (uint32_t k0 = 0; k0 < 8;) {
-        uint32_t bad = 8;
-#pragma unroll 4
-        for (uint32_t k = k0; k < 8; k++) {
-          const uint32_t v = t4[k * BATH_TROW + bath_row(P - bb[4 * k])];
-          bad = (bad == 8 && v == 0xFFu) ? k : bad;
-          if (lane == 0) s.c_start[4 * k] = P;
-          P += 2 * v;
-        }
-        if (bad == 8) break;
-        __syncwarp();
-        P = s.c_start[4 * bad];
-        for (uint32_t j = 4 * bad; j < 4 * bad + 4; j++) {
-          uint32_t cx = t1[j * BATH_TROW + bath_row(P - bb[j])];
-          uint32_t Pn = P + 2 * cx;
-          if (cx == 0xFFu) {
-            // the reference's loop from the actual start; the emitter
-            // first finishes the earlier chunks, so that the ring holds
-            // every draw the loop may read
-            uint32_t sp = 0;
-            while (vs.emit_done < ck) {
-              if (vs.err || ++sp > BATH_SPIN_LIMIT) { fail = true; break; }
-              __nanosleep(32);
-            }
-            if (fail) break;
-            const unsigned long long pj = base + (uint32_t)(P - (uint32_t)base);
-            const unsigned long long pe = bath_exact(s, __shfl_sync(0xffffffffu, my_nb, j),
-                                                     __shfl_sync(0xffffffffu, my_inv, j),
-                                                     __shfl_sync(0xffffffffu, my_mx, j), T1, pj, lim, rr, spins, fail, cx);
-            if (fail) break;
-            Pn = (uint32_t)pe;
-          }
-          if (lane == 0) {
-            s.c_start[j] = P;
-            s.c_cnt[j] = cx;
-          }
-          P = Pn;
-        }
-        if (fail) break;
-        slow |= 1u << bad;
-        k0 = bad + 1;
-      }
-      if (fail) break;
-      __syncwarp();
-      // every neuron's start and events: from its quad's start through the
-      // pair and single tables (entries the quad's own entry was made of),
-      // or as the neuron-by-neuron walk recorded them
-      uint32_t my_start, my_cnt;
-      if ((slow >> (lane >> 2)) & 1u) {
-        my_start = s.c_start[lane];
-        my_cnt = s.c_cnt[lane];
-      } else {
-        uint32_t pq = s.c_start[lane & ~3u];
-        if (lane & 2u) pq += 2 * t2[((lane >> 1) & ~1u) * BATH_TROW + bath_row(pq - bb[lane & ~3u])];
-        if (lane & 1u) pq += 2 * t1[(lane & ~1u) * BATH_TROW + bath_row(pq - bb[lane & ~1u])];
-        my_start = pq;
-        my_cnt = t1[lane * BATH_TROW + bath_row(pq - bb[lane])];
-      }
-      if (lane >= cn) my_cnt = 0;
-      uint32_t tot = my_cnt;
-      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-      pos = base + (uint32_t)(P - (uint32_t)base);
-      // hand the chunk to the emitter: buffer eb is free once chunk ck-2 is emitted
-      if (ck >= 2) {
-        uint32_t sp = 0;
-        while (vs.emit_done < ck - 1) {
-          if (vs.err || ++sp > BATH_SPIN_LIMIT) { fail = true; break; }
-          __nanosleep(32);
-        }
-        if (fail) break;
-      }
-      s.e_start[eb][lane] = my_start;
-      s.e_cnt[eb][lane] = my_cnt;
-      if (lane == 0) {
-        s.e_out[eb] = out;
-        s.e_end[eb] = pos;
-      }
-      out += tot;
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) vs.e_seq = ck + 1;
-    }
-    if (lane == 0) {
-      if (fail) vs.err = 1;
-      vs.pos = pos;
-      __threadfence_block();
-      vs.done = 1;
-    }
-  } else if (warp == 4) {
-    // ---- emitter (warp 4): a chunk's events, each lane replaying its
-    // neuron in the reference's arithmetic
-    double nx_nb = 0, nx_inv = 0;
-    uint32_t nx_mx = 0;
-    if (lane < min(32u, locN)) {
-      nx_nb = d.nb_prev[i0 + lane];
-      nx_inv = d.inv_nu[i0 + lane];
-      nx_mx = d.max_ext[i0 + lane];
-    }
-    for (uint32_t c0 = 0, ck = 0; c0 < locN; c0 += 32, ck++) {
-      const uint32_t cn = min(32u, locN - c0), eb = ck & 1u;
-      const double my_nb = nx_nb, my_inv = nx_inv;
-      const uint32_t my_mx = nx_mx;
-      if (c0 + 32 < locN && lane < min(32u, locN - c0 - 32)) {
-        nx_nb = d.nb_prev[i0 + c0 + 32 + lane];
-        nx_inv = d.inv_nu[i0 + c0 + 32 + lane];
-        nx_mx = d.max_ext[i0 + c0 + 32 + lane];
-      }
-      bool quit = false;
-      uint32_t sp = 0;
-      while (vs.e_seq < ck + 1) {
-        if (vs.err) { quit = true; break; }
-        if (++sp > BATH_SPIN_LIMIT) { vs.err = 1; vs.done = 1; quit = true; break; }
-        __nanosleep(32);
-      }
-      if (__any_sync(0xffffffffu, quit)) break;
-      __threadfence_block();
-      const uint32_t my_start = s.e_start[eb][lane], my_cnt = s.e_cnt[eb][lane];
-      const uint32_t out = s.e_out[eb];
-      const unsigned long long end = s.e_end[eb];
-      if (__any_sync(0xffffffffu, lane < cn && my_cnt > my_mx)) {   // beyond the rank's event slots
-        if (lane == 0) { vs.err = 1; vs.done = 1; }
-        break;
-      }
-      uint32_t incl = my_cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (uint32_t)o) incl += y;
-      }
-      const uint32_t my_off = out + incl - my_cnt;
-      if (lane < cn) {
-        double v = my_nb;
-        uint32_t p = my_start;
-        double *bt = d.bath_time + ev_base + my_off;
-        uint8_t *bl = d.bath_lut + ev_base + my_off;
-        for (uint32_t c = 0; c < my_cnt; c++) {
-          bt[c] = v;
-          bl[c] = s.idx[p & M];
-          v += (double)__uint_as_float(s.lap[(p + 1) & M]) * my_inv;
-          p += 2;
-        }
-        if (my_cnt >= my_mx && my_cnt > 0 && v < T1) {
-          do {   // single draws past the cap
-            v += (double)__uint_as_float(s.lap[p & M]) * my_inv;
-            p += 1;
-          } while (v < T1);
-        }
-        d.nb[i0 + c0 + lane] = v;
-        d.bath_off[i0 + c0 + lane] = my_off;
-        d.bath_cnt[i0 + c0 + lane] = (uint16_t)my_cnt;
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) {
-        vs.emit_pos = end;
-        __threadfence_block();
-        vs.emit_done = ck + 1;
-      }
+  // draws of this launch are numbered from BATH_HIST; the ones before are the
+  // rank's kept history
+  for (uint32_t n = tid; n < BATH_HIST; n += BATH_THREADS) s.raw[n] = d.bath_hist[(size_t)h * BATH_HIST + n];
+  for (uint32_t r = tid; r < 256; r += BATH_THREADS) s.near[r] = d.fix_near[r];
+  for (uint32_t r = tid; r < LOG_TAB_N; r += BATH_THREADS) s.log_tab[r] = d.log_tab[r];
+  if (tid == 0) {
+    s.q[0] = s.q[BATH_PAIRS] = 0;
+    s.a_t[0] = 0;
+    BathCtl c = {};
+    c.raw_end = c.base = BATH_HIST;
+    s.ctl[0] = c;
+  }
+  // the preparers' next neurons, loaded an iteration ahead
+  uint32_t p_i = 0, p_t = 0, x_mx = 0;
+  double x_nb = 0, x_inv = 0;
+  if (warp == 8 || warp == 13) {
+    const uint32_t i = lane + (warp == 8 ? 0 : 32);
+    if (i < locN) {
+      x_nb = d.nb_prev[i0 + i];
+      x_inv = d.inv_nu[i0 + i];
+      x_mx = d.max_ext[i0 + i];
     }
   }
   __syncthreads();
-  if (s.err) {
+  // a round decides a neuron, or brings its draws closer; the limit is far
+  // beyond what a launch takes
+  const uint32_t max_rounds = 64 + 16 * locN;
+  uint32_t r = 0;
+  for (;; r++) {
+    const BathCtl &cur = s.ctl[r & 1];
+    BathCtl &nxt = s.ctl[(r + 1) & 1];
+    if (cur.done || r == max_rounds) break;
+    if (warp < BATH_SEGS) {
+      bath_map(s, cur, warp, lane);
+      asm volatile("bar.sync 1, 256;" ::: "memory");   // the mappers
+      if (warp == 0) bath_compose(d, s, cur, nxt, r & 1, T1, lane);
+    } else if (warp == 15) {
+      // x[n] = x[n-55] - x[n-24] mod 1e9, applied four times over: x[n] = x[n-96] - 4 x[n-127] + 6 x[n-158]
+      // - 4 x[n-189] + x[n-220], so that 96 draws follow from the ones before them at once; keeping BATH_HIST
+      // draws behind the neurons being emitted
+      uint32_t n = cur.raw_end;
+      const uint32_t room =
+          min(cur.base + 2 * (cur.m + BATH_AHEAD + BATH_CONV), cur.base + 2 * cur.keep + BATH_RAW - BATH_HIST);
+      for (int g = 0; g < 8 && n + 96 <= room; g++, n += 96) {
+        uint32_t x[3];
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+          const uint32_t k = n + lane + 32 * v;
+          const int32_t x3 = 2 * (int32_t)s.raw[(k - 158) % BATH_RAW];   // every term below is within 2 MBIG of 0
+          int32_t y = (int32_t)(s.raw[(k - 96) % BATH_RAW] + s.raw[(k - 220) % BATH_RAW]) - x3;
+          int32_t z = (int32_t)(s.raw[(k - 127) % BATH_RAW] + s.raw[(k - 189) % BATH_RAW]) - x3;
+          if (y < 0) y += MBIG;
+          if (y < 0) y += MBIG;
+          if (y >= MBIG) y -= MBIG;
+          if (z < 0) z += MBIG;
+          if (z < 0) z += MBIG;
+          z = 2 * (z >= MBIG ? z - MBIG : z);
+          if (z >= MBIG) z -= MBIG;
+          y -= 2 * z;   // x = y - 4 z
+          if (y < 0) y += MBIG;
+          if (y < 0) y += MBIG;
+          x[v] = (uint32_t)y;
+        }
+#pragma unroll
+        for (int v = 0; v < 3; v++) s.raw[(n + lane + 32 * v) % BATH_RAW] = x[v];
+        __syncwarp();
+      }
+      if (lane == 0) nxt.raw_end = n;
+    } else if (warp == 8 || warp == 13) {
+      // ---- preparers, a warp per 32 neurons: enough queued for the next two rounds
+      const uint32_t pw = warp == 8 ? 0 : 1;
+      uint32_t e = cur.act_end;
+      for (int g = 0; g < 4 && p_i < locN && e < cur.a + 2 * BATH_SB && e + 64 <= cur.sb_a + BATH_ACT; g++, p_i += 64) {
+        const double nb = x_nb, inv = x_inv;
+        const uint32_t mx = x_mx, i = p_i + 32 * pw + lane;
+        if (i + 64 < locN) {
+          x_nb = d.nb_prev[i0 + i + 64];
+          x_inv = d.inv_nu[i0 + i + 64];
+          x_mx = d.max_ext[i0 + i + 64];
+        }
+        const bool act = i < locN && inv > 0 && nb < T1;
+        const uint32_t bal = __ballot_sync(0xffffffffu, act);
+        uint32_t lo = 0, hi1 = 0;
+        if (act) bath_bounds(T1, nb, inv, lo, hi1);
+        const uint32_t tv = act ? min(lo, 64u << 20) + (1u << 20) : 0u;
+        uint32_t incl = tv;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= (uint32_t)o) incl += y;
+        }
+        const uint32_t sum = __shfl_sync(0xffffffffu, incl, 31);
+        s.prep_n[pw] = __popc(bal);
+        s.prep_t[pw] = sum;
+        asm volatile("bar.sync 3, 64;" ::: "memory");   // the two preparers
+        const uint32_t n0 = s.prep_n[0], n1 = s.prep_n[1], t0 = s.prep_t[0], t1 = s.prep_t[1];
+        if (act) {
+          const uint32_t k = (e + pw * n0 + __popc(bal & ((1u << lane) - 1))) & A;
+          s.a_nb[k] = nb;
+          s.a_inv[k] = inv;
+          s.a_b[k] = make_uint4(lo, hi1 - lo, min(mx, 16u), mx);
+          s.a_id[k] = i;
+          s.a_t[k] = p_t + pw * t0 + incl - tv;
+        } else if (i < locN) {
+          d.nb[i0 + i] = nb;
+          d.bath_off[i0 + i] = 0;
+          d.bath_cnt[i0 + i] = 0;
+        }
+        p_t += t0 + t1;
+        e += n0 + n1;
+        asm volatile("bar.sync 3, 64;" ::: "memory");
+      }
+      if (pw == 0 && lane == 0) {
+        s.a_t[e & A] = p_t;
+        nxt.act_end = e;
+        nxt.prep_done = p_i >= locN;
+      }
+    } else if (warp >= 9 && warp < 12) {
+      // ---- converters: up to BATH_AHEAD pairs ahead, and no further than the last neurons need
+      const uint32_t cw = warp - 9;
+      uint32_t k0 = cur.conv_end;
+      uint32_t want = cur.m + BATH_AHEAD;
+      if (cur.prep_done) {
+        const float left = (float)((s.a_t[cur.act_end & A] - s.a_t[cur.a & A]) >> 20);
+        want = min(want, cur.m + 160 + (uint32_t)(left + 4.0f * sqrtf(left)));
+      }
+      const uint32_t room = min(cur.keep + BATH_PAIRS - 1, (cur.raw_end - cur.base) / 2);
+      for (int g = 0; g < 3 && k0 < want && k0 + BATH_CONV <= room && !cur.rebase; g++, k0 += BATH_CONV) {
+        const uint32_t kl = k0 + cw * 64 + 2 * lane, n = cur.base + 2 * kl;
+        const uint32_t mi0 = s.raw[n % BATH_RAW], mi1 = s.raw[(n + 2) % BATH_RAW];
+        const uint32_t mj[2] = {s.raw[(n + 1) % BATH_RAW], s.raw[(n + 3) % BATH_RAW]};
+        float lp[2];
+        bath_lapse<2>(d, s, mj, lp);
+        const uint32_t f0 = lap_fixed(lp[0]), f1 = lap_fixed(lp[1]);
+        uint32_t incl = f0 + f1;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane == 31) s.conv_tot[cw] = incl;
+        asm volatile("bar.sync 2, 96;" ::: "memory");   // the converters
+        uint32_t qb = s.q[k0 & M] + incl;
+        for (uint32_t w = 0; w < cw; w++) qb += s.conv_tot[w];
+        const uint32_t k1 = (kl + 1) & M, k2 = (kl + 2) & M;
+        s.lap[kl & M] = lp[0];
+        s.lap[k1] = lp[1];
+        // the LUT index draw (:617-619): (uint32_t)(u * 256) is mj / (MBIG / 256) for every draw
+        s.idx[kl & M] = (uint8_t)(mi0 / (MBIG / 256));
+        s.idx[k1] = (uint8_t)(mi1 / (MBIG / 256));
+        s.q[k1] = qb - f1;
+        s.q[k2] = qb;
+        if (k1 < BATH_MIRROR) s.q[k1 + BATH_PAIRS] = qb - f1;
+        if (k2 < BATH_MIRROR) s.q[k2 + BATH_PAIRS] = qb;
+        asm volatile("bar.sync 2, 96;" ::: "memory");
+      }
+      if (cw == 0 && lane == 0) nxt.conv_end = cur.rebase ? 0u : k0;
+    } else {
+      // ---- emitters: the neurons of the last round
+      const uint32_t par = (r + 1) & 1;
+      for (uint32_t j = lane + (warp == 12 ? 0 : 32); j < cur.sb_n; j += 64) {
+        const uint32_t a = (cur.sb_a + j) & A, g = j / BATH_SEG, jj = j % BATH_SEG;
+        uint32_t m0, cnt;
+        if ((cur.slow >> g) & 1u) {
+          m0 = s.start[par][j];
+          cnt = s.start[par][j + 1] - m0;
+        } else {
+          const uint2 pk = s.e_pack[par][g];
+          const uint32_t word = jj < 8 ? pk.x : pk.y, sh = 4 * (jj & 7);
+          m0 = s.e_start[par][g] + jj + nibble_sum(word & ((1u << sh) - 1)) + (jj < 8 ? 0u : nibble_sum(pk.x));
+          cnt = ((word >> sh) & 15u) + 1;
+        }
+        const uint32_t i = i0 + s.a_id[a], off = cur.out + m0;
+        const double inv = s.a_inv[a];
+        double v = s.a_nb[a];
+        double *bt = d.bath_time + ev_base + off;
+        uint8_t *bl = d.bath_lut + ev_base + off;
+        for (uint32_t c = 0; c < cnt; c++) {
+          bt[c] = v;
+          bl[c] = s.idx[(m0 + c) & M];
+          v += (double)s.lap[(m0 + c) & M] * inv;
+        }
+        if (v < T1) bath_singles(d, s, cur.base + 2 * (m0 + cnt), cur.raw_end, inv, T1, v);
+        d.nb[i] = v;
+        d.bath_off[i] = off;
+        d.bath_cnt[i] = (uint16_t)cnt;
+      }
+    }
+    __syncthreads();
+  }
+  const BathCtl &fin = s.ctl[r & 1];
+  if (r == max_rounds) {
     if (tid == 0) atomicOr(d.flags, F_BATH_DRAWS);
     return;
   }
-  // convert the generated rounds no converter published (they follow the
-  // published ones, and still hold raw draws), then save the state
-  const unsigned long long re = s.raw_end;
-  for (unsigned long long n = s.conv_base + 24ull * s.published + tid; n < re; n += blockDim.x) {
-    uint8_t ix = 0;
-    const float lp = bath_lapse(d, s.lap[n & M], ix);
-    s.lap[n & M] = __float_as_uint(lp);
-    s.idx[n & M] = ix;
-  }
-  __syncthreads();
-  for (unsigned long long n = s.pos + tid; n < re; n += blockDim.x) {
-    const uint32_t k = (uint32_t)n & M;
-    d.draw_lapse[(size_t)h * BATH_RING + k] = __uint_as_float(s.lap[k]);
-    d.draw_idx[(size_t)h * BATH_RING + k] = s.idx[k];
-  }
-  if (tid < 64) d.bath_hist[h * 64 + tid] = s.hist[tid];
-  if (tid == 0) {
-    d.bath_pos[h] = s.pos;
-    d.bath_produced[h] = re;
-  }
+  // the history of the next launch: the draws before the first unused one
+  const uint32_t pos = fin.base + 2 * fin.m;
+  for (uint32_t n = tid; n < BATH_HIST; n += BATH_THREADS)
+    d.bath_hist[(size_t)h * BATH_HIST + n] = s.raw[(pos - BATH_HIST + n) % BATH_RAW];
+  if (tid == 0) d.bath_t[h] = t + 1;
 }
 
 // LIFCADynamic, non-PerseoDyn branch (DPSNN_neuron_sim.c:664-824): lifca_pre
@@ -2270,9 +2001,6 @@ __global__ void ltp_kernel(Dev d) {
   }
 }
 
-// After each bath launch, on the bath stream: the next bath's step.
-__global__ void bath_tick_kernel(Dev d) { *d.bath_t = *d.bath_t + 1; }
-
 __global__ void end_step_kernel(Dev d) {
   *d.ovf_cnt = 0;
   d.heavy_cnt[0] = 0;
@@ -2378,8 +2106,6 @@ struct dpsnn_engine {
   double ktime[DPSNN_TIMING_SLOTS] = {};
   uint64_t klaunch[DPSNN_TIMING_SLOTS] = {};
   uint64_t launches = 0;               // kernels enqueued by dpsnn_step
-  std::vector<float> fix_vals;
-  std::vector<uint32_t> fix_keys, fix_bucket;
   uint32_t *h_pin = nullptr;          // pinned {flags, spike count} for per-step reads
   // spike lists are read on their own stream as soon as the compaction of
   // their step is done, while the rest of that step (and later ones) run
@@ -2432,38 +2158,27 @@ static int load_logf_fixup(dpsnn_engine *e) {
   if (!f) return dpsnn_fail(DPSNN_E_PARAM, "cannot open %s (built with the engine)", path.c_str());
   uint32_t n = 0;
   bool ok = fread(&n, 4, 1, f) == 1;
-  e->fix_keys.resize(n);
-  e->fix_vals.resize(n);
-  e->fix_bucket.resize(LOGF_FIX_NBUCKET);
-  ok = ok && fread(e->fix_keys.data(), 4, n, f) == n;
-  ok = ok && fread(e->fix_vals.data(), 4, n, f) == n;
-  ok = ok && fread(e->fix_bucket.data(), 4, LOGF_FIX_NBUCKET, f) == LOGF_FIX_NBUCKET;
+  std::vector<uint32_t> keys(n), vals(n), bucket(LOGF_FIX_NBUCKET);
+  ok = ok && fread(keys.data(), 4, n, f) == n;
+  ok = ok && fread(vals.data(), 4, n, f) == n;
+  ok = ok && fread(bucket.data(), 4, LOGF_FIX_NBUCKET, f) == LOGF_FIX_NBUCKET;
   fclose(f);
   if (!ok) return dpsnn_fail(DPSNN_E_PARAM, "truncated %s", path.c_str());
-  uint32_t *k; float *v; uint32_t *b;
-  DALLOC(k, n);
-  DALLOC(v, n);
-  DALLOC(b, LOGF_FIX_NBUCKET);
-  CK(cudaMemcpyAsync(k, e->fix_keys.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
-  CK(cudaMemcpyAsync(v, e->fix_vals.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
-  CK(cudaMemcpyAsync(b, e->fix_bucket.data(), 4ull * LOGF_FIX_NBUCKET, cudaMemcpyHostToDevice, e->stream));
-  e->d.fix.keys = k;
-  e->d.fix.vals = v;
-  e->d.fix.bucket = b;
-  e->d.fix.n = n;
   {
     const size_t words = ((size_t)(0x3F800000u - 0x30000000u) + 1 + 31) / 32;
     std::vector<uint32_t> bm(words, 0u);
-    for (uint32_t key : e->fix_keys)
+    for (uint32_t key : keys)
       if (key >= 0x30000000u && key <= 0x3F800000u) bm[(key - 0x30000000u) >> 5] |= 1u << ((key - 0x30000000u) & 31);
     uint32_t *dbm;
     DALLOC(dbm, words);
     CK(cudaMemcpyAsync(dbm, bm.data(), 4 * words, cudaMemcpyHostToDevice, e->stream));
     e->d.fix_bitmap = dbm;
-    // per result binade, the fix-up inputs' largest distance (ulps) from a
-    // rounding midpoint, with a margin for the device log's last bit
-    std::vector<float> near(256, -1.0f);
-    for (uint32_t key : e->fix_keys) {
+    // per result binade, the fix-up inputs' least distance from the float
+    // their logarithm rounds to (half an ulp at a midpoint), with a margin of
+    // 1e-3 ulp for the device log's last bits
+    std::vector<double> near(256, INFINITY);
+    for (uint32_t i = 0; i < n; i++) {
+      const uint32_t key = keys[i];
       if (key < 0x30000000u || key > 0x3F800000u) continue;
       float xf;
       memcpy(&xf, &key, 4);
@@ -2471,16 +2186,28 @@ static int load_logf_fixup(dpsnn_engine *e) {
       const float f = logf_cr_from(xf, y);
       uint32_t fb;
       memcpy(&fb, &f, 4);
+      // the kernels take a fix-up to be the float on the other side of the
+      // midpoint, as it is for any log with an error below one ulp
+      if (vals[i] != fb + (y < (double)f ? 1u : 0xFFFFFFFFu))
+        return dpsnn_fail(DPSNN_E_PARAM, "%s: logf is off by more than one ulp at 0x%08x", path.c_str(), key);
       const uint32_t E = (fb >> 23) & 0xFFu;
-      if ((fb & 0x7FFFFFu) == 0 || E <= 24) continue;   // always checked on the device
-      const double dist = 0.5 - fabs(y - (double)f) * ldexp(1.0, 150 - (int)E);
-      near[E] = std::max(near[E], (float)(dist + 1e-3));
+      if ((fb & 0x7FFFFFu) == 0) continue;   // always checked on the device
+      near[E] = std::min(near[E], fabs(y - (double)f) - ldexp(1e-3, (int)E - 150));
     }
-    float *dnear;
+    std::vector<double2> tab(LOG_TAB_N);
+    for (int k = 0; k < LOG_TAB_N; k++) {   // the logarithm that goes with the rounded 64/i
+      const double c = 64.0 / (LOG_TAB_0 + k);
+      tab[k] = make_double2(c, c == 1.0 ? 0.0 : -log_cr(c));
+    }
+    double *dnear;
+    double2 *dtab;
     DALLOC(dnear, 256);
-    CK(cudaMemcpyAsync(dnear, near.data(), 4 * 256, cudaMemcpyHostToDevice, e->stream));
+    DALLOC(dtab, LOG_TAB_N);
+    CK(cudaMemcpyAsync(dnear, near.data(), 8 * 256, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(dtab, tab.data(), sizeof(double2) * LOG_TAB_N, cudaMemcpyHostToDevice, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     e->d.fix_near = dnear;
+    e->d.log_tab = dtab;
   }
   return 0;
 }
@@ -2864,7 +2591,7 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   }
   DALLOC(d.heavy_cnt, 2);
   DALLOC(d.t, 1);
-  DALLOC(d.bath_t, 1);
+  DALLOC(d.bath_t, P);
   DALLOC(d.flags, 4);
   DALLOC(d.events, 1);
   init_neurons_kernel<<<(N + 255) / 256, 256, 0, e->stream>>>(d);
@@ -2882,12 +2609,9 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     }
     uint32_t mx_max = 0;
     for (uint32_t i = 0; i < N; i++) mx_max = std::max(mx_max, mx[i]);
-    // one 32-neuron chunk plus one neuron's look-ahead must fit in the draw ring
-    if (mx_max > BATH_MAX_EXT || 66ull * mx_max + 200 > BATH_RING)
+    if (mx_max > BATH_MAX_EXT)
       return dpsnn_fail(DPSNN_E_CAPACITY, "maxExternCurrentCount %u exceeds what the bath ring holds (%d)", mx_max,
-                        (BATH_RING - 200) / 66);
-    n.bath_need = mx_max;
-    CK(cudaMemcpyAsync(d.net, &n, sizeof n, cudaMemcpyHostToDevice, e->stream));
+                        BATH_MAX_EXT);
     DALLOC(d.bath_rank_base, P + 1);
     CK(cudaMemcpyAsync(d.bath_rank_base, base.data(), 8ull * (P + 1), cudaMemcpyHostToDevice, e->stream));
     for (int b = 0; b < 2; b++) {
@@ -2902,8 +2626,7 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     d.bath_cnt = e->bath_cnt2[0];
     // dynamics streams: SetRandomSeed(loc_h) (DPSNN_localNet_init.c:283).
     // Rank 0 continues its generation stream; others re-initialise.
-    std::vector<uint32_t> hist((size_t)P * 64, 0);
-    std::vector<uint64_t> produced(P, 0), pos(P, 1);
+    std::vector<uint32_t> hist((size_t)P * BATH_HIST);
     for (uint32_t h = 0; h < P; h++) {
       uint32_t h55[55];
       if (h == 0) {
@@ -2932,17 +2655,17 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
         g.inext = 0;
         r3_history(g, h55);
       }
-      // x[-55..-1] at ring positions (k-55) & 63
-      for (int k = 0; k < 55; k++) hist[(size_t)h * 64 + ((k - 55) & 63)] = h55[k];
+      // h55 is x[-55..-1].  The neurons' draws start at x[1]: the history is
+      // x[1-BATH_HIST..0], x[0] = x[-55] - x[-24] and the older ones by the
+      // recurrence backwards, x[k] = x[k+55] + x[k+31] (mod MBIG)
+      uint32_t *x = &hist[(size_t)h * BATH_HIST] + BATH_HIST - 1;   // x[0]
+      for (int k = 0; k < 55; k++) x[k - 55] = h55[k];
+      x[0] = x[-55] >= x[-24] ? x[-55] - x[-24] : x[-55] + MBIG - x[-24];
+      for (int k = -56; k > -BATH_HIST; k--) x[k] = (uint32_t)(((uint64_t)x[k + 55] + x[k + 31]) % MBIG);
     }
-    DALLOC(d.bath_hist, (size_t)P * 64);
-    DALLOC(d.bath_produced, P);
-    DALLOC(d.bath_pos, P);
-    DALLOC(d.draw_idx, (size_t)P * BATH_RING);
-    DALLOC(d.draw_lapse, (size_t)P * BATH_RING);
-    CK(cudaMemcpyAsync(d.bath_hist, hist.data(), 4ull * P * 64, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(d.bath_produced, produced.data(), 8ull * P, cudaMemcpyHostToDevice, e->stream));
-    CK(cudaMemcpyAsync(d.bath_pos, pos.data(), 8ull * P, cudaMemcpyHostToDevice, e->stream));
+    DALLOC(d.bath_hist, (size_t)P * BATH_HIST);
+    CK(cudaMemcpyAsync(d.bath_hist, hist.data(), 4ull * P * BATH_HIST, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaStreamSynchronize(e->stream));
   }
   int rc = load_logf_fixup(e);
   if (rc) return rc;
@@ -3103,9 +2826,8 @@ static void enqueue_bath(dpsnn_engine *e, uint32_t t) {
   db.bath_cnt = e->bath_cnt2[b];
   cudaStreamWaitEvent(e->bath_stream, e->ev_neuron[b], 0);
   timed_launch_begin(e, 2, e->bath_stream);
-  // the kernel reads its step from d.bath_t (baths are launched in step order)
+  // each rank's block keeps its step in d.bath_t (baths are launched in step order)
   bath_kernel<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
-  bath_tick_kernel<<<1, 1, 0, e->bath_stream>>>(db);
   timed_launch_end(e, 2);
   cudaEventRecord(e->ev_bath[b], e->bath_stream);
 }
@@ -3118,7 +2840,7 @@ static int enqueue_step(dpsnn_engine *e) {
     cudaStreamWaitEvent(e->bath_stream, e->ev_start, 0);
     enqueue_bath(e, t);
     e->bath_primed = true;
-    e->launches += 2;
+    e->launches++;
   }
   enqueue_bath(e, t + 1);
   if (e->d.stdp_log) {
@@ -3175,7 +2897,7 @@ static int enqueue_step(dpsnn_engine *e) {
     timed_launch_end(e, 4);
   }
   end_step_kernel<<<1, 1, 0, e->stream>>>(d);
-  e->launches += 11 + (e->hnet.stdp_on ? 2 : 0);
+  e->launches += 10 + (e->hnet.stdp_on ? 2 : 0);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return dpsnn_fail(DPSNN_E_CUDA, "kernel launch: %s", cudaGetErrorString(err));
   e->t_host++;

@@ -1,0 +1,38 @@
+"""The Poisson bath kernel at the sizes and rates where its rounds, segments
+and caps have edges, against the CPU restatement: nextBath (the sum of every
+lapse drawn) and the raster must be the same bits."""
+import numpy as np
+import pytest
+
+import dpsnn_oracle as O
+from tests.conftest import engine_module, netconfig
+
+pytestmark = pytest.mark.gpu
+E = engine_module()
+nc = netconfig()
+
+
+@pytest.mark.parametrize("n_exc, n_inh, ranks", [
+    (26, 13, 4),    # ranks of 65 neurons: segments of 16 and one neuron
+    (51, 26, 4),    # 128: one round of 8 full segments
+    (51, 27, 4),    # 129: a round and one neuron
+    (130, 41, 1),   # 1204: several rounds, a ragged end
+])
+# mean events per ms; the cap is ceil(20 * rate): 0.01 and 0.06 reach it (1 and
+# 2 events, then single draws that shift the pairs), 6.05 is the largest
+# supported (121)
+@pytest.mark.parametrize("rate", [0.01, 0.06, 0.5, 3.0, 6.05])
+def test_next_bath_and_raster_match_oracle(n_exc, n_inh, ranks, rate):
+    cfg = nc.cortical_grid(2, 2, n_exc_a=n_exc, n_exc_b=n_exc, n_inh=n_inh, p1=0.2, mu=0.6, nu_ext_hz=rate,
+                           total_ms=40, seed=5, glob_h=ranks)
+    eng, orc = E.Engine(cfg), O.OracleNet(cfg, 1)
+    for t in range(40):
+        eng.step(1)
+        ids, te = eng.spikes(t)
+        oi, ot = orc.step()
+        np.testing.assert_array_equal(ids, oi)
+        np.testing.assert_array_equal(te, ot)
+    st, so = eng.state(), orc.state()
+    for k in st:
+        np.testing.assert_array_equal(st[k], so[k], err_msg=k)
+    eng.close()
