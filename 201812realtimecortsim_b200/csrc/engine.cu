@@ -195,14 +195,20 @@ __device__ static inline uint32_t subpop_of(const NetConst *net, uint32_t in_cm)
 }
 
 // ------------------------------------------------------------------ generation
-// One thread walks one cortical module's neurons in order, consuming that
-// module's serial ran3 stream exactly as simpleCM_invokeIndivSynGenerators
-// (DPSNN_LIFCAcorticalModuleGen.cpp:62-220) does.  Modules are independent
-// streams (SetRandomSeed(module) at :96-107) except for NormDev's cached
-// value, which carries from one module to the next inside a rank; pass A runs
-// each module under both hypotheses for that cache (empty, or holding a value
-// that the module's first weight accepts) and pass B regenerates the chosen
-// one, writing synapses straight into their CSR slots.
+// A cortical module's neurons consume its serial ran3 stream in order
+// (simpleCM_invokeIndivSynGenerators, DPSNN_LIFCAcorticalModuleGen.cpp:62-220).
+// Modules are independent streams (SetRandomSeed(module) at :96-107) except
+// for NormDev's cached value, which carries from one module to the next
+// inside a rank.  Two forms:
+//  - where no weight can be rejected (below, and the rule in engine_build), a
+//    warp per module finds every neuron's position in the stream
+//    (gen_chain_kernel), and a warp per neuron then generates its synapses
+//    (gen_fill_kernel);
+//  - otherwise one thread walks one module (gen_kernel): a rejected weight
+//    draws again, so that a neuron's draws depend on its weights.  Pass A runs
+//    each module under both hypotheses for NormDev's cache (empty, or holding
+//    a value that the module's first weight accepts) and pass B regenerates
+//    the chosen one, writing synapses straight into their CSR slots.
 struct GenRecord {
   uint32_t nsyn;
   int32_t used_normdev, set_out, err;
@@ -233,7 +239,7 @@ __device__ static inline uint32_t empty_random_synapses(Ran3 &g, float pf, uint3
 #define DELAY_LEVEL_ERR 0xFFFFFFFFu   // level >= DSD__delayNum
 #define DELAY_RANGE_ERR 0xFFFFFFFEu   // delay beyond the pair's DMax
 
-__device__ static inline uint32_t random_delay_uni(const NetConst *net, Ran3 &g, uint32_t s, uint32_t t) {
+__device__ static inline uint32_t random_delay_uni(const NetConst *net, double u, uint32_t s, uint32_t t) {
   // getRandomDelay_UNI (DPSNN_LIFCAcorticalModuleGen.cpp:299-338)
   float outF, DMin, DMax, DelayMin, DelayMax, DelayStep, DelayNum;
   DMin = (float)net->DMin[s * DPSNN_MAX_SUBPOP + t];
@@ -246,7 +252,7 @@ __device__ static inline uint32_t random_delay_uni(const NetConst *net, Ran3 &g,
   DelayMin += DelayStep / 2;
   DMax = roundr2i((DMax - DelayMin) / DelayStep) * DelayStep + DelayMin;
   DMin = roundr2i((DMin - DelayMin) / DelayStep) * DelayStep + DelayMin;
-  outF = (float)((r3_rand(g) * (DMax - DMin) + DMin - DelayMin) / DelayStep);
+  outF = (float)((u * (DMax - DMin) + DMin - DelayMin) / DelayStep);
   (void)DelayMax;
   // the reference stops here: "delay level generated %f > %f max allowed
   // delay levels" (:322-326); the level goes back in the error argument
@@ -259,7 +265,7 @@ __device__ static inline uint32_t random_delay_uni(const NetConst *net, Ran3 &g,
 // getRandomDelay_EXP (DPSNN_LIFCAcorticalModuleGen.cpp:247-297), the
 // reference Makefile's default: a truncated exponential over [DMin, DMax);
 // DELAY_LEVEL_ERR / DELAY_RANGE_ERR where the reference stops with an error.
-__device__ static inline uint32_t random_delay_exp(const NetConst *net, Ran3 &g, uint32_t s, uint32_t t) {
+__device__ static inline uint32_t random_delay_exp(const NetConst *net, double u, uint32_t s, uint32_t t) {
   float outfuncF, DMin, DMax, DelayMin, DelayMax, DelayStep, DelayNum;
   const float InvLogTN = net->inv_log_tn;
   DMin = (float)net->DMin[s * DPSNN_MAX_SUBPOP + t];
@@ -273,13 +279,32 @@ __device__ static inline uint32_t random_delay_exp(const NetConst *net, Ran3 &g,
   DMax = roundr2i((DMax - DelayMin) / DelayStep) * DelayStep + DelayMin;
   DMin = roundr2i((DMin - DelayMin) / DelayStep) * DelayStep + DelayMin;
   outfuncF = (float)((((double)DMin + (double)(DMax - DMin - DelayStep) *
-                       log_cr(1.0 - r3_rand(g) * (1.0 - 0.05)) * (double)InvLogTN) -
+                       log_cr(1.0 - u * (1.0 - 0.05)) * (double)InvLogTN) -
                       (double)DelayMin) / (double)DelayStep);
   if (outfuncF >= DelayNum) return DELAY_LEVEL_ERR;
   const uint32_t outfunc = roundr2i(outfuncF * DelayStep);
   if (outfunc >= net->DMax[s * DPSNN_MAX_SUBPOP + t]) return DELAY_RANGE_ERR;
   (void)DelayMax;
   return outfunc;
+}
+
+// The external bath rate of one neuron
+// (ModuleGen.cpp:201-211, LIFCAconnectome.cpp:871-887).
+__device__ static inline void gen_bath_rate(const NetConst *net, const uint32_t *__restrict__ bath_tmpl, uint32_t ssub,
+                                            uint32_t cfx, uint32_t cfy, double &inv_nu, uint32_t &max_ext) {
+  const float nu = (float)net->NuExt[ssub];
+  uint32_t bx = cfx, by = cfy;
+  if (bx >= net->cfx / 2) bx = 0u - (bx - net->cfx + 1u);   // unsigned, as the reference computes it
+  if (by >= net->cfy / 2) by = 0u - (by - net->cfy + 1u);
+  if (bx >= net->stencil_dim) bx = net->stencil_dim - 1;
+  if (by >= net->stencil_dim) by = net->stencil_dim - 1;
+  const float cext = (float)bath_tmpl[bx * net->stencil_dim + by];
+  inv_nu = 0;
+  max_ext = 0;
+  if (cext != 0) {
+    inv_nu = 1000.0 / (nu * cext);
+    max_ext = (uint32_t)ceil(20 / inv_nu);
+  }
 }
 
 #define GEN_THREADS 16          // generation streams per block
@@ -359,7 +384,8 @@ __global__ void gen_kernel(const NetConst *__restrict__ net, const float *__rest
     for (uint32_t j = 0; j < tot; j++) {
       uint32_t tg = tl[j];
       uint32_t tsub = subpop_of(net, tg % npcm);
-      uint32_t delay = net->delay_exp ? random_delay_exp(net, g, ssub, tsub) : random_delay_uni(net, g, ssub, tsub);
+      const double u = r3_rand(g);
+      uint32_t delay = net->delay_exp ? random_delay_exp(net, u, ssub, tsub) : random_delay_uni(net, u, ssub, tsub);
       if (delay == DELAY_LEVEL_ERR) { R->err = GEN_ERR_DELAY_LEVEL; R->err_arg = gi; return; }
       if (delay == DELAY_RANGE_ERR) { R->err = GEN_ERR_DELAY_RANGE; R->err_arg = gi; return; }
       if (delay >= D) { R->err = GEN_ERR_DELAY; R->err_arg = delay; return; }
@@ -392,22 +418,7 @@ __global__ void gen_kernel(const NetConst *__restrict__ net, const float *__rest
       uint16_t *co = cnt_out + ((size_t)hyp * N + gi) * D;
       for (uint32_t d = 0; d < D; d++) co[d] = cnt[d];
     } else {
-      // external bath rate (ModuleGen.cpp:201-211, LIFCAconnectome.cpp:871-887)
-      float nu = (float)net->NuExt[ssub];
-      uint32_t bx = cfx, by = cfy;
-      if (bx >= net->cfx / 2) bx = 0u - (bx - net->cfx + 1u);   // unsigned, as the reference computes it
-      if (by >= net->cfy / 2) by = 0u - (by - net->cfy + 1u);
-      if (bx >= net->stencil_dim) bx = net->stencil_dim - 1;
-      if (by >= net->stencil_dim) by = net->stencil_dim - 1;
-      float cext = (float)bath_tmpl[bx * net->stencil_dim + by];
-      if (cext != 0) {
-        double inv = 1000.0 / (nu * cext);
-        inv_nu[gi] = inv;
-        max_ext[gi] = (uint32_t)ceil(20 / inv);
-      } else {
-        inv_nu[gi] = 0;
-        max_ext[gi] = 0;
-      }
+      gen_bath_rate(net, bath_tmpl, ssub, cfx, cfy, inv_nu[gi], max_ext[gi]);
     }
   }
   R->nsyn = nsyn;
@@ -415,6 +426,460 @@ __global__ void gen_kernel(const NetConst *__restrict__ net, const float *__rest
   R->set_out = ns.set;
   R->cache_out = ns.cache;
   r3_history(g, R->hist);
+}
+
+// ---- the warp form
+// One (target sub-population, stencil cell) of a source sub-population with
+// a connection probability, in the reference's order.
+struct GenRow {
+  int32_t dx, dy;
+  uint32_t ts, tab;   // tab: its probability's table
+};
+// A probability's table of getEmptyRandomSynapses (DPSNN_LIFCAconnectome.cpp:1079-1133):
+// C[n] = the sum of the reference's first n terms, n = 1 .. len, so that a
+// draw r gives the first n with C[n] >= r, len + 1 if there is none.
+struct GenTab {
+  float pf, inv_log2q;   // 1 / log2(1 - pf): the first guess at n
+  uint32_t len;
+  uint32_t off;          // C[1] at gen_c[off]
+};
+__global__ void gen_tab_kernel(const GenTab *__restrict__ tab, uint32_t n, double *__restrict__ gen_c) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double connectivity = (double)tab[i].pf;
+  double P = connectivity, C = P;
+  for (uint32_t k = 0; k < tab[i].len; k++) {
+    gen_c[tab[i].off + k] = C;
+    P *= 1 - connectivity;
+    C += P;
+  }
+}
+
+// A ran3 stream in a warp's shared ring: draw n at n % GEN_RING, drawn up to
+// `end`, the 220 draws before it kept.
+#define GEN_RING 512
+#define GEN_HIST 55
+struct GenStream {
+  uint32_t *x;
+  uint32_t end;
+  __device__ uint32_t at(uint32_t n) const { return x[n % GEN_RING]; }
+  __device__ double u(uint32_t n) const { return (__hiloint2double(0x43300000, (int)at(n)) - 0x1p52) * (1.0 / (double)MBIG); }
+};
+// The draws before n0 from their last 55 (already at n0-55 .. n0-1): the
+// recurrence backwards, x[k] = x[k+55] + x[k+31] (mod MBIG), 31 at a time.
+__device__ static inline void gen_backfill(GenStream &g, uint32_t n0, uint32_t lane) {
+  __syncwarp();
+  for (uint32_t hi = n0 - GEN_HIST; hi > n0 - 224; hi -= 31) {
+    const uint32_t k = hi - 1 - lane;
+    uint32_t v = g.at(k + 55) + g.at(k + 31);
+    if (v >= MBIG) v -= MBIG;
+    __syncwarp();
+    if (lane < 31) g.x[k % GEN_RING] = v;
+    __syncwarp();
+  }
+  g.end = n0;
+}
+// Draws up to n: x[n] = x[n-96] - 4 x[n-127] + 6 x[n-158] - 4 x[n-189] + x[n-220] (bath_kernel), 96 at a time.
+__device__ static inline void gen_draw(GenStream &g, uint32_t n, uint32_t lane) {
+  while ((int32_t)(n - g.end) > 0) {
+    uint32_t x[3];
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+      const uint32_t k = g.end + lane + 32 * v;
+      const int32_t x3 = 2 * (int32_t)g.at(k - 158);
+      int32_t y = (int32_t)(g.at(k - 96) + g.at(k - 220)) - x3, z = (int32_t)(g.at(k - 127) + g.at(k - 189)) - x3;
+      if (y < 0) y += MBIG;
+      if (y < 0) y += MBIG;
+      if (y >= MBIG) y -= MBIG;
+      if (z < 0) z += MBIG;
+      if (z < 0) z += MBIG;
+      z = 2 * (z >= MBIG ? z - MBIG : z);
+      if (z >= MBIG) z -= MBIG;
+      y -= 2 * z;
+      if (y < 0) y += MBIG;
+      if (y < 0) y += MBIG;
+      x[v] = (uint32_t)y;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < 3; v++) g.x[(g.end + lane + 32 * v) % GEN_RING] = x[v];
+    __syncwarp();
+    g.end += 96;
+  }
+}
+
+// getEmptyRandomSynapses for raw draw mj (u as ran3 returns it): a guess from
+// the logarithm, then the table decides.
+__device__ static inline uint32_t gen_skip(const GenTab &tb, const double *__restrict__ gen_c, uint32_t mj, double u) {
+  int n = (int)ceilf(__log2f((float)(MBIG - mj) * 1e-9f) * tb.inv_log2q);
+  const int len = (int)tb.len;
+  n = max(1, min(n, len + 1));
+  const double *C = gen_c + tb.off - 1;
+  while (n <= len && __ldg(&C[n]) < u) n++;
+  while (n > 1 && __ldg(&C[n - 1]) >= u) n--;
+  return (uint32_t)n;
+}
+
+// One row's targets from draw pos on (K draws per lane at once): `emit`
+// receives (index in the row's list, index in the sub-population).  Returns
+// their number; pos moves past the row's draws.
+template <int K, typename Emit>
+__device__ static inline uint32_t gen_row(GenStream &g, const GenTab &tb, const double *__restrict__ gen_c, uint32_t count,
+                                          uint32_t &pos, uint32_t lane, const Emit &emit) {
+  int32_t at = -1;
+  uint32_t tot = 0;
+  for (;;) {
+    gen_draw(g, pos + 32 * K, lane);
+    int32_t s[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t n = pos + K * lane + k;
+      s[k] = (int32_t)gen_skip(tb, gen_c, g.at(n), g.u(n));
+    }
+#pragma unroll
+    for (int k = 1; k < K; k++) s[k] += s[k - 1];
+    int32_t incl = s[K - 1];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= (uint32_t)o) incl += y;
+    }
+    const int32_t base = at + incl - s[K - 1];
+    uint32_t v = 0;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (base + s[k] < (int32_t)count) {
+        emit(tot + K * lane + k, (uint32_t)(base + s[k]));
+        v++;
+      }
+    const uint32_t full = __popc(__ballot_sync(0xffffffffu, v == K));   // the lanes before the row's end
+    if (full == 32) {
+      tot += 32 * K;
+      pos += 32 * K;
+      at = __shfl_sync(0xffffffffu, base + s[K - 1], 31);
+      continue;
+    }
+    const uint32_t last = full * K + __shfl_sync(0xffffffffu, v, full);
+    pos += last + 1;
+    return tot + last;
+  }
+}
+template <typename Emit>
+__device__ static inline uint32_t gen_row(GenStream &g, const GenTab &tb, const double *__restrict__ gen_c, uint32_t count,
+                                          uint32_t &pos, uint32_t lane, const Emit &emit) {
+  return tb.pf * (float)count > 48.0f ? gen_row<4>(g, tb, gen_c, count, pos, lane, emit)
+                                      : gen_row<1>(g, tb, gen_c, count, pos, lane, emit);
+}
+
+// The weights' draws.  Without rejected weights two targets in a row draw
+// one delay, pairs of uniforms until one lies in the unit circle (NormDev,
+// randdev.c:584-606; its second value is cached) and the other's delay: in
+// steps of two draws from the first target's, pair g is at draw 1 + 2 g, and
+// after an accepted pair g the next unit starts at step g + 2.  So of a run
+// of acceptable pairs every other one is accepted, starting with the first.
+// gen_pairs: of the 64 pairs from draw p on, which are accepted; carry: the
+// pair before them was (and the first of them is skipped).
+__device__ static inline uint64_t gen_pairs(const GenStream &g, uint32_t p, bool carry, uint32_t lane) {
+  bool ok[2];
+#pragma unroll
+  for (int v = 0; v < 2; v++) {
+    const uint32_t n = p + 2 * (lane + 32 * v);
+    const double v1 = 2.0 * g.u(n) - 1.0, v2 = 2.0 * g.u(n + 1) - 1.0, r = v1 * v1 + v2 * v2;
+    ok[v] = !(r >= 1.0 || r == 0.0);
+  }
+  const uint64_t m0 = __ballot_sync(0xffffffffu, ok[0]) | ((uint64_t)__ballot_sync(0xffffffffu, ok[1]) << 32);
+  const uint64_t m = m0 & ~(uint64_t)carry, E = 0x5555555555555555ull;
+  // adding a run's first bit clears the run: the runs that start at even positions, then the others
+  const uint64_t even = m & ~(m + (m & ~(m << 1) & E));
+  return (even & E) | (m & ~even & ~E);
+}
+
+// What gen_chain_kernel leaves of a module's stream (2 per module: NormDev's
+// cache empty, or full, as the module starts).
+struct GenChain {
+  uint64_t nsyn;
+  uint32_t err, err_arg;
+  uint32_t set_out, c_out[2];   // cache at the end, and the pair of draws it comes from
+  uint32_t hist[GEN_HIST];
+};
+// Per neuron and hypothesis: the draws before its first, whether NormDev's
+// cache is full (2: from before the module), and the pair it comes from.
+struct GenStart {
+  uint32_t hist[GEN_HIST];
+  uint32_t set, c[2];
+};
+
+// A warp per stream: every neuron's first draw and number of synapses.
+// What bounds it: the serial chain of a module's neurons, about 40 rows and 20
+// windows of pairs each; a warp does 32 or 128 draws of a row, or 64 pairs,
+// per step.  Measured: 20 ms for a module of 1250 neurons (16 us per neuron),
+// 40 ms for the 576 modules of the 24x24 network under both hypotheses; a
+// thread per module took 2 s per pass, and two passes.
+__global__ void __launch_bounds__(32) gen_chain_kernel(const NetConst *__restrict__ net, const GenRow *__restrict__ rows,
+                                                       const uint32_t *__restrict__ row_off, const GenTab *__restrict__ tabs,
+                                                       const double *__restrict__ gen_c, GenChain *chain,
+                                                       GenStart *__restrict__ start, uint32_t *__restrict__ tot_out) {
+  __shared__ uint32_t ring[GEN_RING];
+  const uint32_t lane = threadIdx.x, m = blockIdx.x >> 1, hyp = blockIdx.x & 1;
+  GenChain *R = &chain[blockIdx.x];
+  if (hyp && m % net->mods_per_rank == 0) return;   // a rank starts with an empty cache
+  const uint32_t N = net->N, npcm = net->npcm, cfy = m / net->cfx, cfx = m % net->cfx, n0 = 256;
+  GenStream g{ring, n0};
+  if (lane == 0) {
+    Ran3 r;
+    r.iff = 0;
+    r.idum = 0;
+    r.inext = r.inextp = 0;
+    if (m % net->mods_per_rank == 0) r3_seed(r, (int32_t)net->global_seed);  // localNet_init.c:119
+    r3_seed(r, (int32_t)m);  // module start (ModuleGen.cpp:96-107); m==0 does not re-initialise
+    r3_history(r, ring + n0 - GEN_HIST);
+  }
+  gen_backfill(g, n0, lane);
+  uint32_t pos = n0, set = hyp ? 2u : 0u, c0 = 0, c1 = 0;
+  uint64_t nsyn = 0;
+  for (uint32_t k = 0; k < npcm; k++) {
+    const uint32_t ssub = subpop_of(net, k), gi = m * npcm + k;
+    GenStart &S = start[(size_t)hyp * N + gi];
+    for (uint32_t i = lane; i < GEN_HIST; i += 32) S.hist[i] = g.at(pos - GEN_HIST + i);
+    if (lane == 0) {
+      S.set = set;
+      S.c[0] = c0;
+      S.c[1] = c1;
+    }
+    uint32_t tot = 0;
+    for (uint32_t i = row_off[ssub]; i < row_off[ssub + 1]; i++) {
+      const GenRow w = rows[i];
+      const int32_t nx = (int32_t)cfx + w.dx, ny = (int32_t)cfy + w.dy;
+      if (nx < 0 || nx >= (int32_t)net->cfx || ny < 0 || ny >= (int32_t)net->cfy) continue;
+      tot += gen_row(g, tabs[w.tab], gen_c, net->count[w.ts], pos, lane, [](uint32_t, uint32_t) {});
+      if (tot >= MAX_SYN_PER_NEURON) {
+        if (lane == 0) {
+          R->err = GEN_ERR_TOO_MANY;
+          R->err_arg = gi;
+        }
+        return;
+      }
+    }
+    if (lane == 0) tot_out[(size_t)hyp * N + gi] = tot;
+    nsyn += tot;
+    uint32_t rem = tot;
+    if (rem && set) {   // the first target's weight comes from the cache
+      set = 0;
+      pos++;
+      rem--;
+    }
+    uint32_t units = (rem + 1) / 2;
+    bool carry = false;
+    for (uint32_t p = pos; units; p += 128) {
+      gen_draw(g, p + 1 + 128, lane);
+      uint64_t acc = gen_pairs(g, p + 1, carry, lane);
+      const uint32_t cnt = __popcll(acc);
+      carry = acc >> 63;
+      if (cnt < units) {
+        units -= cnt;
+        continue;
+      }
+      // the last unit's pair: the units-th set bit
+      uint32_t at = 0, want = units;
+      for (uint32_t w = 32; w > 0; w >>= 1) {
+        const uint32_t c = __popcll(acc & ((1ull << w) - 1));
+        if (c < want) {
+          want -= c;
+          acc >>= w;
+          at += w;
+        }
+      }
+      pos = p + 2 * at + ((rem & 1) ? 3 : 4);
+      if (rem & 1) {
+        set = 1;
+        c0 = g.at(p + 1 + 2 * at);
+        c1 = g.at(p + 2 + 2 * at);
+      }
+      units = 0;
+    }
+    gen_draw(g, pos, lane);
+  }
+  for (uint32_t i = lane; i < GEN_HIST; i += 32) R->hist[i] = g.at(pos - GEN_HIST + i);
+  if (lane == 0) {
+    R->nsyn = nsyn;
+    R->set_out = set;
+    R->c_out[0] = c0;
+    R->c_out[1] = c1;
+  }
+}
+
+#define GEN_FILL_WARPS 4
+#define GEN_FILL_LIST 1536      // a neuron's synapses held in shared memory; more in the warp's global scratch
+struct GenFillWarp {
+  uint32_t ring[GEN_RING];
+  uint32_t tg[GEN_FILL_LIST];
+  int16_t w[GEN_FILL_LIST];
+  uint8_t dl[GEN_FILL_LIST];
+  uint32_t cnt[RING_SLOTS + 1];
+  uint8_t pair[32];
+};
+struct GenFillScratch {   // per warp
+  uint32_t tg[MAX_SYN_PER_NEURON];
+  int16_t w[MAX_SYN_PER_NEURON];
+  uint8_t dl[MAX_SYN_PER_NEURON];
+};
+
+// One synapse's delay and weight from its draws; GEN_ERR_* where the
+// reference stops.
+__device__ static inline uint32_t gen_synapse(const NetConst *net, uint32_t ssub, uint32_t tsub, double ud, double z,
+                                              uint32_t &delay, int16_t &w) {
+  delay = net->delay_exp ? random_delay_exp(net, ud, ssub, tsub) : random_delay_uni(net, ud, ssub, tsub);
+  if (delay == DELAY_LEVEL_ERR) return GEN_ERR_DELAY_LEVEL;
+  if (delay == DELAY_RANGE_ERR) return GEN_ERR_DELAY_RANGE;
+  if (delay >= net->D) return GEN_ERR_DELAY;
+  const float mean = (float)net->J[ssub * DPSNN_MAX_SUBPOP + tsub];
+  const float sigma = (float)(net->DJ[ssub * DPSNN_MAX_SUBPOP + tsub] * (double)mean);
+  if (mean == 0.0f) return GEN_ERR_ZERO_MEAN;
+  const float wf = (float)(mean + z * sigma);
+  if ((wf < net->min_w) || (wf > (-net->min_w))) return GEN_ERR_WEIGHT_RANGE;
+  w = (int16_t)(wf * net->f2w);
+  return 0;
+}
+
+// A warp per neuron: its targets, delays and weights from its first draw on
+// (in shared memory), then its CSR row, sorted by delay and in generation
+// order within one.  What bounds it: issue slots, the correctly rounded log
+// of a pair's radius above all, which 28 of 32 lanes do at a time.  Measured:
+// 37 ms for the 0.81 G synapses of the 24x24 network (a row's 1125 synapses in
+// about 120 us of a warp's time, 16 warps per SM).
+__global__ void __launch_bounds__(32 * GEN_FILL_WARPS)
+    gen_fill_kernel(const NetConst *__restrict__ net, const GenRow *__restrict__ rows, const uint32_t *__restrict__ row_off,
+                    const GenTab *__restrict__ tabs, const double *__restrict__ gen_c, const GenStart *__restrict__ start,
+                    const int32_t *__restrict__ hyp, const uint2 *__restrict__ mod_cache,
+                    const uint64_t *__restrict__ row_ptr, uint16_t *__restrict__ sub_off, uint32_t *__restrict__ post,
+                    int16_t *__restrict__ w16, GenFillScratch *scratch, unsigned long long *err,
+                    const uint32_t *__restrict__ bath_tmpl, double *__restrict__ inv_nu, uint32_t *__restrict__ max_ext,
+                    uint8_t *__restrict__ sub) {
+  extern __shared__ __align__(16) unsigned char gen_fill_raw[];
+  const uint32_t lane = threadIdx.x & 31, wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  GenFillWarp &s = reinterpret_cast<GenFillWarp *>(gen_fill_raw)[threadIdx.x >> 5];
+  const uint32_t N = net->N, D = net->D, npcm = net->npcm, n0 = 256;
+  for (uint32_t gi = wid; gi < N; gi += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t m = gi / npcm, cfy = m / net->cfx, cfx = m % net->cfx, ssub = subpop_of(net, gi % npcm);
+    const GenStart &S = start[(size_t)hyp[m] * N + gi];
+    const uint64_t row = row_ptr[gi];
+    const uint32_t tot = (uint32_t)(row_ptr[gi + 1] - row);
+    const bool big = tot > GEN_FILL_LIST;   // scratch is there when a neuron has that many
+    uint32_t *tg = big ? scratch[wid].tg : s.tg;
+    int16_t *wl = big ? scratch[wid].w : s.w;
+    uint8_t *dl = big ? scratch[wid].dl : s.dl;
+    GenStream g{s.ring, n0};
+    for (uint32_t i = lane; i < GEN_HIST; i += 32) s.ring[n0 - GEN_HIST + i] = S.hist[i];
+    for (uint32_t i = lane; i <= D; i += 32) s.cnt[i] = 0;
+    gen_backfill(g, n0, lane);
+    // targets, with their sub-population in the top bits (a network has fewer than 2^25 neurons)
+    uint32_t pos = n0, k0 = 0;
+    for (uint32_t i = row_off[ssub]; i < row_off[ssub + 1]; i++) {
+      const GenRow w = rows[i];
+      const int32_t nx = (int32_t)cfx + w.dx, ny = (int32_t)cfy + w.dy;
+      if (nx < 0 || nx >= (int32_t)net->cfx || ny < 0 || ny >= (int32_t)net->cfy) continue;
+      const uint32_t first = net->offset[w.ts] + (uint32_t)nx * npcm + (uint32_t)ny * npcm * net->cfx, top = w.ts << 25;
+      k0 += gen_row(g, tabs[w.tab], gen_c, net->count[w.ts], pos, lane, [&](uint32_t k, uint32_t at) {
+        if (k0 + k < tot) tg[k0 + k] = top | (first + at);
+      });
+    }
+    __syncwarp();
+    auto synapse = [&](uint32_t k, double ud, double z) {
+      uint32_t delay = 0;
+      int16_t w = 0;
+      const uint32_t e = gen_synapse(net, ssub, tg[k] >> 25, ud, z, delay, w);
+      if (e) {
+        atomicMin(err, ((unsigned long long)gi << 39) | ((unsigned long long)k << 26) | ((unsigned long long)e << 22) |
+                           min(e == GEN_ERR_DELAY ? delay : 0u, 0x3FFFFFu));
+        delay = 0;
+      }
+      dl[k] = (uint8_t)delay;
+      wl[k] = w;
+      atomicAdd(&s.cnt[delay], 1u);
+    };
+    auto polar = [&](uint32_t a, uint32_t b, double &z2, double &z1) {   // NormDev of the pair of draws (a, b)
+      const double v1 = 2.0 * ((double)a * (1.0 / (double)MBIG)) - 1.0;
+      const double v2 = 2.0 * ((double)b * (1.0 / (double)MBIG)) - 1.0;
+      const double r = v1 * v1 + v2 * v2, fac = sqrt(-2.0 * log_cr(r) / r);
+      z1 = v1 * fac;
+      z2 = v2 * fac;
+    };
+    uint32_t done = 0;
+    if (tot && S.set) {   // the first target's weight comes from the cache
+      if (lane == 0) {
+        double z2, z1;
+        if (S.set == 2) polar(mod_cache[m].x, mod_cache[m].y, z2, z1);
+        else polar(S.c[0], S.c[1], z2, z1);
+        synapse(0, g.u(pos), z1);
+      }
+      pos++;
+      done = 1;
+    }
+    bool carry = false;
+    int32_t prev = -2;   // pair of the last unit, from this window's first: the next unit starts two on
+    for (uint32_t p = pos; done < tot; p += 128) {
+      gen_draw(g, p + 130, lane);   // the last pair's unit ends with the draw after it
+      const uint64_t acc = gen_pairs(g, p + 1, carry, lane);
+      carry = acc >> 63;
+      // the window's accepted pairs (at most 32, no two adjacent), a lane each
+#pragma unroll
+      for (int v = 0; v < 2; v++) {
+        const uint32_t b = lane + 32 * v;
+        if ((acc >> b) & 1ull) s.pair[__popcll(acc & ((1ull << b) - 1))] = (uint8_t)b;
+      }
+      __syncwarp();
+      const uint32_t cnt = __popcll(acc), k = done + 2 * lane;
+      if (lane < cnt && k < tot) {
+        const int32_t pr = s.pair[lane], before = lane ? (int32_t)s.pair[lane - 1] : prev;
+        double z2, z1;
+        polar(g.at(p + 1 + 2 * pr), g.at(p + 2 + 2 * pr), z2, z1);
+        synapse(k, g.u(p + 2 * (before + 2)), z2);
+        if (k + 1 < tot) synapse(k + 1, g.u(p + 2 * pr + 3), z1);
+      }
+      prev = (cnt ? (int32_t)s.pair[cnt - 1] : prev) - 64;
+      done += 2 * cnt;
+      __syncwarp();
+    }
+    __syncwarp();
+    // offsets of the delays, then the row: each synapse after those of its
+    // delay generated before it
+    uint32_t acc = 0;
+    for (uint32_t d0 = 0; d0 <= D; d0 += 32) {
+      const uint32_t d = d0 + lane, c = d < D ? s.cnt[d] : 0u;
+      uint32_t incl = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+      }
+      if (d <= D) {
+        s.cnt[d] = acc + incl - c;
+        sub_off[(size_t)gi * (D + 1) + d] = (uint16_t)(acc + incl - c);
+      }
+      acc += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    __syncwarp();
+    for (uint32_t k = lane; k - lane < tot; k += 32) {
+      const uint32_t d = k < tot ? dl[k] : 0xFFu;
+      const uint32_t same = __match_any_sync(0xffffffffu, d), before = __popc(same & ((1u << lane) - 1));
+      uint32_t at = 0;
+      if (k < tot) at = s.cnt[d] + before;
+      __syncwarp();
+      if (k < tot) {
+        if (before == 0) s.cnt[d] += __popc(same);
+        post[row + at] = tg[k] & ((1u << 25) - 1);
+        w16[row + at] = wl[k];
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      double inv;
+      uint32_t mx;
+      gen_bath_rate(net, bath_tmpl, ssub, cfx, cfy, inv, mx);
+      inv_nu[gi] = inv;
+      max_ext[gi] = mx;
+      sub[gi] = (uint8_t)ssub;
+    }
+    __syncwarp();
+  }
 }
 
 // ------------------------------------------------------------------ step kernels
@@ -2274,6 +2739,8 @@ static int set_kernel_attributes(int device) {
   if ((int)done.size() <= device) done.resize(device + 1, 0);
   if (done[device]) return 0;
   CK(cudaFuncSetAttribute(gen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM));
+  CK(cudaFuncSetAttribute(gen_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          (int)(GEN_FILL_WARPS * sizeof(GenFillWarp))));
   CK(cudaFuncSetAttribute(bath_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BathSmem)));
   // the bath's blocks stay resident for most of a step: with the largest
   // shared-memory carveout, the SMs that hold two of them still have room for
@@ -2281,6 +2748,236 @@ static int set_kernel_attributes(int device) {
   CK(cudaFuncSetAttribute(bath_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                           (int)cudaSharedmemCarveoutMaxShared));
   done[device] = 1;
+  return 0;
+}
+
+// ---- synapse generation, host side
+static int gen_error(uint32_t err, uint32_t arg) {
+  const char *what[] = {"", "too many synapses generated for neuron", "synaptic weight out of minSynWeight_f range",
+                        "connection probability in (0,1e-5] is not supported", "delay >= env_D",
+                        "zero mean synaptic efficacy",
+                        "ERROR: delay level generated beyond the 80 max allowed delay levels, source neuron",
+                        "ERROR: delay generated beyond the pair's DMax, source neuron"};
+  return dpsnn_fail(DPSNN_E_MODEL, "synapse generation: %s (%u)", what[err], arg);
+}
+
+struct GenPlan {
+  std::vector<GenRow> rows;
+  std::vector<uint32_t> row_off;   // [nsub + 1] by source sub-population
+  std::vector<GenTab> tabs;
+  size_t c_len = 0;
+};
+#define GEN_TABS_MAX 4096   // distinct probabilities (a 10 x 10 stencil has at most 100 per pair)
+
+// The warp form's plan; false where the thread form has to do: a weight may
+// be rejected (NormDev's values are below sqrt(-2 ln 4e-18) = 8.96, so with
+// sigma under 1/8.97 of the mean none is), a probability that the reference
+// does not take, or more distinct probabilities than tables.
+static bool gen_plan(const NetConst &n, const std::vector<float> &prob, GenPlan &g) {
+  const uint32_t st = n.stencil, M = n.max_mod;
+  g.row_off.push_back(0);
+  for (uint32_t s = 0; s < n.nsub; s++) {
+    for (uint32_t t = 0; t < n.nsub; t++)
+      for (uint32_t x = 0; x < st; x++)
+        for (uint32_t y = 0; y < st; y++) {
+          const float pf = prob[(((size_t)s * DPSNN_MAX_SUBPOP + t) * st + x) * st + y];
+          if (!(pf > 0)) continue;
+          if (!(pf > 0.00001f) || !(8.97 * fabs(n.DJ[s * DPSNN_MAX_SUBPOP + t]) <= 0.999)) return false;
+          uint32_t k = 0;
+          while (k < g.tabs.size() && g.tabs[k].pf != pf) k++;
+          if (k == g.tabs.size()) {
+            if (k == GEN_TABS_MAX) return false;
+            g.tabs.push_back(GenTab{pf, (float)(1.0 / log2(1.0 - (double)pf)), 0, 0});
+          }
+          g.tabs[k].len = std::max(g.tabs[k].len, n.count[t] + 1);
+          g.rows.push_back(GenRow{(int32_t)x - (int32_t)M, (int32_t)y - (int32_t)M, t, k});
+        }
+    g.row_off.push_back((uint32_t)g.rows.size());
+  }
+  for (GenTab &tb : g.tabs) {
+    tb.off = (uint32_t)g.c_len;
+    g.c_len += tb.len;
+  }
+  return g.c_len < (1u << 28);
+}
+
+// The CSR rows from the neurons' synapse counts, and the connectome's arrays.
+static int alloc_rows(dpsnn_engine *e, const std::vector<uint32_t> &len) {
+  const uint32_t N = e->hnet.N;
+  std::vector<uint64_t> hrow(N + 1);
+  hrow[0] = 0;
+  for (uint32_t i = 0; i < N; i++) hrow[i + 1] = hrow[i] + len[i];
+  e->S = hrow[N];
+  DALLOC(e->d.row_ptr, N + 1);
+  CK(cudaMemcpyAsync(e->d.row_ptr, hrow.data(), 8ull * (N + 1), cudaMemcpyHostToDevice, e->stream));
+  DALLOC(e->d.post, e->S);
+  DALLOC(e->d.w16, e->S);
+  CK(cudaStreamSynchronize(e->stream));
+  return 0;
+}
+
+static int generate_by_warps(dpsnn_engine *e, const GenPlan &g, const uint32_t *bath_tmpl, uint32_t *hist0) {
+  const NetConst &n = e->hnet;
+  Dev &d = e->d;
+  const uint32_t N = n.N, nmod = n.nmod, hyps = n.mods_per_rank > 1 ? 2 : 1;
+  GenRow *rows;
+  GenTab *tabs;
+  GenChain *chain;
+  GenStart *start;
+  double *gen_c;
+  uint32_t *row_off, *tot;
+  TALLOC(rows, g.rows.size());
+  TALLOC(tabs, g.tabs.size());
+  TALLOC(gen_c, g.c_len);
+  TALLOC(row_off, n.nsub + 1);
+  TALLOC(chain, 2 * nmod);
+  TALLOC(start, (size_t)hyps * N);
+  TALLOC(tot, (size_t)hyps * N);
+  CK(cudaMemcpyAsync(rows, g.rows.data(), sizeof(GenRow) * g.rows.size(), cudaMemcpyHostToDevice, e->stream));
+  CK(cudaMemcpyAsync(tabs, g.tabs.data(), sizeof(GenTab) * g.tabs.size(), cudaMemcpyHostToDevice, e->stream));
+  CK(cudaMemcpyAsync(row_off, g.row_off.data(), 4 * g.row_off.size(), cudaMemcpyHostToDevice, e->stream));
+  if (!g.tabs.empty())
+    gen_tab_kernel<<<((uint32_t)g.tabs.size() + 31) / 32, 32, 0, e->stream>>>(tabs, (uint32_t)g.tabs.size(), gen_c);
+  gen_chain_kernel<<<2 * nmod, 32, 0, e->stream>>>(d.net, rows, row_off, tabs, gen_c, chain, start, tot);
+  CK(cudaGetLastError());
+  std::vector<GenChain> rec(2 * nmod);
+  std::vector<uint32_t> htot((size_t)hyps * N);
+  CK(cudaMemcpyAsync(rec.data(), chain, sizeof(GenChain) * 2 * nmod, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaMemcpyAsync(htot.data(), tot, 4 * htot.size(), cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  // NormDev's cache from module to module of a rank
+  std::vector<int32_t> hyp(nmod, 0);
+  std::vector<uint2> cache(nmod, make_uint2(0, 0));
+  for (uint32_t h = 0; h < n.P; h++) {
+    bool full = false;
+    uint2 c = make_uint2(0, 0);
+    for (uint32_t m = h * n.mods_per_rank; m < (h + 1) * n.mods_per_rank; m++) {
+      hyp[m] = full ? 1 : 0;
+      cache[m] = c;
+      const GenChain &r = rec[2 * m + hyp[m]];
+      if (r.err) return gen_error(r.err, r.err_arg);
+      if (r.set_out == 2) continue;   // no synapse: as the module found it
+      full = r.set_out != 0;
+      c = make_uint2(r.c_out[0], r.c_out[1]);
+    }
+  }
+  std::vector<uint32_t> len(N);
+  for (uint32_t m = 0; m < nmod; m++)
+    memcpy(&len[(size_t)m * n.npcm], &htot[(size_t)hyp[m] * N + (size_t)m * n.npcm], 4ull * n.npcm);
+  DALLOC(d.sub_off, (size_t)N * (n.D + 1));
+  int rc = alloc_rows(e, len);
+  if (rc) return rc;
+  int32_t *dhyp;
+  uint2 *dcache;
+  unsigned long long *derr, herr = ~0ull;
+  GenFillScratch *scratch = nullptr;
+  TALLOC(dhyp, nmod);
+  TALLOC(dcache, nmod);
+  TALLOC(derr, 1);
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+  const uint32_t blocks = std::min<uint32_t>((N + GEN_FILL_WARPS - 1) / GEN_FILL_WARPS, (uint32_t)sms * 4);
+  if (N && *std::max_element(len.begin(), len.end()) > GEN_FILL_LIST) TALLOC(scratch, (size_t)blocks * GEN_FILL_WARPS);
+  CK(cudaMemcpyAsync(dhyp, hyp.data(), 4ull * nmod, cudaMemcpyHostToDevice, e->stream));
+  CK(cudaMemcpyAsync(dcache, cache.data(), sizeof(uint2) * nmod, cudaMemcpyHostToDevice, e->stream));
+  CK(cudaMemcpyAsync(derr, &herr, 8, cudaMemcpyHostToDevice, e->stream));
+  gen_fill_kernel<<<blocks, 32 * GEN_FILL_WARPS, GEN_FILL_WARPS * sizeof(GenFillWarp), e->stream>>>(
+      d.net, rows, row_off, tabs, gen_c, start, dhyp, dcache, d.row_ptr, d.sub_off, d.post, d.w16, scratch, derr,
+      bath_tmpl, d.inv_nu, d.max_ext, d.sub);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(&herr, derr, 8, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  if (herr != ~0ull) {
+    const uint32_t err = (uint32_t)(herr >> 22) & 15u;
+    return gen_error(err, err == GEN_ERR_DELAY ? (uint32_t)herr & 0x3FFFFFu : (uint32_t)(herr >> 39));
+  }
+  memcpy(hist0, rec[2 * (n.mods_per_rank - 1) + hyp[n.mods_per_rank - 1]].hist, sizeof(uint32_t) * GEN_HIST);
+  return 0;
+}
+
+static int generate_by_threads(dpsnn_engine *e, const std::vector<float> &prob, const uint32_t *bath_tmpl,
+                               uint32_t *hist0) {
+  const NetConst &n = e->hnet;
+  Dev &d = e->d;
+  const uint32_t N = n.N, D = n.D, P = n.P, nmod = n.nmod;
+  float *dprob;
+  TALLOC(dprob, prob.size());
+  CK(cudaMemcpyAsync(dprob, prob.data(), prob.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+  // pass A (both NormDev-cache hypotheses)
+  GenRecord *drec;
+  uint16_t *cnt_out;
+  uint32_t *scratch;
+  TALLOC(drec, 2 * nmod);
+  TALLOC(cnt_out, 2ull * N * D);
+  TALLOC(scratch, (size_t)2 * nmod * MAX_SYN_PER_NEURON);
+  int32_t *dhyp;
+  double *dcache;
+  TALLOC(dhyp, nmod);
+  TALLOC(dcache, nmod);
+  gen_kernel<<<(2 * nmod + GEN_THREADS - 1) / GEN_THREADS, GEN_THREADS, GEN_SMEM, e->stream>>>(
+      d.net, dprob, 0, drec, dhyp, dcache, cnt_out,
+                                                          nullptr, nullptr, nullptr, nullptr, scratch,
+                                                          bath_tmpl, nullptr, nullptr, nullptr);
+  CK(cudaGetLastError());
+  std::vector<GenRecord> rec(2 * nmod);
+  CK(cudaMemcpyAsync(rec.data(), drec, sizeof(GenRecord) * 2 * nmod, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  for (uint32_t k = 0; k < 2 * nmod; k++)
+    if (rec[k].err && !((k & 1) && (k / 2) % n.mods_per_rank == 0)) return gen_error(rec[k].err, rec[k].err_arg);
+  // resolve the NormDev cache hand-off rank by rank, module by module
+  std::vector<int32_t> hyp(nmod);
+  std::vector<double> cache(nmod, 0.0);
+  for (uint32_t h = 0; h < P; h++) {
+    int32_t set = 0;
+    double cval = 0.0;
+    for (uint32_t mm = 0; mm < n.mods_per_rank; mm++) {
+      uint32_t m = h * n.mods_per_rank + mm;
+      int choose = 0;
+      if (mm > 0 && set == 1) {
+        const GenRecord &r1 = rec[2 * m + 1];
+        if (!r1.used_normdev) {
+          choose = 1;
+        } else {
+          float mean = r1.first_mean, sigma = r1.first_sigma;
+          float wf = (float)(mean + cval * sigma);
+          bool acc = (mean > 0.0) ? !((wf < 0.0) || (wf >= 2.0 * mean)) : !((wf <= 2.0 * mean) || (wf > 0));
+          choose = acc ? 1 : 0;
+        }
+      }
+      hyp[m] = choose;
+      cache[m] = cval;
+      const GenRecord &r = rec[2 * m + choose];
+      if (r.used_normdev) {
+        set = r.set_out;
+        cval = r.cache_out;
+      }
+    }
+  }
+  CK(cudaMemcpyAsync(dhyp, hyp.data(), 4ull * nmod, cudaMemcpyHostToDevice, e->stream));
+  CK(cudaMemcpyAsync(dcache, cache.data(), 8ull * nmod, cudaMemcpyHostToDevice, e->stream));
+  // ---- CSR offsets from the chosen counts
+  uint32_t *row_len;
+  DALLOC(d.sub_off, (size_t)N * (D + 1));
+  TALLOC(row_len, N);
+  counts_to_csr_kernel<<<(N + 255) / 256, 256, 0, e->stream>>>(d.net, cnt_out, dhyp, d.sub_off, row_len);
+  CK(cudaGetLastError());
+  std::vector<uint32_t> hlen(N);
+  CK(cudaMemcpyAsync(hlen.data(), row_len, 4ull * N, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  int rc = alloc_rows(e, hlen);
+  if (rc) return rc;
+  // ---- pass B: regenerate the chosen hypothesis straight into the CSR
+  gen_kernel<<<(nmod + GEN_THREADS - 1) / GEN_THREADS, GEN_THREADS, GEN_SMEM, e->stream>>>(
+      d.net, dprob, 1, drec, dhyp, dcache, cnt_out, d.row_ptr,
+                                                      d.sub_off, d.post, d.w16, scratch, bath_tmpl, d.inv_nu,
+                                                      d.max_ext, d.sub);
+  CK(cudaGetLastError());
+  std::vector<GenRecord> recB(nmod);
+  CK(cudaMemcpyAsync(recB.data(), drec, sizeof(GenRecord) * nmod, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  for (uint32_t m = 0; m < nmod; m++)
+    if (recB[m].err) return dpsnn_fail(DPSNN_E_MODEL, "synapse generation pass B error %d", recB[m].err);
+  memcpy(hist0, recB[n.mods_per_rank - 1].hist, sizeof(uint32_t) * GEN_HIST);
   return 0;
 }
 
@@ -2390,10 +3087,10 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     CK(cudaStreamSynchronize(e->stream));
   }
   // mirrored stencil probabilities (initProbConnectMatrix, LIFCAconnectome.cpp:136-198)
-  float *dprob;
+  const uint32_t st = n.stencil;
+  std::vector<float> prob((size_t)DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP * st * st, 0.0f);
   {
-    const uint32_t st = n.stencil, M = n.max_mod, S = p->stencil_dim;
-    std::vector<float> prob((size_t)DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP * st * st, 0.0f);
+    const uint32_t M = n.max_mod, S = p->stencil_dim;
     for (uint32_t s = 0; s < n.nsub; s++)
       for (uint32_t t = 0; t < n.nsub; t++)
         for (uint32_t x = 0; x <= M; x++)
@@ -2407,9 +3104,6 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
             at(M - x, M - y) = v;
             at(M + x, M - y) = v;
           }
-    TALLOC(dprob, prob.size());
-    CK(cudaMemcpyAsync(dprob, prob.data(), prob.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-    CK(cudaStreamSynchronize(e->stream));
   }
   // neuron arrays
   DALLOC(d.v, N); DALLOC(d.c, N); DALLOC(d.tr, N); DALLOC(d.te, N);
@@ -2421,105 +3115,23 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   e->grid_neuron = (N + NEURON_BLOCK - 1) / NEURON_BLOCK;
   DALLOC(d.block_fired, e->grid_neuron);
 
-  // ---- synapse generation, pass A (both NormDev-cache hypotheses)
-  const uint32_t nmod = n.nmod;
-  GenRecord *drec;
-  uint16_t *cnt_out;
-  uint32_t *scratch;
-  TALLOC(drec, 2 * nmod);
-  TALLOC(cnt_out, 2ull * N * D);
+  // ---- synapse generation
   const uint32_t SD = p->stencil_dim;
   uint32_t *bath_tmpl;
   {
-    TALLOC(scratch, (size_t)2 * nmod * MAX_SYN_PER_NEURON);
     TALLOC(bath_tmpl, SD * SD);
     std::vector<uint32_t> bath(p->bath, p->bath + SD * SD);
     CK(cudaMemcpyAsync(bath_tmpl, bath.data(), 4ull * SD * SD, cudaMemcpyHostToDevice, e->stream));
-  }
-  int32_t *dhyp;
-  double *dcache;
-  TALLOC(dhyp, nmod);
-  TALLOC(dcache, nmod);
-  {
     int rc = set_kernel_attributes(e->device);
     if (rc) return rc;
   }
-  gen_kernel<<<(2 * nmod + GEN_THREADS - 1) / GEN_THREADS, GEN_THREADS, GEN_SMEM, e->stream>>>(
-      d.net, dprob, 0, drec, dhyp, dcache, cnt_out,
-                                                          nullptr, nullptr, nullptr, nullptr, scratch,
-                                                          bath_tmpl, nullptr, nullptr, nullptr);
-  CK(cudaGetLastError());
-  std::vector<GenRecord> rec(2 * nmod);
-  CK(cudaMemcpyAsync(rec.data(), drec, sizeof(GenRecord) * 2 * nmod, cudaMemcpyDeviceToHost, e->stream));
-  CK(cudaStreamSynchronize(e->stream));
-  for (uint32_t k = 0; k < 2 * nmod; k++)
-    if (rec[k].err && !((k & 1) && (k / 2) % n.mods_per_rank == 0)) {
-      const char *what[] = {"", "too many synapses generated for neuron", "synaptic weight out of minSynWeight_f range",
-                            "connection probability in (0,1e-5] is not supported", "delay >= env_D",
-                            "zero mean synaptic efficacy",
-                            "ERROR: delay level generated beyond the 80 max allowed delay levels, source neuron",
-                            "ERROR: delay generated beyond the pair's DMax, source neuron"};
-      return dpsnn_fail(DPSNN_E_MODEL, "synapse generation: %s (%u)", what[rec[k].err], rec[k].err_arg);
-    }
-  // resolve the NormDev cache hand-off rank by rank, module by module
-  std::vector<int32_t> hyp(nmod);
-  std::vector<double> cache(nmod, 0.0);
-  for (uint32_t h = 0; h < P; h++) {
-    int32_t set = 0;
-    double cval = 0.0;
-    for (uint32_t mm = 0; mm < n.mods_per_rank; mm++) {
-      uint32_t m = h * n.mods_per_rank + mm;
-      int choose = 0;
-      if (mm > 0 && set == 1) {
-        const GenRecord &r1 = rec[2 * m + 1];
-        if (!r1.used_normdev) {
-          choose = 1;
-        } else {
-          float mean = r1.first_mean, sigma = r1.first_sigma;
-          float wf = (float)(mean + cval * sigma);
-          bool acc = (mean > 0.0) ? !((wf < 0.0) || (wf >= 2.0 * mean)) : !((wf <= 2.0 * mean) || (wf > 0));
-          choose = acc ? 1 : 0;
-        }
-      }
-      hyp[m] = choose;
-      cache[m] = cval;
-      const GenRecord &rc = rec[2 * m + choose];
-      if (rc.used_normdev) {
-        set = rc.set_out;
-        cval = rc.cache_out;
-      }
-    }
+  uint32_t hist0[GEN_HIST];   // rank 0's stream after the build: its dynamics go on from there
+  GenPlan plan;
+  {
+    const bool warp_form = gen_plan(n, prob, plan);
+    int rc = warp_form ? generate_by_warps(e, plan, bath_tmpl, hist0) : generate_by_threads(e, prob, bath_tmpl, hist0);
+    if (rc) return rc;
   }
-  CK(cudaMemcpyAsync(dhyp, hyp.data(), 4ull * nmod, cudaMemcpyHostToDevice, e->stream));
-  CK(cudaMemcpyAsync(dcache, cache.data(), 8ull * nmod, cudaMemcpyHostToDevice, e->stream));
-  // ---- CSR offsets from the chosen counts
-  uint32_t *row_len;
-  DALLOC(d.sub_off, (size_t)N * (D + 1));
-  TALLOC(row_len, N);
-  counts_to_csr_kernel<<<(N + 255) / 256, 256, 0, e->stream>>>(d.net, cnt_out, dhyp, d.sub_off, row_len);
-  CK(cudaGetLastError());
-  std::vector<uint32_t> hlen(N);
-  std::vector<uint64_t> hrow(N + 1);
-  CK(cudaMemcpyAsync(hlen.data(), row_len, 4ull * N, cudaMemcpyDeviceToHost, e->stream));
-  CK(cudaStreamSynchronize(e->stream));
-  hrow[0] = 0;
-  for (uint32_t i = 0; i < N; i++) hrow[i + 1] = hrow[i] + hlen[i];
-  e->S = hrow[N];
-  DALLOC(d.row_ptr, N + 1);
-  CK(cudaMemcpyAsync(d.row_ptr, hrow.data(), 8ull * (N + 1), cudaMemcpyHostToDevice, e->stream));
-  DALLOC(d.post, e->S);
-  DALLOC(d.w16, e->S);
-  // ---- pass B: regenerate the chosen hypothesis straight into the CSR
-  gen_kernel<<<(nmod + GEN_THREADS - 1) / GEN_THREADS, GEN_THREADS, GEN_SMEM, e->stream>>>(
-      d.net, dprob, 1, drec, dhyp, dcache, cnt_out, d.row_ptr,
-                                                      d.sub_off, d.post, d.w16, scratch, bath_tmpl, d.inv_nu,
-                                                      d.max_ext, d.sub);
-  CK(cudaGetLastError());
-  std::vector<GenRecord> recB(nmod);
-  CK(cudaMemcpyAsync(recB.data(), drec, sizeof(GenRecord) * nmod, cudaMemcpyDeviceToHost, e->stream));
-  CK(cudaStreamSynchronize(e->stream));
-  for (uint32_t m = 0; m < nmod; m++)
-    if (recB[m].err) return dpsnn_fail(DPSNN_E_MODEL, "synapse generation pass B error %d", recB[m].err);
   // ---- run-over-group-end check (see DPSNN_synapse.c:211-265): the reference's
   // search continues past a (delay, source rank) group while the next entry has
   // the same presynaptic index; this happens only when the last source of a
@@ -2630,7 +3242,7 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     for (uint32_t h = 0; h < P; h++) {
       uint32_t h55[55];
       if (h == 0) {
-        memcpy(h55, recB[n.mods_per_rank - 1].hist, sizeof h55);
+        memcpy(h55, hist0, sizeof h55);
       } else {
         Ran3 g;
         memset(&g, 0, sizeof g);
