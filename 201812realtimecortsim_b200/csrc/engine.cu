@@ -2521,20 +2521,33 @@ __global__ void in_fill_kernel(const NetConst *net, const uint32_t *post, uint64
 }
 
 // per (rank, delay): max and min presynaptic index among synapses aimed at
-// that rank -- used to detect the reference's run-over-group-end search case
+// that rank -- used to detect the reference's run-over-group-end search case.
+// Most of a network's synapses cannot move an extremum that the first sources
+// looked at have set: the minima are taken over ascending sources, the maxima
+// over descending ones, and a synapse does an atomic only where it would
+// change what it reads (a stale value only costs an atomic).  An atomic or two
+// per synapse took 55 ms at the 24x24 network's 0.81 G.
 __global__ void group_extrema_kernel(const NetConst *net, const uint64_t *row_ptr, const uint16_t *sub_off,
                                      const uint32_t *post, uint32_t *gmax, uint32_t *gmin) {
   const uint32_t N = net->N, D = net->D, lane = threadIdx.x & 31;
-  for (uint32_t P = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; P < N; P += (gridDim.x * blockDim.x) >> 5) {
-    for (uint32_t dl = 0; dl < D; dl++) {
-      uint64_t b = row_ptr[P] + sub_off[(size_t)P * (D + 1) + dl], e = row_ptr[P] + sub_off[(size_t)P * (D + 1) + dl + 1];
-      for (uint64_t k = b + lane; k < e; k += 32) {
-        uint32_t h = post[k] / net->locN;
-        atomicMax(&gmax[h * D + dl], P);
-        atomicMin(&gmin[h * D + dl], P);
+  const uint32_t nw = (gridDim.x * blockDim.x) >> 5, w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  for (int up = 0; up < 2; up++)
+    for (uint32_t w = w0; w < N; w += nw) {
+      const uint32_t P = up ? w : N - 1 - w;
+      const uint64_t row = row_ptr[P];
+      const uint16_t *so = sub_off + (size_t)P * (D + 1);
+      const uint32_t len = so[D];
+      uint32_t dl = 0;
+      for (uint32_t k = lane; k < len; k += 32) {
+        while (so[dl + 1] <= k) dl++;
+        const uint32_t g = post[row + k] / net->locN * D + dl;
+        if (up) {
+          if (gmin[g] > P) atomicMin(&gmin[g], P);
+        } else {
+          if (gmax[g] < P) atomicMax(&gmax[g], P);
+        }
       }
     }
-  }
 }
 
 // ------------------------------------------------------------------ host engine
@@ -2615,6 +2628,32 @@ static void free_temps(dpsnn_engine *e) {
   e->temps.clear();
 }
 
+// The fix-up table on the device: a bit per float that has one, and per result
+// binade the fix-up inputs' least distance from the float their logarithm
+// rounds to (half an ulp at a midpoint), with a margin of 1e-3 ulp for the
+// last bits of the log that bath_lapse takes.  A bitmap built on the host is
+// 32 MB to fill and upload, and its 184 699 logarithms as much again: 9 ms of
+// a small network's build.
+__global__ void fix_clear_kernel(double *near) { near[threadIdx.x] = INFINITY; }
+__global__ void fix_table_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint32_t n,
+                                 uint32_t *bitmap, double *near, uint32_t *err) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t key = keys[i];
+  if (key < 0x30000000u || key > 0x3F800000u) return;
+  atomicOr(&bitmap[(key - 0x30000000u) >> 5], 1u << ((key - 0x30000000u) & 31));
+  const float x = __uint_as_float(key);
+  const double y = log((double)x);
+  const float f = logf_cr_from(x, y);
+  const uint32_t fb = __float_as_uint(f), E = (fb >> 23) & 0xFFu;
+  // bath_lapse takes a fix-up to be the float on the other side of the
+  // midpoint, as it is for any log with an error below one ulp
+  if (vals[i] != fb + (y < (double)f ? 1u : 0xFFFFFFFFu)) atomicMax(err, key);
+  if ((fb & 0x7FFFFFu) == 0) return;   // always looked up
+  const double dist = fabs(y - (double)f) - ldexp(1e-3, (int)E - 150);
+  atomicMin((unsigned long long *)&near[E], (unsigned long long)__double_as_longlong(dist));   // positive doubles
+}
+
 static int load_logf_fixup(dpsnn_engine *e) {
   std::string path = std::string(dpsnn_library_dir()) + "/logf_fixup.bin";
   const char *envp = getenv("DPSNN_LOGF_FIXUP");
@@ -2631,46 +2670,31 @@ static int load_logf_fixup(dpsnn_engine *e) {
   if (!ok) return dpsnn_fail(DPSNN_E_PARAM, "truncated %s", path.c_str());
   {
     const size_t words = ((size_t)(0x3F800000u - 0x30000000u) + 1 + 31) / 32;
-    std::vector<uint32_t> bm(words, 0u);
-    for (uint32_t key : keys)
-      if (key >= 0x30000000u && key <= 0x3F800000u) bm[(key - 0x30000000u) >> 5] |= 1u << ((key - 0x30000000u) & 31);
-    uint32_t *dbm;
+    uint32_t *dbm, *dkeys, *dvals, *derr, herr = 0;
+    double *dnear;
     DALLOC(dbm, words);
-    CK(cudaMemcpyAsync(dbm, bm.data(), 4 * words, cudaMemcpyHostToDevice, e->stream));
-    e->d.fix_bitmap = dbm;
-    // per result binade, the fix-up inputs' least distance from the float
-    // their logarithm rounds to (half an ulp at a midpoint), with a margin of
-    // 1e-3 ulp for the device log's last bits
-    std::vector<double> near(256, INFINITY);
-    for (uint32_t i = 0; i < n; i++) {
-      const uint32_t key = keys[i];
-      if (key < 0x30000000u || key > 0x3F800000u) continue;
-      float xf;
-      memcpy(&xf, &key, 4);
-      const double y = log((double)xf);
-      const float f = logf_cr_from(xf, y);
-      uint32_t fb;
-      memcpy(&fb, &f, 4);
-      // the kernels take a fix-up to be the float on the other side of the
-      // midpoint, as it is for any log with an error below one ulp
-      if (vals[i] != fb + (y < (double)f ? 1u : 0xFFFFFFFFu))
-        return dpsnn_fail(DPSNN_E_PARAM, "%s: logf is off by more than one ulp at 0x%08x", path.c_str(), key);
-      const uint32_t E = (fb >> 23) & 0xFFu;
-      if ((fb & 0x7FFFFFu) == 0) continue;   // always checked on the device
-      near[E] = std::min(near[E], fabs(y - (double)f) - ldexp(1e-3, (int)E - 150));
-    }
+    DALLOC(dnear, 256);
+    TALLOC(dkeys, n);
+    TALLOC(dvals, n);
+    TALLOC(derr, 1);
+    CK(cudaMemcpyAsync(dkeys, keys.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(dvals, vals.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
+    fix_clear_kernel<<<1, 256, 0, e->stream>>>(dnear);
+    fix_table_kernel<<<(n + 255) / 256 + 1, 256, 0, e->stream>>>(dkeys, dvals, n, dbm, dnear, derr);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, e->stream));
     std::vector<double2> tab(LOG_TAB_N);
     for (int k = 0; k < LOG_TAB_N; k++) {   // the logarithm that goes with the rounded 64/i
       const double c = 64.0 / (LOG_TAB_0 + k);
       tab[k] = make_double2(c, c == 1.0 ? 0.0 : -log_cr(c));
     }
-    double *dnear;
     double2 *dtab;
-    DALLOC(dnear, 256);
     DALLOC(dtab, LOG_TAB_N);
-    CK(cudaMemcpyAsync(dnear, near.data(), 8 * 256, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(dtab, tab.data(), sizeof(double2) * LOG_TAB_N, cudaMemcpyHostToDevice, e->stream));
     CK(cudaStreamSynchronize(e->stream));
+    if (herr)
+      return dpsnn_fail(DPSNN_E_PARAM, "%s: logf is off by more than one ulp at 0x%08x", path.c_str(), herr);
+    e->d.fix_bitmap = dbm;
     e->d.fix_near = dnear;
     e->d.log_tab = dtab;
   }
