@@ -92,6 +92,7 @@ struct NetConst {
   double Tau[DPSNN_MAX_SUBPOP], Theta[DPSNN_MAX_SUBPOP], H[DPSNN_MAX_SUBPOP];
   double Tarp[DPSNN_MAX_SUBPOP], AlphaC[DPSNN_MAX_SUBPOP], TauC[DPSNN_MAX_SUBPOP];
   double gC[DPSNN_MAX_SUBPOP], NuExt[DPSNN_MAX_SUBPOP];
+  double r_tau[DPSNN_MAX_SUBPOP], r_tauC[DPSNN_MAX_SUBPOP];   // 1/Tau, 1/TauC (div_by)
   double J[DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP], DJ[DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP];
   double DMin[DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP], DMax[DPSNN_MAX_SUBPOP * DPSNN_MAX_SUBPOP];
   float f2w, w2f, min_w;
@@ -893,6 +894,8 @@ struct Dev {
   uint8_t *sub, *fired;
   int32_t *last_spike_ms;
   uint32_t *block_fired;    // per NEURON_BLOCK block
+  uint32_t *fired_bits;     // [N/32] a small network's form of both: a bit per neuron
+  uint32_t *ticket;         // blocks of tail_small_kernel that are done
   // connectome
   uint64_t *row_ptr;
   uint16_t *sub_off;
@@ -927,10 +930,8 @@ struct Dev {
   // bath
   uint32_t *bath_hist;      // [P][BATH_HIST] the draws before each rank's next one
   uint64_t *bath_rank_base; // [P+1]
-  uint32_t *bath_off;       // [N]
-  uint16_t *bath_cnt;       // [N]
-  double *bath_time;
-  uint8_t *bath_lut;
+  uint2 *bath_at;           // [N] first bath event of this step, and their number
+  double2 *bath_ev;         // {time, input} per bath event
   const uint32_t *fix_bitmap; // one bit per float in [0x30000000, 0x3F800000]: key has a fix-up
   const double *fix_near;     // [256] by the result's exponent: a fix-up input's exact log lies at least
                               // this far from the float it rounds to
@@ -1082,20 +1083,108 @@ __device__ static inline void deliver_event(const Dev &d, const NetConst *net, u
   }
 }
 
-__global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
+// A small network's compaction (step 1), by every block of the kernel that
+// needs the list: its fired bits are at most SMALL_N / 32 words, so each block
+// counts them all and knows every spike's place without a launch or a wait;
+// the blocks share the ring's writes.
+#define SMALL_N 32768
+#define SMALL_WORDS (SMALL_N / 32)
+struct SmallSpikes {
+  uint32_t bits[SMALL_WORDS];   // neurons that fired, a bit each
+  uint32_t pre[SMALL_WORDS];    // spikes in the words before
+  uint32_t warp_sum[DELIVER_THREADS / 32];
+  uint32_t cnt;
+  // the q-th spike's neuron
+  __device__ uint32_t id(uint32_t q, uint32_t words) const {
+    uint32_t lo = 0, hi = words - 1;   // the last word with pre <= q (empty words share their successor's pre)
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (pre[mid] <= q) lo = mid; else hi = mid - 1;
+    }
+    uint32_t k = q - pre[lo], w = bits[lo], at = 0;
+    for (uint32_t h = 16; h > 0; h >>= 1) {   // the k-th set bit
+      const uint32_t c = __popc(w & ((1u << h) - 1));
+      if (k >= c) {
+        k -= c;
+        w >>= h;
+        at += h;
+      }
+    }
+    return 32 * lo + at;
+  }
+};
+static_assert(SMALL_WORDS == 4 * DELIVER_THREADS, "four words per thread");
+
+__device__ static inline void compact_small(const Dev &d, SmallSpikes &s, uint32_t t) {
+  const uint32_t N = d.net->N, slot = t % RING_SLOTS, words = (N + 31) / 32;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, w0 = 4 * tid;
+  uint32_t b[4], c = 0;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    b[k] = w0 + k < words ? d.fired_bits[w0 + k] : 0u;
+    c += __popc(b[k]);
+  }
+  uint32_t incl = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= (uint32_t)o) incl += y;
+  }
+  if (lane == 31) s.warp_sum[tid >> 5] = incl;
+  __syncthreads();
+  uint32_t acc = incl - c;
+  for (uint32_t w = 0; w < (tid >> 5); w++) acc += s.warp_sum[w];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    s.bits[w0 + k] = b[k];
+    s.pre[w0 + k] = acc;
+    acc += __popc(b[k]);
+  }
+  if (tid == DELIVER_THREADS - 1) {
+    s.cnt = acc;
+    if (blockIdx.x == 0) d.ring_cnt[slot] = acc;
+  }
+  __syncthreads();
+  for (uint32_t w = blockIdx.x + gridDim.x * tid; w < words; w += gridDim.x * DELIVER_THREADS) {
+    uint32_t q = s.pre[w];
+    for (uint32_t m = s.bits[w]; m; m &= m - 1, q++) {
+      const uint32_t i = 32 * w + __ffs(m) - 1;
+      d.ring_ids[(size_t)slot * N + q] = i;
+      d.ring_te[(size_t)slot * N + q] = d.te[i];
+      d.last_spike_ms[i] = (int32_t)t;
+      if (d.row_ptr[i + 1] == d.row_ptr[i]) atomicOr(d.flags, F_NO_TARGET);
+    }
+  }
+}
+
+// The compaction alone, where plasticity reads the last spike times before
+// and in the delivery.
+__global__ void __launch_bounds__(DELIVER_THREADS) compact_small_kernel(Dev d) {
+  __shared__ SmallSpikes s;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  compact_small(d, s, *d.t);
+}
+
+// FUSED: the step's compaction is done here (compact_small).
+template <bool FUSED>
+__device__ static inline void deliver(const Dev &d, SmallSpikes *sp) {
   const NetConst *net = d.net;
   const uint32_t t = *d.t, N = net->N, D = net->D, cap = net->ev_cap;
   __shared__ uint32_t s_pre[RING_SLOTS + 1];
   __shared__ uint32_t s_off[DELIVER_THREADS / 32][33];     // per warp: exclusive prefix of lengths
   __shared__ unsigned long long s_beg[DELIVER_THREADS / 32][32];
   __shared__ uint32_t s_key[DELIVER_THREADS / 32][32];
+  if (threadIdx.x < 32) {   // counts of the slots, then their prefix
+    for (uint32_t dd = threadIdx.x; dd < D; dd += 32)
+      s_pre[dd + 1] = FUSED && dd == 0 ? 0u : d.ring_cnt[(t + RING_SLOTS - dd) % RING_SLOTS];
+  }
+  if (FUSED) compact_small(d, *sp, t);
+  else __syncthreads();
   if (threadIdx.x == 0) {
+    if (FUSED) s_pre[1] = sp->cnt;
     uint32_t acc = 0;
-    for (uint32_t dd = 0; dd < D; dd++) {
-      s_pre[dd] = acc;
-      acc += d.ring_cnt[(t + RING_SLOTS - dd) % RING_SLOTS];
-    }
-    s_pre[D] = acc;
+    s_pre[0] = 0;
+    for (uint32_t dd = 1; dd <= D; dd++) s_pre[dd] = acc += s_pre[dd];
   }
   __syncthreads();
   const uint32_t total = s_pre[D];
@@ -1107,7 +1196,9 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
   uint32_t *ky = s_key[wb];
   unsigned long long my_events = 0;
   const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; w0 < total; w0 += nwarps * 32u) {
+  // items per warp at a time: 32, or fewer when they would leave warps idle
+  const uint32_t ipw = max(1u, min(32u, (total + nwarps - 1) / nwarps));
+  for (uint32_t w0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ipw; w0 < total; w0 += nwarps * ipw) {
     const uint32_t w = w0 + lane;
     uint64_t beg = 0;
     uint32_t len = 0, key = 0;
@@ -1120,11 +1211,11 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
       const uint32_t mid = (dl + hi) >> 1;
       if (s_pre[mid + 1] <= w0) dl = mid + 1; else hi = mid;
     }
-    if (w < total) {
+    if (w < total && lane < ipw) {
       while (s_pre[dl + 1] <= w) dl++;
       const uint32_t q = w - s_pre[dl];
       const uint32_t slot = (t + RING_SLOTS - dl) % RING_SLOTS;
-      const uint32_t P = d.ring_ids[(size_t)slot * N + q];
+      const uint32_t P = FUSED && dl == 0 ? sp->id(q, (N + 31) / 32) : d.ring_ids[(size_t)slot * N + q];
       const uint16_t *so = d.sub_off + (size_t)P * (D + 1);
       const uint32_t a = so[dl], b = so[dl + 1];
       beg = d.row_ptr[P] + a;
@@ -1189,6 +1280,18 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
   }
   for (int o = 16; o > 0; o >>= 1) my_events += __shfl_down_sync(0xffffffffu, my_events, o);
   if (lane == 0 && my_events) atomicAdd(d.events, my_events);
+}
+
+__global__ void __launch_bounds__(DELIVER_THREADS) deliver_kernel(Dev d) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  deliver<false>(d, nullptr);
+}
+__global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
+  __shared__ SmallSpikes s;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  deliver<true>(d, &s);
 }
 
 // Step 3: the Poisson bath (regularDynamicTimeStep, DPSNN_neuron_sim.c:604-640,
@@ -1280,7 +1383,7 @@ struct BathSmem {
   uint8_t idx[BATH_PAIRS];
   double a_nb[BATH_ACT], a_inv[BATH_ACT];   // queued neuron a at a % BATH_ACT
   uint4 a_b[BATH_ACT];              // bounds lo and hi - lo, min(cap, 16), cap
-  uint32_t a_id[BATH_ACT];
+  uint32_t a_id[BATH_ACT];          // neuron of the rank, its sub-population in the top bits
   uint32_t a_t[BATH_ACT];           // expected q advance of the queued neurons before a (2^-20 units)
   uint2 pack[BATH_SEGS][BATH_NC];   // a segment's counts less one, a nibble per neuron, by candidate
   uint16_t end[BATH_SEGS][BATH_NC + 2];   // its end, from win[], or BATH_UNDECIDED, BATH_NOT_YET
@@ -1298,7 +1401,7 @@ struct BathSmem {
 // The correctly rounded float log in the rare case that the double one does
 // not decide it; out of line, since inlined it takes the registers of the
 // whole kernel.
-__device__ __noinline__ static float logf_cr_undecided(float x) { return (float)log_cr((double)x); }
+__device__ __forceinline__ static float logf_cr_undecided(float x) { return (float)log_cr((double)x); }
 
 // The double of a normal float's bits (no conversion instruction: those have a
 // quarter of the rate).
@@ -1568,7 +1671,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
   const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1;
   const uint32_t t = d.bath_t[h], locN = net->locN, i0 = h * locN;
   const double T1 = (double)((double)t + 1.0);
-  const uint64_t ev_base = d.bath_rank_base[h];
+  const uint32_t ev_base = (uint32_t)d.bath_rank_base[h];
   // draws of this launch are numbered from BATH_HIST; the ones before are the
   // rank's kept history
   for (uint32_t n = tid; n < BATH_HIST; n += BATH_THREADS) s.raw[n] = d.bath_hist[(size_t)h * BATH_HIST + n];
@@ -1582,7 +1685,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
     s.ctl[0] = c;
   }
   // the preparers' next neurons, loaded an iteration ahead
-  uint32_t p_i = 0, p_t = 0, x_mx = 0;
+  uint32_t p_i = 0, p_t = 0, x_mx = 0, x_sub = 0;
   double x_nb = 0, x_inv = 0;
   if (warp == 8 || warp == 13) {
     const uint32_t i = lane + (warp == 8 ? 0 : 32);
@@ -1590,6 +1693,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
       x_nb = d.nb_prev[i0 + i];
       x_inv = d.inv_nu[i0 + i];
       x_mx = d.max_ext[i0 + i];
+      x_sub = d.sub[i0 + i];
     }
   }
   __syncthreads();
@@ -1643,11 +1747,12 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
       uint32_t e = cur.act_end;
       for (int g = 0; g < 4 && p_i < locN && e < cur.a + 2 * BATH_SB && e + 64 <= cur.sb_a + BATH_ACT; g++, p_i += 64) {
         const double nb = x_nb, inv = x_inv;
-        const uint32_t mx = x_mx, i = p_i + 32 * pw + lane;
+        const uint32_t mx = x_mx, sub = x_sub, i = p_i + 32 * pw + lane;
         if (i + 64 < locN) {
           x_nb = d.nb_prev[i0 + i + 64];
           x_inv = d.inv_nu[i0 + i + 64];
           x_mx = d.max_ext[i0 + i + 64];
+          x_sub = d.sub[i0 + i + 64];
         }
         const bool act = i < locN && inv > 0 && nb < T1;
         const uint32_t bal = __ballot_sync(0xffffffffu, act);
@@ -1669,12 +1774,11 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           s.a_nb[k] = nb;
           s.a_inv[k] = inv;
           s.a_b[k] = make_uint4(lo, hi1 - lo, min(mx, 16u), mx);
-          s.a_id[k] = i;
+          s.a_id[k] = i | (sub << 25);
           s.a_t[k] = p_t + pw * t0 + incl - tv;
         } else if (i < locN) {
           d.nb[i0 + i] = nb;
-          d.bath_off[i0 + i] = 0;
-          d.bath_cnt[i0 + i] = 0;
+          d.bath_at[i0 + i] = make_uint2(0, 0);
         }
         p_t += t0 + t1;
         e += n0 + n1;
@@ -1739,20 +1843,18 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           m0 = s.e_start[par][g] + jj + nibble_sum(word & ((1u << sh) - 1)) + (jj < 8 ? 0u : nibble_sum(pk.x));
           cnt = ((word >> sh) & 15u) + 1;
         }
-        const uint32_t i = i0 + s.a_id[a], off = cur.out + m0;
+        const uint32_t id = s.a_id[a], i = i0 + (id & ((1u << 25) - 1)), at = ev_base + cur.out + m0;
+        const double *lut = d.lut + 256 * (id >> 25);
         const double inv = s.a_inv[a];
         double v = s.a_nb[a];
-        double *bt = d.bath_time + ev_base + off;
-        uint8_t *bl = d.bath_lut + ev_base + off;
+        double2 *ev = d.bath_ev + at;
         for (uint32_t c = 0; c < cnt; c++) {
-          bt[c] = v;
-          bl[c] = s.idx[(m0 + c) & M];
+          ev[c] = make_double2(v, __ldg(&lut[s.idx[(m0 + c) & M]]));
           v += (double)s.lap[(m0 + c) & M] * inv;
         }
         if (v < T1) bath_singles(d, s, cur.base + 2 * (m0 + cnt), cur.raw_end, inv, T1, v);
         d.nb[i] = v;
-        d.bath_off[i] = off;
-        d.bath_cnt[i] = (uint16_t)cnt;
+        d.bath_at[i] = make_uint2(at, cnt);
       }
     }
     __syncthreads();
@@ -1775,39 +1877,90 @@ struct NeuronRegs {
   double v, c, tr, te;
   int fired;
 };
+// A sub-population's parameters, and 1/Tau, 1/TauC rounded to nearest: read
+// from memory where they are used (LifcaMem), or kept in registers.  The
+// thread-per-neuron kernel, whose events' buffers already fill its 64
+// registers, takes 0.137 ms per 24x24 step with the first and 0.159 with the
+// second; the merged streams' kernel (80 registers) 30 us per busy 16 000
+// neurons with the second and 35 with the first.
+struct LifcaMem {
+  const NetConst *net;
+  uint32_t s;
+  __device__ double Tau() const { return net->Tau[s]; }
+  __device__ double r_tau() const { return net->r_tau[s]; }
+  __device__ double TauC() const { return net->TauC[s]; }
+  __device__ double r_tauC() const { return net->r_tauC[s]; }
+  __device__ double Theta() const { return net->Theta[s]; }
+  __device__ double H() const { return net->H[s]; }
+  __device__ double Tarp() const { return net->Tarp[s]; }
+  __device__ double AlphaC() const { return net->AlphaC[s]; }
+  __device__ double gC() const { return net->gC[s]; }
+};
+struct LifcaRegs {
+  double tau, rtau, tauc, rtauc, theta, h, tarp, alphac, gc;
+  __device__ LifcaRegs(const NetConst *net, uint32_t s)
+      : tau(net->Tau[s]), rtau(net->r_tau[s]), tauc(net->TauC[s]), rtauc(net->r_tauC[s]), theta(net->Theta[s]),
+        h(net->H[s]), tarp(net->Tarp[s]), alphac(net->AlphaC[s]), gc(net->gC[s]) {}
+  __device__ double Tau() const { return tau; }
+  __device__ double r_tau() const { return rtau; }
+  __device__ double TauC() const { return tauc; }
+  __device__ double r_tauC() const { return rtauc; }
+  __device__ double Theta() const { return theta; }
+  __device__ double H() const { return h; }
+  __device__ double Tarp() const { return tarp; }
+  __device__ double AlphaC() const { return alphac; }
+  __device__ double gC() const { return gc; }
+};
+// a / b by b's reciprocal r (Markstein's theorem, IBM J. Res. Dev. 34, 1990:
+// with r the reciprocal rounded to nearest and q within an ulp of a/b, q +
+// r (a - b q) rounds to the quotient rounded to nearest; the first correction
+// brings q = a r within an ulp).  Five operations and no branch, where a
+// division's code has both; r = 0: b is out of the range in which nothing
+// overflows or underflows on the way, and is divided by.
+__device__ static inline double div_by(double a, double b, double r) {
+  if (r == 0.0) return a / b;
+  double q = a * r;
+  q = fma(fma(-q, b, a), r, q);
+  return fma(fma(-q, b, a), r, q);
+}
+
 // The coefficients of one update: deltaT = t - Tr.  They depend on event
 // times only (Tr is the previous event's time), so the neuron run computes
 // them one event ahead, off the dependent chain of v and c.
-__device__ static inline void lifca_coeff(double Tau, double TauC, double deltaT, double &dth, double &rmh,
-                                          double &poly) {
+template <typename Par>
+__device__ static inline void lifca_coeff(const Par &p, double deltaT, double &dth, double &rmh, double &poly) {
   dth = deltaT / 2;
-  rmh = dth / Tau;
-  const double rc = deltaT / TauC;
+  rmh = div_by(dth, p.Tau(), p.r_tau());
+  const double rc = div_by(deltaT, p.TauC(), p.r_tauC());
   poly = 1 - rc + rc * rc / 2;
 }
 
+// The calcium decay over the refractory period: once per spike, so out of
+// line (inlined, its double-double arithmetic takes the registers of the
+// neuron kernels).
+__device__ __forceinline__ static double exp_cr_call(double x) { return exp_cr(x); }
+
 // LIFCADynamic with the coefficients of this event computed ahead; the branch
 // that leaves the refractory period moves deltaT, and recomputes them.
-__device__ static inline void lifca_pre(const NetConst *net, uint32_t s, NeuronRegs &n, double t, double I,
-                                        double dth, double rmh, double poly) {
-  const double Tau = net->Tau[s], Theta = net->Theta[s], H = net->H[s], Tarp = net->Tarp[s];
-  const double AlphaC = net->AlphaC[s], TauC = net->TauC[s], gC = net->gC[s];
+template <typename Par>
+__device__ static inline void lifca_pre(const Par &p, NeuronRegs &n, double t, double I, double dth, double rmh,
+                                        double poly) {
   double v = n.v, c = n.c, Te = n.te;
   const double Tr = n.tr, TFLES = t - Te;
-  if (TFLES > Tarp) {
+  if (TFLES > p.Tarp()) {
     const double TrTe = Tr - Te;
-    if (TrTe < Tarp) {
+    if (TrTe < p.Tarp()) {
       const double deltaT0 = t - Tr;
-      c *= exp_cr(-(deltaT0 - TFLES + Tarp) / TauC);
-      lifca_coeff(Tau, TauC, TFLES - Tarp, dth, rmh, poly);
+      c *= exp_cr_call(-(deltaT0 - TFLES + p.Tarp()) / p.TauC());
+      lifca_coeff(p, TFLES - p.Tarp(), dth, rmh, poly);
     }
-    v = v - v * rmh - gC * c * dth;
-    v = v - v * rmh - gC * c * dth;
+    v = v - v * rmh - p.gC() * c * dth;
+    v = v - v * rmh - p.gC() * c * dth;
     c = c * poly;
     v += I;
-    if (v >= Theta) {
-      v = H;
-      c += AlphaC;
+    if (v >= p.Theta()) {
+      v = p.H();
+      c += p.AlphaC();
       Te = t;
       n.fired = 1;
     }
@@ -1843,10 +1996,14 @@ __device__ static inline bool sortev_gt(const SortEv &a, const SortEv &b) {
 }
 
 
+// be: its nb bath events ({time, input}; the bath's emitters look the input
+// up, where the time, then the LUT index, then the LUT value were three
+// dependent loads per event), in global memory or staged in shared memory.
 template <typename Events>
-__device__ static inline int run_neuron_ev(const Dev &d, uint32_t i, uint32_t t, const Events &evs, uint32_t ns) {
-  const NetConst *net = d.net;
-  const uint32_t s = d.sub[i];
+__device__ static inline int run_neuron_ev(const Dev &d, uint32_t i, uint32_t t, const Events &evs, uint32_t ns,
+                                           const double2 *be, uint32_t nb) {
+  const LifcaMem par{d.net, d.sub[i]};
+  double2 b0 = nb ? be[0] : make_double2(0.0, 0.0);
   NeuronRegs n;
   n.v = d.v[i];
   n.c = d.c[i];
@@ -1854,38 +2011,34 @@ __device__ static inline int run_neuron_ev(const Dev &d, uint32_t i, uint32_t t,
   n.te = d.te[i];
   n.fired = 0;
   const double T0 = (double)t;
-  const uint32_t boff = d.bath_off[i], bc = d.bath_cnt[i];
-  const uint64_t bbase = d.bath_rank_base[i / net->locN] + boff;
-  const double *lut = d.lut + (size_t)s * 256;
-  const double Tau = net->Tau[s], TauC = net->TauC[s];
   uint32_t a = 0, b = 0;
-  double bt = (b < bc) ? d.bath_time[bbase] : 0.0;
   // the merge's next event (time, input)
   auto next = [&](double &ct, double &I) -> bool {
-    if (a < ns && (b >= bc || evs.time(a) <= bt)) {
+    if (a < ns && (b >= nb || evs.time(a) <= b0.x)) {
       ct = evs.time(a);
       I = (double)evs.weight(a);
       a++;
       return true;
     }
-    if (b < bc) {
-      ct = bt;
-      I = lut[d.bath_lut[bbase + b]];
+    if (b < nb) {
+      ct = b0.x;
+      I = b0.y;
       b++;
-      if (b < bc) bt = d.bath_time[bbase + b];
+      if (b < nb) b0 = be[b];
       return true;
     }
     return false;
   };
+  bool bad = false;
   double ct = 0, I = 0, dth = 0, rmh = 0, poly = 0;
   bool have = next(ct, I);
-  if (have) lifca_coeff(Tau, TauC, ct - n.tr, dth, rmh, poly);
+  if (have) lifca_coeff(par, ct - n.tr, dth, rmh, poly);
   while (have) {
     double ct1 = 0, I1 = 0, dth1 = 0, rmh1 = 0, poly1 = 0;
     const bool have1 = next(ct1, I1);
-    if (have1) lifca_coeff(Tau, TauC, ct1 - ct, dth1, rmh1, poly1);   // after this event Tr = ct
-    if (((ct - T0) >= 1.0) || ((ct - T0) < 0)) atomicOr(d.flags, F_TIME_WINDOW);
-    lifca_pre(net, s, n, ct, I, dth, rmh, poly);
+    if (have1) lifca_coeff(par, ct1 - ct, dth1, rmh1, poly1);   // after this event Tr = ct
+    bad |= ((ct - T0) >= 1.0) || ((ct - T0) < 0);
+    lifca_pre(par, n, ct, I, dth, rmh, poly);
     ct = ct1;
     I = I1;
     dth = dth1;
@@ -1893,11 +2046,11 @@ __device__ static inline int run_neuron_ev(const Dev &d, uint32_t i, uint32_t t,
     poly = poly1;
     have = have1;
   }
+  if (bad) atomicOr(d.flags, F_TIME_WINDOW);
   d.v[i] = n.v;
   d.c[i] = n.c;
   d.tr[i] = n.tr;
   d.te[i] = n.te;
-  if (n.fired) d.fired[i] = 1;
   return n.fired;
 }
 
@@ -1915,10 +2068,14 @@ struct EvRecords {  // sorted 16-byte records
 
 __device__ static inline int run_neuron(const Dev &d, uint32_t i, uint32_t t, const double *tau,
                                         const float *val, uint32_t ns) {
-  return run_neuron_ev(d, i, t, EvArrays{tau, val}, ns);
+  const uint2 at = d.bath_at[i];
+  return run_neuron_ev(d, i, t, EvArrays{tau, val}, ns, d.bath_ev + at.x, at.y);
 }
-__device__ static inline int run_neuron_se(const Dev &d, uint32_t i, uint32_t t, const SortEv *se, uint32_t ns) {
-  return run_neuron_ev(d, i, t, EvRecords{se}, ns);
+
+// A neuron that fired, run apart from its block.
+__device__ static inline void mark_fired(const Dev &d, uint32_t i) {
+  d.fired[i] = 1;
+  atomicAdd(&d.block_fired[i / NEURON_BLOCK], 1u);
 }
 
 // Step 4: neuron update (regularDynamicTimeStep, DPSNN_neuron_sim.c:522-662).
@@ -1927,10 +2084,73 @@ __device__ static inline int run_neuron_se(const Dev &d, uint32_t i, uint32_t t,
 // Heavier neurons are queued for the heavy path below.
 __device__ static inline uint32_t warp_path_max(const NetConst *net);
 
+// A warp's neurons' bath events follow one another in memory (one rank's are
+// written in neuron order): the warp loads them into shared memory at once,
+// coalesced, and each thread reads its own from there.  A warp that spans two
+// ranks, or whose neurons have more than NEURON_STAGE events, reads global
+// memory.  What bounds it: the latency of a warp's chain, events one after
+// another in 16 lanes of 32 on average (at 24x24, 720 000 neurons without
+// synaptic events: 80 us alone, DRAM at 7 %, an instruction every 4 cycles
+// per scheduler).  A step of 24x24 takes 228 us with the staged pairs and
+// div_by against 239 with three dependent loads per event and two divisions.
+#define NEURON_STAGE 192
+
+// The warp's bath events staged in st where they fit; the thread's first one.
+__device__ static inline const double2 *stage_bath(const Dev &d, uint2 at, double2 *st, uint32_t lane) {
+  const double2 *be = d.bath_ev + at.x;
+  const uint32_t lo = __reduce_min_sync(0xffffffffu, at.y ? at.x : 0xFFFFFFFFu);
+  const uint32_t hi = __reduce_max_sync(0xffffffffu, at.y ? at.x + at.y : 0u);
+  if (hi > lo && hi - lo <= NEURON_STAGE) {
+    for (uint32_t k = lane; k < hi - lo; k += 32) st[k] = d.bath_ev[lo + k];
+    be = st + (at.y ? at.x - lo : 0u);
+  }
+  __syncwarp();
+  return be;
+}
+
+// A light neuron: at most LOCAL_EVENTS synaptic events, sorted by insertion.
+__device__ static inline int run_light(const Dev &d, uint32_t i, uint32_t t, uint32_t cnt, const double2 *be,
+                                       uint32_t nb) {
+  const uint32_t N = d.net->N, D = d.net->D, cap = d.net->ev_cap;
+        SortEv se[LOCAL_EVENTS];
+        const uint2 *ev = d.ev + (size_t)i * cap;
+        // events in groups of NEURON_BATCH: the loads, then the arrival-time
+        // gathers, are all in flight together; then insertion by (time, key)
+        for (uint32_t e0 = 0; e0 < cnt; e0 += NEURON_BATCH) {
+          uint2 x[NEURON_BATCH];
+          double tm[NEURON_BATCH];
+  #pragma unroll
+          for (int u = 0; u < NEURON_BATCH; u++)
+            if (e0 + u < cnt) x[u] = ev[e0 + u];
+  #pragma unroll
+          for (int u = 0; u < NEURON_BATCH; u++)
+            if (e0 + u < cnt) tm[u] = event_time(d, x[u].x, t, D, N);
+  #pragma unroll
+          for (int u = 0; u < NEURON_BATCH; u++) {
+            if (e0 + u < cnt) {
+              SortEv y;
+              y.tau = tm[u];
+              y.key = x[u].x;
+              y.val = __uint_as_float(x[u].y);
+              uint32_t p = e0 + u;
+              while (p > 0 && sortev_gt(se[p - 1], y)) {
+                se[p] = se[p - 1];
+                p--;
+              }
+              se[p] = y;
+            }
+          }
+        }
+  return run_neuron_ev(d, i, t, EvRecords{se}, cnt, be, nb);
+}
+
 __global__ void __launch_bounds__(NEURON_BLOCK, 4) neuron_kernel(Dev d) {
+  __shared__ double2 s_bath[NEURON_BLOCK / 32][NEURON_STAGE];
   const NetConst *net = d.net;
-  const uint32_t t = *d.t, N = net->N, D = net->D, cap = net->ev_cap;
-  const uint32_t i = blockIdx.x * NEURON_BLOCK + threadIdx.x;
+  const uint32_t t = *d.t, N = net->N;
+  const uint32_t i = blockIdx.x * NEURON_BLOCK + threadIdx.x, lane = threadIdx.x & 31;
+  const uint2 at = i < N ? d.bath_at[i] : make_uint2(0, 0);
+  const double2 *be = stage_bath(d, at, s_bath[threadIdx.x >> 5], lane);
   int fired = 0;
   if (i < N) {
     const uint32_t cnt = d.ev_cnt[i];
@@ -1943,36 +2163,8 @@ __global__ void __launch_bounds__(NEURON_BLOCK, 4) neuron_kernel(Dev d) {
         d.heavy_list[2ull * N * path + N + k] = cnt;
       }
     } else {
-      SortEv se[LOCAL_EVENTS];
-      const uint2 *ev = d.ev + (size_t)i * cap;
-      // events in groups of NEURON_BATCH: the loads, then the arrival-time
-      // gathers, are all in flight together; then insertion by (time, key)
-      for (uint32_t e0 = 0; e0 < cnt; e0 += NEURON_BATCH) {
-        uint2 x[NEURON_BATCH];
-        double tm[NEURON_BATCH];
-#pragma unroll
-        for (int u = 0; u < NEURON_BATCH; u++)
-          if (e0 + u < cnt) x[u] = ev[e0 + u];
-#pragma unroll
-        for (int u = 0; u < NEURON_BATCH; u++)
-          if (e0 + u < cnt) tm[u] = event_time(d, x[u].x, t, D, N);
-#pragma unroll
-        for (int u = 0; u < NEURON_BATCH; u++) {
-          if (e0 + u < cnt) {
-            SortEv y;
-            y.tau = tm[u];
-            y.key = x[u].x;
-            y.val = __uint_as_float(x[u].y);
-            uint32_t p = e0 + u;
-            while (p > 0 && sortev_gt(se[p - 1], y)) {
-              se[p] = se[p - 1];
-              p--;
-            }
-            se[p] = y;
-          }
-        }
-      }
-      fired = run_neuron_se(d, i, t, se, cnt);
+      fired = run_light(d, i, t, cnt, be, at.y);
+      if (fired) d.fired[i] = 1;
     }
   }
   const uint32_t bc = __syncthreads_count(fired);
@@ -2064,8 +2256,9 @@ template <int E>
 __device__ static inline bool heavy_sort_one(const Dev &d, uint32_t i, uint2 *ev, uint32_t n, uint32_t t, uint32_t D,
                                              uint32_t N, uint32_t cap, uint32_t lane, HeavySortWarp &w) {
   const double T0 = (double)t;
-  const uint32_t bcnt = d.bath_cnt[i];
-  const uint64_t bbase = d.bath_rank_base[i / d.net->locN] + d.bath_off[i];
+  const uint2 at = d.bath_at[i];
+  const double2 *be = d.bath_ev + at.x;
+  const uint32_t bcnt = at.y;
   const bool merged = n + bcnt <= cap / 2 && bcnt <= HS_BATH_MAX;
   const uint32_t bc = merged ? bcnt : 0u;
   for (uint32_t b = lane; b <= HS_BUCKETS; b += 32) w.start[b] = 0;
@@ -2091,7 +2284,7 @@ __device__ static inline bool heavy_sort_one(const Dev &d, uint32_t i, uint2 *ev
   for (int r = 0; r < HS_BATH_MAX / 32; r++) {
     const uint32_t j = lane + 32u * r;
     if (j < bc) {
-      const double btj = d.bath_time[bbase + j];
+      const double btj = be[j].x;
       const uint32_t b = min((uint32_t)((btj - T0) * (double)HS_BUCKETS), (uint32_t)HS_BUCKETS - 1);
       bb[r] = (b << 16) | atomicAdd(&w.start[b], 1u);
     }
@@ -2133,7 +2326,7 @@ __device__ static inline bool heavy_sort_one(const Dev &d, uint32_t i, uint2 *ev
     const uint32_t j = lane + 32u * r;
     if (j < bc) {
       const uint32_t b = bb[r] >> 16, p = w.start[b] + (bb[r] & 0xFFFFu);
-      w.tau[p] = d.bath_time[bbase + j];
+      w.tau[p] = be[j].x;
       w.key[p] = HS_BATH_KEY + j;
       bb[r] = (b << 16) | p;
     }
@@ -2170,11 +2363,10 @@ __device__ static inline bool heavy_sort_one(const Dev &d, uint32_t i, uint2 *ev
     }
   }
   if (merged) {
-    const double *lut = d.lut + (size_t)d.sub[i] * 256;
 #pragma unroll
     for (int r = 0; r < HS_BATH_MAX / 32; r++) {
       const uint32_t j = lane + 32u * r;
-      if (j < bc) ms[place(bb[r])] = make_double2(w.tau[bb[r] & 0xFFFFu], lut[d.bath_lut[bbase + j]]);
+      if (j < bc) ms[place(bb[r])] = be[j];
     }
   }
   __syncwarp();   // the warp's next neuron reuses the staging arrays
@@ -2263,8 +2455,7 @@ __device__ static inline bool huge_runs_here(const NetConst *net, uint32_t cnt) 
 // four being applied, each update's coefficients computed off the v/c chain.
 __device__ static inline int run_neuron_merged(const Dev &d, uint32_t i, uint32_t t, const double2 *ms,
                                                uint32_t ne) {
-  const NetConst *net = d.net;
-  const uint32_t s = d.sub[i];
+  const LifcaRegs par(d.net, d.sub[i]);
   NeuronRegs n;
   n.v = d.v[i];
   n.c = d.c[i];
@@ -2272,7 +2463,6 @@ __device__ static inline int run_neuron_merged(const Dev &d, uint32_t i, uint32_
   n.te = d.te[i];
   n.fired = 0;
   const double T0 = (double)t;
-  const double Tau = net->Tau[s], TauC = net->TauC[s];
   double2 cur[4], nxt[4];
 #pragma unroll
   for (int u = 0; u < 4; u++) cur[u] = (u < (int)ne) ? ms[u] : make_double2(0.0, 0.0);
@@ -2285,9 +2475,9 @@ __device__ static inline int run_neuron_merged(const Dev &d, uint32_t i, uint32_
       if (e0 + u < ne) {
         const double ct = cur[u].x;
         double dth, rmh, poly;
-        lifca_coeff(Tau, TauC, ct - n.tr, dth, rmh, poly);
+        lifca_coeff(par, ct - n.tr, dth, rmh, poly);
         bad |= ((ct - T0) >= 1.0) || ((ct - T0) < 0);
-        lifca_pre(net, s, n, ct, cur[u].y, dth, rmh, poly);
+        lifca_pre(par, n, ct, cur[u].y, dth, rmh, poly);
       }
     }
 #pragma unroll
@@ -2298,7 +2488,6 @@ __device__ static inline int run_neuron_merged(const Dev &d, uint32_t i, uint32_
   d.c[i] = n.c;
   d.tr[i] = n.tr;
   d.te[i] = n.te;
-  if (n.fired) d.fired[i] = 1;
   return n.fired;
 }
 
@@ -2310,9 +2499,8 @@ __global__ void __launch_bounds__(128, 6) heavy_run_kernel(Dev d) {
   for (uint32_t hh = blockIdx.x * blockDim.x + threadIdx.x; hh < nh; hh += gridDim.x * blockDim.x) {
     const uint32_t i = d.heavy_list[hh], ns = d.heavy_list[N + hh];
     if (!(ns & HEAVY_MERGED)) continue;
-    const uint32_t ne = (ns & ~HEAVY_MERGED) + d.bath_cnt[i];
-    if (run_neuron_merged(d, i, t, reinterpret_cast<const double2 *>(d.ev + (size_t)i * cap), ne))
-      atomicAdd(&d.block_fired[i / NEURON_BLOCK], 1u);
+    const uint32_t ne = (ns & ~HEAVY_MERGED) + d.bath_at[i].y;
+    if (run_neuron_merged(d, i, t, reinterpret_cast<const double2 *>(d.ev + (size_t)i * cap), ne)) mark_fired(d, i);
   }
 }
 
@@ -2338,7 +2526,7 @@ __global__ void heavy_rest_kernel(Dev d) {
     const uint2 *ev = d.ev + (size_t)i * cap;
     const double *st = reinterpret_cast<const double *>(ev);
     const float *sv = reinterpret_cast<const float *>(ev + cap / 2);
-    if (run_neuron_ev(d, i, t, EvArrays{st, sv}, ns)) atomicAdd(&d.block_fired[i / NEURON_BLOCK], 1u);
+    if (run_neuron(d, i, t, st, sv, ns)) mark_fired(d, i);
   }
 }
 
@@ -2371,7 +2559,10 @@ __device__ static inline uint32_t gather_events(const Dev &d, uint32_t i, uint32
   return min(*counter, capacity);
 }
 
-__global__ void __launch_bounds__(HEAVY_THREADS) huge_kernel(Dev d) {
+// The block path's list, neurons strided over the blocks; fired(i) for a
+// neuron run here.
+template <typename Fired>
+__device__ static inline void huge_sort(const Dev &d, const Fired &fired) {
   // 32 KB of shared memory, so that a block fits on an SM beside the bath's
   // blocks; the rare neuron with more events sorts in its block's global
   // scratch (HEAVY_MAX events)
@@ -2419,9 +2610,137 @@ __global__ void __launch_bounds__(HEAVY_THREADS) huge_kernel(Dev d) {
         sv[e] = s_val[e];
       }
     } else if (tid == 0) {
-      if (run_neuron(d, i, t, s_tau, s_val, n)) atomicAdd(&d.block_fired[i / NEURON_BLOCK], 1u);
+      if (run_neuron(d, i, t, s_tau, s_val, n)) fired(i);
     }
     __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(HEAVY_THREADS) huge_kernel(Dev d) {
+  huge_sort(d, [&](uint32_t i) { mark_fired(d, i); });
+}
+
+// ------------------------------------------------------------------ small networks
+// Up to SMALL_N neurons a step is bound by its launches, about 5 us each with
+// the gap between two, and most of the large form's blocks find nothing to do.
+// Here a step is three kernels (and the bath): deliver_small_kernel with the
+// compaction, neuron_small_kernel with the warp path's sorts and runs, and
+// tail_small_kernel, each brought up while the one before it ends.  Measured
+// per step: 19 us from 45 for 100 neurons, 23 from 54 for 1155 in 5 ranks, 67
+// from 113 for 16 000 busy ones (8 events per neuron); what is left is the
+// update's chain of events, and the bath where a rank is long.
+
+// A block of WARPS warps per 32 neurons: warp 0 runs the light ones while the
+// others (and then it too) sort the heavier ones, which then run a lane each.
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) neuron_small_kernel(Dev d) {
+  __shared__ HeavySortWarp s_ws[WARPS];
+  __shared__ double2 s_bath[NEURON_STAGE];
+  __shared__ uint32_t s_i[32], s_n[32], s_nh, s_next;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  const NetConst *net = d.net;
+  const uint32_t t = *d.t, N = net->N, D = net->D, cap = net->ev_cap;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t i = blockIdx.x * 32 + lane;
+  uint32_t cnt = 0;
+  bool light = false;
+  if (warp == 0) {
+    if (i < N) {
+      cnt = d.ev_cnt[i];
+      if (cnt) d.ev_cnt[i] = 0;
+    }
+    light = i < N && cnt <= net->light_max;
+    const bool heavy = !light && cnt && cnt <= warp_path_max(net);
+    const uint32_t bal = __ballot_sync(0xffffffffu, heavy);
+    if (heavy) {
+      const uint32_t k = __popc(bal & ((1u << lane) - 1));
+      s_i[k] = i;
+      s_n[k] = cnt;
+    } else if (i < N && !light) {
+      const uint32_t k = atomicAdd(&d.heavy_cnt[1], 1u);
+      d.heavy_list[2ull * N + k] = i;
+      d.heavy_list[3ull * N + k] = cnt;
+    }
+    if (lane == 0) {
+      s_nh = __popc(bal);
+      s_next = 0;
+    }
+  }
+  __syncthreads();
+  const uint32_t nh = s_nh;
+  uint32_t bits = 0;
+  if (warp == 0) {
+    const uint2 at = i < N ? d.bath_at[i] : make_uint2(0, 0);
+    const double2 *be = stage_bath(d, at, s_bath, lane);
+    int fired = 0;
+    if (light) fired = run_light(d, i, t, cnt, be, at.y);
+    bits = __ballot_sync(0xffffffffu, fired);
+  }
+  if (nh) {
+    for (;;) {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(&s_next, 1u);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= nh) break;
+      const uint32_t j = s_i[k], n = s_n[k];
+      uint2 *ev = d.ev + (size_t)j * cap;
+      const bool merged = n <= 32    ? heavy_sort_one<1>(d, j, ev, n, t, D, N, cap, lane, s_ws[warp])
+                          : n <= 64  ? heavy_sort_one<2>(d, j, ev, n, t, D, N, cap, lane, s_ws[warp])
+                          : n <= 128 ? heavy_sort_one<4>(d, j, ev, n, t, D, N, cap, lane, s_ws[warp])
+                                     : heavy_sort_one<8>(d, j, ev, n, t, D, N, cap, lane, s_ws[warp]);
+      if (merged && lane == 0) s_n[k] = n | HEAVY_MERGED;
+    }
+    __syncthreads();
+  }
+  if (warp == 0) {
+    uint32_t mine = 0;
+    if (lane < nh) {
+      const uint32_t j = s_i[lane], n = s_n[lane] & ~HEAVY_MERGED;
+      const uint2 *ev = d.ev + (size_t)j * cap;
+      const int fired =
+          (s_n[lane] & HEAVY_MERGED)
+              ? run_neuron_merged(d, j, t, reinterpret_cast<const double2 *>(ev), n + d.bath_at[j].y)
+              : run_neuron(d, j, t, reinterpret_cast<const double *>(ev), reinterpret_cast<const float *>(ev + cap / 2), n);
+      if (fired) mine = 1u << (j & 31);
+    }
+    bits |= __reduce_or_sync(0xffffffffu, mine);
+    if (lane == 0) d.fired_bits[blockIdx.x] = bits;
+  }
+}
+
+// Neurons beyond the warp path, sorted by blocks and then run a thread each,
+// and the end of the step (the last block to finish).
+__global__ void __launch_bounds__(HEAVY_THREADS) tail_small_kernel(Dev d) {
+  __shared__ uint32_t s_last;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  const NetConst *net = d.net;
+  const uint32_t N = net->N, nh = min(d.heavy_cnt[1], N);
+  if (nh) {
+    const uint32_t t = *d.t, cap = net->ev_cap;
+    auto fired = [&](uint32_t i) { atomicOr(&d.fired_bits[i >> 5], 1u << (i & 31)); };
+    huge_sort(d, fired);
+    __syncthreads();
+    for (uint32_t hh = blockIdx.x + gridDim.x * threadIdx.x; hh < nh; hh += gridDim.x * blockDim.x) {
+      const uint32_t i = d.heavy_list[2ull * N + hh], ns = d.heavy_list[3ull * N + hh];
+      if (!huge_runs_here(net, ns)) continue;
+      const uint2 *ev = d.ev + (size_t)i * cap;
+      if (run_neuron(d, i, t, reinterpret_cast<const double *>(ev), reinterpret_cast<const float *>(ev + cap / 2), ns))
+        fired(i);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(d.ticket, 1u) == gridDim.x - 1;
+    if (s_last) {
+      *d.ticket = 0;
+      *d.ovf_cnt = 0;
+      d.heavy_cnt[0] = 0;
+      d.heavy_cnt[1] = 0;
+      *d.t = *d.t + 1;
+    }
   }
 }
 
@@ -2560,10 +2879,9 @@ struct dpsnn_engine {
   cudaStream_t bath_stream = nullptr;
   cudaEvent_t ev_bath[2] = {nullptr, nullptr}, ev_neuron[2] = {nullptr, nullptr}, ev_start = nullptr;
   bool bath_primed = false;
-  double *nb2[2] = {nullptr, nullptr}, *bath_time2[2] = {nullptr, nullptr};
-  uint8_t *bath_lut2[2] = {nullptr, nullptr};
-  uint32_t *bath_off2[2] = {nullptr, nullptr};
-  uint16_t *bath_cnt2[2] = {nullptr, nullptr};
+  double *nb2[2] = {nullptr, nullptr};
+  double2 *bath_ev2[2] = {nullptr, nullptr};
+  uint2 *bath_at2[2] = {nullptr, nullptr};
   int device = 0;
   uint64_t S = 0;
   uint32_t t_host = 0;   // steps enqueued
@@ -2574,7 +2892,7 @@ struct dpsnn_engine {
   std::vector<void *> allocs;
   std::vector<void *> temps;       // build scratch, released when the build ends
   uint64_t bytes = 0;              // device memory held (allocs)
-  uint32_t grid_neuron = 0, grid_deliver = 0, grid_heavy = 0, grid_heavy_run = 0, grid_huge = 0;
+  uint32_t grid_neuron = 0, grid_deliver = 0, grid_heavy = 0, grid_heavy_run = 0, grid_huge = 0, grid_tail = 0;
   int sms = 148;                   // the device's SMs (default grids)
   int timing = 0;
   bool capturing = false;          // steps are being recorded into a graph
@@ -2592,6 +2910,26 @@ struct dpsnn_engine {
 };
 
 static void collect_timings(dpsnn_engine *e);
+
+// The rule between a step's two forms.  The small one is faster at every size
+// its fired bits allow (per step, settled: 16 000 neurons in 64 ranks 34 us
+// against 53, 30 173 in 143 ranks 39 against 63, 100 in one 19 against 45),
+// except for a network that waits for long ranks' baths anyway and whose update
+// is large enough to slow them beside it (30 173 in 11 ranks: 102 against 97).
+static bool small_form(uint64_t neurons, uint64_t rank_neurons) {
+  return neurons <= SMALL_N && (neurons <= SMALL_N / 2 || rank_neurons <= 2048);
+}
+
+// The grids that dpsnn_set_launch_shape sets (0: the default).  The
+// delivery's default is a warp per four neurons, up to eight blocks per SM:
+// a spike's 20 or so segments are items of its warps, and a small network's
+// further blocks would only look for items.
+static void default_grids(dpsnn_engine *e, uint32_t deliver, uint32_t heavy_sort, uint32_t heavy_run) {
+  const uint32_t sms = (uint32_t)e->sms;
+  e->grid_deliver = deliver ? deliver : std::max(4u, std::min(sms * 8, (e->hnet.N + 31) / 32));
+  e->grid_heavy = heavy_sort ? heavy_sort : sms * 8;
+  e->grid_heavy_run = heavy_run ? heavy_run : sms * 16;
+}
 
 // Device allocations are stream-ordered on the engine stream (the
 // device's memory pool): unlike cudaMalloc/cudaFree they do not synchronise
@@ -3045,6 +3383,9 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     n.Tarp[s] = p->Tarp[s];
     n.AlphaC[s] = p->AlphaC[s];
     n.TauC[s] = p->TauC[s];
+    auto reciprocal = [](double x) { return x > 1e-100 && x < 1e100 ? 1.0 / x : 0.0; };
+    n.r_tau[s] = reciprocal(n.Tau[s]);
+    n.r_tauC[s] = reciprocal(n.TauC[s]);
     n.gC[s] = p->gC[s];
     n.NuExt[s] = p->NuExt[s];
     for (uint32_t t = 0; t < n.nsub; t++) {
@@ -3138,6 +3479,8 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   DALLOC(d.last_spike_ms, N);
   e->grid_neuron = (N + NEURON_BLOCK - 1) / NEURON_BLOCK;
   DALLOC(d.block_fired, e->grid_neuron);
+  DALLOC(d.fired_bits, (N + 31) / 32);
+  DALLOC(d.ticket, 1);
 
   // ---- synapse generation
   const uint32_t SD = p->stencil_dim;
@@ -3251,15 +3594,11 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     DALLOC(d.bath_rank_base, P + 1);
     CK(cudaMemcpyAsync(d.bath_rank_base, base.data(), 8ull * (P + 1), cudaMemcpyHostToDevice, e->stream));
     for (int b = 0; b < 2; b++) {
-      DALLOC(e->bath_time2[b], base[P]);
-      DALLOC(e->bath_lut2[b], base[P]);
-      DALLOC(e->bath_off2[b], N);
-      DALLOC(e->bath_cnt2[b], N);
+      DALLOC(e->bath_ev2[b], base[P]);   // below 2^25 * BATH_MAX_EXT < 2^32
+      DALLOC(e->bath_at2[b], N);
     }
-    d.bath_time = e->bath_time2[0];
-    d.bath_lut = e->bath_lut2[0];
-    d.bath_off = e->bath_off2[0];
-    d.bath_cnt = e->bath_cnt2[0];
+    d.bath_ev = e->bath_ev2[0];
+    d.bath_at = e->bath_at2[0];
     // dynamics streams: SetRandomSeed(loc_h) (DPSNN_localNet_init.c:283).
     // Rank 0 continues its generation stream; others re-initialise.
     std::vector<uint32_t> hist((size_t)P * BATH_HIST);
@@ -3308,9 +3647,8 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
   e->sms = sms;
-  e->grid_deliver = (uint32_t)sms * 8;
-  e->grid_heavy = (uint32_t)sms * 8;
-  e->grid_heavy_run = (uint32_t)sms * 16;
+  default_grids(e, 0, 0, 0);
+  e->grid_tail = std::min<uint32_t>((uint32_t)sms, (N + 255) / 256);
   e->grid_huge = (uint32_t)sms;
   free_temps(e);   // after their last use on this stream
   CK(cudaStreamSynchronize(e->stream));
@@ -3329,13 +3667,20 @@ extern "C" int dpsnn_create(const dpsnn_params *p, const dpsnn_options *opts, dp
   } else {
     cudaGetDevice(&e->device);
   }
-  // The bath of the next step runs beside this step's kernels and has a
-  // step of slack; the main stream's blocks go first when both wait for room.
+  // The bath of the next step runs beside this step's kernels.  A network that
+  // fills the GPU waits for its main stream, whose blocks go first when both
+  // wait for room; a small one for its bath, whose few blocks would otherwise
+  // wait for the update's to drain (16 000 neurons in 64 busy ranks: 76 us per
+  // step against 67).
+  uint64_t npcm = 0;
+  for (uint32_t s = 0; s < std::min<uint32_t>(p->nsub, DPSNN_MAX_SUBPOP); s++) npcm += p->count[s];
+  const uint64_t neurons = npcm * p->cfx * p->cfy;
+  const bool small = small_form(neurons, p->glob_h ? neurons / p->glob_h : 0);
   int prio_least = 0, prio_greatest = 0;
   bool ok = cudaSetDevice(e->device) == cudaSuccess &&
             cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest) == cudaSuccess &&
-            cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, prio_greatest) == cudaSuccess &&
-            cudaStreamCreateWithPriority(&e->bath_stream, cudaStreamNonBlocking, prio_least) == cudaSuccess;
+            cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, small ? prio_least : prio_greatest) == cudaSuccess &&
+            cudaStreamCreateWithPriority(&e->bath_stream, cudaStreamNonBlocking, small ? prio_greatest : prio_least) == cudaSuccess;
   for (int b = 0; b < 2 && ok; b++)
     ok = cudaEventCreateWithFlags(&e->ev_bath[b], cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&e->ev_neuron[b], cudaEventDisableTiming) == cudaSuccess;
@@ -3456,58 +3801,114 @@ static void enqueue_bath(dpsnn_engine *e, uint32_t t) {
   const int b = t & 1;
   db.nb_prev = e->nb2[b ^ 1];
   db.nb = e->nb2[b];
-  db.bath_time = e->bath_time2[b];
-  db.bath_lut = e->bath_lut2[b];
-  db.bath_off = e->bath_off2[b];
-  db.bath_cnt = e->bath_cnt2[b];
+  db.bath_ev = e->bath_ev2[b];
+  db.bath_at = e->bath_at2[b];
   cudaStreamWaitEvent(e->bath_stream, e->ev_neuron[b], 0);
   timed_launch_begin(e, 2, e->bath_stream);
   // each rank's block keeps its step in d.bath_t (baths are launched in step order)
   bath_kernel<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
+  e->launches++;
   timed_launch_end(e, 2);
   cudaEventRecord(e->ev_bath[b], e->bath_stream);
 }
 
-static int enqueue_step(dpsnn_engine *e) {
-  const uint32_t t = e->t_host;
-  const int b = t & 1;
-  if (!e->bath_primed) {   // the first bath waits for the network build
-    cudaEventRecord(e->ev_start, e->stream);
-    cudaStreamWaitEvent(e->bath_stream, e->ev_start, 0);
-    enqueue_bath(e, t);
-    e->bath_primed = true;
-    e->launches++;
-  }
-  enqueue_bath(e, t + 1);
-  if (e->d.stdp_log) {
-    cudaMemsetAsync(e->d.stdp_log_cnt, 0, 4, e->stream);
-    e->stdp_log_t = t;
-  }
-  Dev d = e->d;
-  d.bath_time = e->bath_time2[b];
-  d.bath_lut = e->bath_lut2[b];
-  d.bath_off = e->bath_off2[b];
-  d.bath_cnt = e->bath_cnt2[b];
-  timed_launch_begin(e, 0);
-  compact_kernel<<<e->grid_neuron, NEURON_BLOCK, 0, e->stream>>>(d);
-  timed_launch_end(e, 0);
-  // slot t is final (inside a graph: an event the graph records on every run)
+// A kernel of the main stream.  With `early` it may be brought up while the
+// kernel before it on the stream still runs (it starts by waiting for that
+// kernel's end): the gap between two dependent kernels is then about 1 us.
+template <typename K>
+static void launch_main(dpsnn_engine *e, K kernel, uint32_t grid, uint32_t block, const Dev &d, bool early) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.stream = e->stream;
+  cudaLaunchAttribute a[1];
+  a[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = a;
+  c.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, d);
+  e->launches++;
+}
+
+// Slot t of the ring is final: spike lists may be read (inside a graph: an
+// event the graph records on every run).
+static void record_slot(dpsnn_engine *e, uint32_t t) {
   if (e->capturing)
     cudaEventRecordWithFlags(e->ev_slot[t % RING_SLOTS], e->stream, cudaEventRecordExternal);
   else
     cudaEventRecord(e->ev_slot[t % RING_SLOTS], e->stream);
+}
+
+// The plasticity kernels around the delivery and after the update.
+static void enqueue_causal(dpsnn_engine *e, const Dev &d) {
+  timed_launch_begin(e, 4);
+  causal_stdp_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
+  timed_launch_end(e, 4);
+  e->launches++;
+}
+static void enqueue_anti_log(dpsnn_engine *e, const Dev &d) {
+  if (!d.stdp_log) return;
+  stdp_anti_log_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
+  e->launches++;
+}
+static void enqueue_ltp(dpsnn_engine *e, const Dev &d, uint32_t t) {
+  if (d.probe_w && t % 1000 == 999 && t >= e->hnet.start_pl && t <= e->hnet.stop_pl) e->probe_t = t;
+  timed_launch_begin(e, 4);
+  ltp_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
+  timed_launch_end(e, 4);
+  e->launches++;
+}
+
+// A small network's step: three kernels.  Bath t+1 writes the buffers that
+// step t-1 read, and follows step t's delivery.
+static void enqueue_small(dpsnn_engine *e, const Dev &d, uint32_t t) {
+  const int b = t & 1;
   if (e->hnet.stdp_on) {
-    timed_launch_begin(e, 4);
-    causal_stdp_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
-    timed_launch_end(e, 4);
+    timed_launch_begin(e, 0);
+    launch_main(e, compact_small_kernel, std::min<uint32_t>(e->grid_deliver, 32), DELIVER_THREADS, d, true);
+    timed_launch_end(e, 0);
+    record_slot(e, t);
+    enqueue_causal(e, d);
+    timed_launch_begin(e, 1);
+    launch_main(e, deliver_kernel, e->grid_deliver, DELIVER_THREADS, d, false);
+    timed_launch_end(e, 1);
+    enqueue_anti_log(e, d);
+  } else {
+    timed_launch_begin(e, 1);
+    launch_main(e, deliver_small_kernel, e->grid_deliver, DELIVER_THREADS, d, true);
+    timed_launch_end(e, 1);
+    record_slot(e, t);
   }
+  cudaEventRecord(e->ev_neuron[b ^ 1], e->stream);
+  enqueue_bath(e, t + 1);
+  cudaStreamWaitEvent(e->stream, e->ev_bath[b], 0);
+  timed_launch_begin(e, 3);
+  // four warps per 32 neurons while all the blocks are resident at once (four
+  // per SM), then two
+  const uint32_t blocks = (e->hnet.N + 31) / 32;
+  if (blocks <= 4 * (uint32_t)e->sms)
+    launch_main(e, neuron_small_kernel<4>, blocks, 128, d, false);
+  else
+    launch_main(e, neuron_small_kernel<2>, blocks, 64, d, false);
+  timed_launch_end(e, 3);
+  if (e->hnet.stdp_on) enqueue_ltp(e, d, t);
+  timed_launch_begin(e, 7);
+  launch_main(e, tail_small_kernel, e->grid_tail, HEAVY_THREADS, d, !e->hnet.stdp_on);
+  timed_launch_end(e, 7);
+}
+
+static void enqueue_large(dpsnn_engine *e, const Dev &d, uint32_t t) {
+  const int b = t & 1;
+  enqueue_bath(e, t + 1);
+  timed_launch_begin(e, 0);
+  compact_kernel<<<e->grid_neuron, NEURON_BLOCK, 0, e->stream>>>(d);
+  timed_launch_end(e, 0);
+  record_slot(e, t);
+  if (e->hnet.stdp_on) enqueue_causal(e, d);
   timed_launch_begin(e, 1);
   deliver_kernel<<<e->grid_deliver, DELIVER_THREADS, 0, e->stream>>>(d);
   timed_launch_end(e, 1);
-  if (d.stdp_log) {
-    stdp_anti_log_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
-    e->launches++;
-  }
+  enqueue_anti_log(e, d);
   cudaStreamWaitEvent(e->stream, e->ev_bath[b], 0);
   timed_launch_begin(e, 3);
   neuron_kernel<<<e->grid_neuron, NEURON_BLOCK, 0, e->stream>>>(d);
@@ -3526,14 +3927,31 @@ static int enqueue_step(dpsnn_engine *e) {
   heavy_rest_kernel<<<e->grid_huge, 128, 0, e->stream>>>(d);
   timed_launch_end(e, 7);
   cudaEventRecord(e->ev_neuron[b], e->stream);
-  if (e->hnet.stdp_on) {
-    if (d.probe_w && t % 1000 == 999 && t >= e->hnet.start_pl && t <= e->hnet.stop_pl) e->probe_t = t;
-    timed_launch_begin(e, 4);
-    ltp_kernel<<<e->grid_deliver, 256, 0, e->stream>>>(d);
-    timed_launch_end(e, 4);
-  }
+  if (e->hnet.stdp_on) enqueue_ltp(e, d, t);
   end_step_kernel<<<1, 1, 0, e->stream>>>(d);
-  e->launches += 10 + (e->hnet.stdp_on ? 2 : 0);
+  e->launches += 9;
+}
+
+static int enqueue_step(dpsnn_engine *e) {
+  const uint32_t t = e->t_host;
+  const int b = t & 1;
+  if (!e->bath_primed) {   // the first bath waits for the network build
+    cudaEventRecord(e->ev_start, e->stream);
+    cudaStreamWaitEvent(e->bath_stream, e->ev_start, 0);
+    enqueue_bath(e, t);
+    e->bath_primed = true;
+  }
+  if (e->d.stdp_log) {
+    cudaMemsetAsync(e->d.stdp_log_cnt, 0, 4, e->stream);
+    e->stdp_log_t = t;
+  }
+  Dev d = e->d;
+  d.bath_ev = e->bath_ev2[b];
+  d.bath_at = e->bath_at2[b];
+  if (small_form(e->hnet.N, e->hnet.locN))
+    enqueue_small(e, d, t);
+  else
+    enqueue_large(e, d, t);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return dpsnn_fail(DPSNN_E_CUDA, "kernel launch: %s", cudaGetErrorString(err));
   e->t_host++;
@@ -3722,9 +4140,7 @@ extern "C" int dpsnn_set_launch_shape(dpsnn_engine *e, uint32_t deliver_blocks, 
   const uint32_t lim = 1u << 20;
   if (deliver_blocks > lim || heavy_sort_blocks > lim || heavy_run_blocks > lim)
     return dpsnn_fail(DPSNN_E_PARAM, "a grid of more than %u blocks", lim);
-  e->grid_deliver = deliver_blocks ? deliver_blocks : (uint32_t)e->sms * 8;
-  e->grid_heavy = heavy_sort_blocks ? heavy_sort_blocks : (uint32_t)e->sms * 8;
-  e->grid_heavy_run = heavy_run_blocks ? heavy_run_blocks : (uint32_t)e->sms * 16;
+  default_grids(e, deliver_blocks, heavy_sort_blocks, heavy_run_blocks);
   return 0;
 }
 

@@ -82,9 +82,12 @@ def estimate_device_bytes(cfg: nc.NetConfig, events_per_neuron: int = 1024) -> i
         if p.count and p.NuExt > 0:
             inv = 1000.0 / (p.NuExt * cfg.bath_cext)
             max_ext = max(max_ext, math.ceil(20 / inv))
-    per_neuron = 66 + 2 * (cfg.D + 1) + 8 + 80 * 12 + 8 * cap + 20 + 12 + 2 * 9 * max_ext + 2 * 2 * cfg.D + 4
+    # the build's scratch: where each neuron's synapses start in its module's
+    # stream, under one or two hypotheses for NormDev's cache
+    starts = (1 if cfg.glob_h == cfg.n_modules else 2) * 236
+    per_neuron = 66 + 2 * (cfg.D + 1) + 8 + 80 * 12 + 8 * cap + 20 + 12 + 2 * (16 * max_ext + 8) + starts + 4
     per_syn = 6 + (12 if cfg.stdp is not None else 0)
-    fixed = (116 << 20) + cfg.glob_h * 90_000 + cfg.n_modules * 2 * 7500 * 4
+    fixed = (116 << 20) + cfg.glob_h * 1_100 + cfg.n_modules * 600
     return int(N * per_neuron + 1.1 * expected_synapses(cfg) * per_syn + fixed)
 
 
