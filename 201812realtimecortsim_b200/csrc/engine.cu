@@ -2869,6 +2869,52 @@ __global__ void group_extrema_kernel(const NetConst *net, const uint64_t *row_pt
     }
 }
 
+// Spike lists of a run of steps for the host, written straight into its
+// pinned memory: the error flags, the counts, and the lists one after another
+// when they fit.  One kernel and one wait; a copy per step and array cost
+// about 9 us each (80 steps of a small network: 240 copies, 2 ms).
+struct SpikeRead {
+  uint32_t flags, total;
+  uint32_t counts[RING_SLOTS];
+};
+static __host__ __device__ inline double *spike_read_te(SpikeRead *r) { return reinterpret_cast<double *>(r + 1); }
+static_assert(sizeof(SpikeRead) % 8 == 0, "the emission times follow, then the ids");
+#define READ_PACK_THREADS 256
+__global__ void __launch_bounds__(READ_PACK_THREADS) read_pack_kernel(Dev d, uint32_t t0, uint32_t n, uint32_t cap,
+                                                                      SpikeRead *out) {
+  __shared__ uint32_t s_pre[RING_SLOTS + 1];
+  const uint32_t N = d.net->N;
+  for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) s_pre[k + 1] = d.ring_cnt[(t0 + k) % RING_SLOTS];
+  __syncthreads();
+  if (blockIdx.x == 0)
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) out->counts[k] = s_pre[k + 1];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t acc = 0;   // at most RING_SLOTS * 2^25 < 2^32
+    s_pre[0] = 0;
+    for (uint32_t k = 1; k <= n; k++) s_pre[k] = acc += s_pre[k];
+    if (blockIdx.x == 0) {
+      out->flags = *d.flags;
+      out->total = acc;
+    }
+  }
+  __syncthreads();
+  const uint32_t total = s_pre[n];
+  if (total > cap) return;
+  double *te = spike_read_te(out);
+  uint32_t *ids = reinterpret_cast<uint32_t *>(te + cap);
+  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
+    uint32_t lo = 0, hi = n - 1;   // the last step that starts at or before g
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi + 1) >> 1;
+      if (s_pre[mid] <= g) lo = mid; else hi = mid - 1;
+    }
+    const size_t at = (size_t)((t0 + lo) % RING_SLOTS) * N + (g - s_pre[lo]);
+    te[g] = d.ring_te[at];
+    ids[g] = d.ring_ids[at];
+  }
+}
+
 // ------------------------------------------------------------------ host engine
 struct dpsnn_engine {
   NetConst hnet;
@@ -2902,7 +2948,9 @@ struct dpsnn_engine {
   double ktime[DPSNN_TIMING_SLOTS] = {};
   uint64_t klaunch[DPSNN_TIMING_SLOTS] = {};
   uint64_t launches = 0;               // kernels enqueued by dpsnn_step
-  uint32_t *h_pin = nullptr;          // pinned {flags, spike count} for per-step reads
+  uint32_t *h_pin = nullptr;          // pinned {flags, spike count} of dpsnn_rank_spikes_noalloc
+  SpikeRead *h_read = nullptr;        // pinned, mapped: what read_pack_kernel writes, h_read_cap spikes
+  uint32_t h_read_cap = 0;
   // spike lists are read on their own stream as soon as the compaction of
   // their step is done, while the rest of that step (and later ones) run
   cudaStream_t read_stream = nullptr;
@@ -3688,7 +3736,12 @@ extern "C" int dpsnn_create(const dpsnn_params *p, const dpsnn_options *opts, dp
   ok = ok && cudaStreamCreateWithFlags(&e->read_stream, cudaStreamNonBlocking) == cudaSuccess;
   for (int k = 0; k < RING_SLOTS && ok; k++)
     ok = cudaEventCreateWithFlags(&e->ev_slot[k], cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaMallocHost((void **)&e->h_pin, 2 * sizeof(uint32_t)) == cudaSuccess;
+  // the read buffer: what 80 steps of a network at rest make several times
+  // over (a burst's lists are copied one by one)
+  e->h_read_cap = (uint32_t)std::min<uint64_t>(32768, std::max<uint64_t>(1024, 4 * neurons));
+  const size_t read_bytes = sizeof(SpikeRead) + 12ull * e->h_read_cap;
+  ok = ok && cudaHostAlloc((void **)&e->h_read, read_bytes + 8, cudaHostAllocMapped) == cudaSuccess;
+  if (ok) e->h_pin = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(e->h_read) + read_bytes);
   if (!ok) {
     const int dev = e->device;
     dpsnn_destroy(e);
@@ -3726,7 +3779,7 @@ extern "C" void dpsnn_destroy(dpsnn_engine *e) {
     cudaStreamSynchronize(e->read_stream);
     cudaStreamDestroy(e->read_stream);
   }
-  if (e->h_pin) cudaFreeHost(e->h_pin);
+  if (e->h_read) cudaFreeHost(e->h_read);
   if (e->bath_stream) cudaStreamDestroy(e->bath_stream);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
@@ -4163,31 +4216,41 @@ extern "C" uint64_t dpsnn_events_delivered(const dpsnn_engine *e) {
   return v;
 }
 
+// The lists of steps t0 .. t0+n-1 (1 <= n <= RING_SLOTS) after the compaction
+// of the last of them (steps complete in order on the engine stream; the rest
+// of that step and later ones may still run): the error flags, the counts, and
+// whether the lists fitted the read buffer.
+static int read_lists(dpsnn_engine *e, uint32_t t0, uint32_t n, bool &packed) {
+  CK(cudaStreamWaitEvent(e->read_stream, e->ev_slot[(t0 + n - 1) % RING_SLOTS], 0));
+  read_pack_kernel<<<n == 1 ? 2 : 16, READ_PACK_THREADS, 0, e->read_stream>>>(e->d, t0, n, e->h_read_cap, e->h_read);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(e->read_stream));
+  packed = e->h_read->total <= e->h_read_cap;
+  return flags_error(e->h_read->flags);
+}
+static const uint32_t *read_ids(const dpsnn_engine *e) {
+  return reinterpret_cast<const uint32_t *>(spike_read_te(e->h_read) + e->h_read_cap);
+}
+
 extern "C" int dpsnn_spikes(dpsnn_engine *e, uint32_t t_ms, uint32_t *ids, double *te, uint32_t cap,
                             uint32_t *count) {
   if (!e || !count) return dpsnn_fail(DPSNN_E_PARAM, "null argument");
   if (t_ms >= e->t_host || t_ms + RING_SLOTS < e->t_host)
     return dpsnn_fail(DPSNN_E_STATE, "step %u is not among the last %d completed steps", t_ms, RING_SLOTS);
   cudaSetDevice(e->device);
-  const uint32_t slot = t_ms % RING_SLOTS;
-  // wait only for the compaction of step t_ms (the rest of that step and
-  // later steps may still run): one round trip for the error flags and the
-  // count, one for the list
-  CK(cudaStreamWaitEvent(e->read_stream, e->ev_slot[slot], 0));
-  CK(cudaMemcpyAsync(e->h_pin, e->d.flags, 4, cudaMemcpyDeviceToHost, e->read_stream));
-  CK(cudaMemcpyAsync(e->h_pin + 1, e->d.ring_cnt + slot, 4, cudaMemcpyDeviceToHost, e->read_stream));
-  CK(cudaStreamSynchronize(e->read_stream));
-  int rc = flags_error(e->h_pin[0]);
+  bool packed;
+  int rc = read_lists(e, t_ms, 1, packed);
   if (rc) return rc;
-  const uint32_t cnt = e->h_pin[1];
+  const uint32_t cnt = e->h_read->total, k = std::min(cnt, cap);
   *count = cnt;
-  const uint32_t k = std::min(cnt, cap);
-  if (k && ids)
-    CK(cudaMemcpyAsync(ids, e->d.ring_ids + (size_t)slot * e->hnet.N, 4ull * k, cudaMemcpyDeviceToHost,
-                       e->read_stream));
-  if (k && te)
-    CK(cudaMemcpyAsync(te, e->d.ring_te + (size_t)slot * e->hnet.N, 8ull * k, cudaMemcpyDeviceToHost,
-                       e->read_stream));
+  if (packed) {
+    if (ids) memcpy(ids, read_ids(e), 4ull * k);
+    if (te) memcpy(te, spike_read_te(e->h_read), 8ull * k);
+    return 0;
+  }
+  const size_t at = (size_t)(t_ms % RING_SLOTS) * e->hnet.N;
+  if (k && ids) CK(cudaMemcpyAsync(ids, e->d.ring_ids + at, 4ull * k, cudaMemcpyDeviceToHost, e->read_stream));
+  if (k && te) CK(cudaMemcpyAsync(te, e->d.ring_te + at, 8ull * k, cudaMemcpyDeviceToHost, e->read_stream));
   if (k && (ids || te)) CK(cudaStreamSynchronize(e->read_stream));
   return 0;
 }
@@ -4200,20 +4263,18 @@ extern "C" int dpsnn_spikes_range(dpsnn_engine *e, uint32_t t0, uint32_t n, uint
     return dpsnn_fail(DPSNN_E_STATE, "steps %u..%u are not among the last %d completed steps", t0, t0 + n - 1,
                       RING_SLOTS);
   cudaSetDevice(e->device);
-  // after the compaction of the last step of the run (steps complete in
-  // order on the engine stream): the counts and the error flags, then the lists
-  CK(cudaStreamWaitEvent(e->read_stream, e->ev_slot[(t0 + n - 1) % RING_SLOTS], 0));
-  CK(cudaMemcpyAsync(e->h_pin, e->d.flags, 4, cudaMemcpyDeviceToHost, e->read_stream));
-  for (uint32_t k = 0; k < n; k++)
-    CK(cudaMemcpyAsync(counts + k, e->d.ring_cnt + (t0 + k) % RING_SLOTS, 4, cudaMemcpyDeviceToHost,
-                       e->read_stream));
-  CK(cudaStreamSynchronize(e->read_stream));
-  int rc = flags_error(e->h_pin[0]);
+  bool packed;
+  int rc = read_lists(e, t0, n, packed);
+  memcpy(counts, e->h_read->counts, 4ull * n);
   if (rc) return rc;
-  uint64_t off = 0;
-  for (uint32_t k = 0; k < n; k++) off += counts[k];
+  uint64_t off = e->h_read->total;
   if (off > cap) return dpsnn_fail(DPSNN_E_CAPACITY, "%llu spikes in steps %u..%u exceed the buffers (%llu)",
                                    (unsigned long long)off, t0, t0 + n - 1, (unsigned long long)cap);
+  if (packed) {
+    memcpy(ids, read_ids(e), 4ull * off);
+    memcpy(te, spike_read_te(e->h_read), 8ull * off);
+    return 0;
+  }
   off = 0;
   for (uint32_t k = 0; k < n; k++) {
     const size_t slot = (t0 + k) % RING_SLOTS;
