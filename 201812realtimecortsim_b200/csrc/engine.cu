@@ -928,7 +928,8 @@ struct Dev {
   uint32_t *heavy_list, *heavy_cnt;   // [4N]: neuron, event count of the warp path, then of
                                       // the block path; heavy_cnt[0..1]: their lengths
   // bath
-  uint32_t *bath_hist;      // [P][BATH_HIST] the draws before each rank's next one
+  uint32_t *bath_hist;      // [P][BATH_KEEP] the BATH_HIST draws before each rank's next one, and some after
+  uint32_t *bath_kept;      // [P] their number
   uint64_t *bath_rank_base; // [P+1]
   uint2 *bath_at;           // [N] first bath event of this step, and their number
   double2 *bath_ev;         // {time, input} per bath event
@@ -1346,7 +1347,8 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
 #define BATH_PAIRS 2048        // pairs resident: two rounds behind (the emitters' and the walk's own), and ahead
 #define BATH_MIRROR 1024       // the ring's first words again past its end: a round's reads do not wrap
 #define BATH_RAW (2 * BATH_PAIRS)   // raw draws resident
-#define BATH_HIST 256          // raw draws kept between launches (the generator reads 220 back)
+#define BATH_HIST 256          // raw draws kept between launches (the generator reads 220 back),
+#define BATH_KEEP 640          // and as many of those ahead as there are, up to 384: the first round converts them
 #define BATH_ACT 512           // queued neurons: those being emitted, decided and prepared
 #define BATH_CONV 192          // pairs converted at a time: 2 per lane of three warps
 #define BATH_AHEAD 960         // pairs converted ahead of the decided ones, at most
@@ -1382,7 +1384,7 @@ struct BathSmem {
   float lap[BATH_PAIRS];
   uint8_t idx[BATH_PAIRS];
   double a_nb[BATH_ACT], a_inv[BATH_ACT];   // queued neuron a at a % BATH_ACT
-  uint4 a_b[BATH_ACT];              // bounds lo and hi - lo, min(cap, 16), cap
+  uint4 a_b[BATH_ACT + BATH_SEG];   // bounds lo and hi - lo, the latter for the mappers, cap; mirrored at the end
   uint32_t a_id[BATH_ACT];          // neuron of the rank, its sub-population in the top bits
   uint32_t a_t[BATH_ACT];           // expected q advance of the queued neurons before a (2^-20 units)
   uint2 pack[BATH_SEGS][BATH_NC];   // a segment's counts less one, a nibble per neuron, by candidate
@@ -1510,6 +1512,26 @@ __device__ static inline uint32_t bath_singles(const Dev &d, const BathSmem &s, 
   return n;
 }
 
+// One neuron of a mapper's segment from its lane's candidate (pair p, whose
+// q is qm): 1 + the number of sums of 1..16 lapses below lo, by fours, then
+// within the four.  Returns the count less one.
+__device__ __forceinline__ uint32_t bath_count(const BathSmem &s, const uint4 &k, uint32_t &p, uint32_t &qm,
+                                               uint32_t &bad) {
+  const uint32_t T = qm + k.x;
+  const uint32_t x =
+      p + 4 * (((s.q[p + 4] - T) >> 31) + ((s.q[p + 8] - T) >> 31) + ((s.q[p + 12] - T) >> 31));
+  const uint32_t y1 = s.q[x + 1] - T, y2 = s.q[x + 2] - T, y3 = s.q[x + 3] - T, y4 = s.q[x + 4] - T;
+  const uint32_t e = x + (y1 >> 31) + (y2 >> 31) + (y3 >> 31) + (y4 >> 31), c = e - p;
+  // the first sum not below lo, less lo: the negative ones are large unsigned
+  const uint32_t over = min(min(y1, y2), min(y3, y4));
+  // undecided, in bad's top bit: the sum lies between lo and hi, or none of
+  // the sixteen reaches lo (k.z: hi - lo, or 2^31 where the cap is below 16)
+  bad |= over - k.z;
+  qm = T + over;
+  p = e + 1;
+  return c;
+}
+
 // Mapper w: its segment's end and counts from every candidate start.
 __device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t w, uint32_t lane) {
   const uint32_t A = BATH_ACT - 1, a0 = cur.a + BATH_SEG * w;
@@ -1526,90 +1548,72 @@ __device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t
         first + 4 * __popc(__ballot_sync(0xffffffffu, at <= lim && (int32_t)(s.q[b + at] - T) < 0)) - 2;
     win = max(pred, (uint32_t)BATH_NC / 2) - BATH_NC / 2;
   }
-  uint32_t p = b + win + lane, qm = s.q[p];
-  uint32_t pk = 0, pk0 = 0;
-  bool bad = false;
-  uint4 nb = s.a_b[a0 & A];
+  uint32_t p = b + win + lane, qm = s.q[p], bad = 0;
+  uint2 pk = make_uint2(0, 0);
+  const uint4 *k = &s.a_b[a0 & A];   // mirrored past the ring's end
+  if (n == BATH_SEG) {
+#pragma unroll
+    for (int j = 0; j < 8; j++) pk.x += bath_count(s, k[j], p, qm, bad) << (4 * j);
+#pragma unroll
+    for (int j = 0; j < 8; j++) pk.y += bath_count(s, k[8 + j], p, qm, bad) << (4 * j);
+  } else {
 #pragma unroll 1
-  for (uint32_t j = 0; j < n; j++) {
-    // the neuron's count: 1 + the number of sums of 1..16 lapses below lo,
-    // by fours, then within the four
-    const uint4 k = nb;
-    nb = s.a_b[(a0 + j + 1) & A];
-    const uint32_t T = qm + k.x;
-    const uint32_t n4 = ((s.q[p + 4] - T) >> 31) + ((s.q[p + 8] - T) >> 31) + ((s.q[p + 12] - T) >> 31);
-    const uint32_t x = p + 4 * n4;
-    const uint32_t y1 = s.q[x + 1] - T, y2 = s.q[x + 2] - T, y3 = s.q[x + 3] - T, y4 = s.q[x + 4] - T;
-    const uint32_t e = x + (y1 >> 31) + (y2 >> 31) + (y3 >> 31) + (y4 >> 31), c = e - p;
-    // the first sum not below lo, less lo: the negative ones are large unsigned
-    const uint32_t over = min(min(y1, y2), min(y3, y4));
-    // undecided: the sum lies between lo and hi, or the count is beyond
-    // sixteen or the neuron's cap
-    bad |= c >= k.z || over < k.y;
-    qm = T + over;
-    p = e + 1;
-    pk |= c << (4 * (j & 7));
-    if (j == 7) {
-      pk0 = pk;
-      pk = 0;
+    for (uint32_t j = 0; j < n; j++) {
+      const uint32_t c = bath_count(s, k[j], p, qm, bad) << (4 * (j & 7));
+      if (j < 8) pk.x += c; else pk.y += c;
     }
   }
   // an end within 16 pairs of the converted ones may rest on stale words
   const uint32_t e = p - b;
-  s.end[w][lane] = (uint16_t)(e + 16 > lim ? BATH_NOT_YET : bad ? BATH_UNDECIDED : e - win);
-  s.pack[w][lane] = n > 7 ? make_uint2(pk0, pk) : make_uint2(pk, 0u);
+  s.end[w][lane] = (uint16_t)(e + 16 > lim ? BATH_NOT_YET : (int32_t)bad < 0 ? BATH_UNDECIDED : e - win);
+  s.pack[w][lane] = pk;
   if (lane == 0) {
     reinterpret_cast<uint32_t *>(s.win)[w] = cur.m + win;
     s.end[w][BATH_NC] = BATH_NOT_YET;
   }
 }
 
-// Warp 0, the segments mapped: the chain over them, and the next round's
-// start.  A segment with no decided entry at its start runs neuron by
-// neuron: the sums of 1..32 lapses by lane and a vote, or the reference's
-// loop.
+// Every mapper, the segments mapped: the chain over them.  Each hands its own
+// segment over if the chain reaches it decided; warp 0 also writes the next
+// round's start.  A segment with no decided entry at its start runs neuron
+// by neuron (warp 0) and ends the round: the sums of 1..32 lapses by lane and
+// a vote, or the reference's loop.
 __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const BathCtl &cur, BathCtl &nxt, uint32_t par,
-                                           double T1, uint32_t lane) {
-  const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1, lim = cur.conv_end;
+                                           double T1, uint32_t w, uint32_t lane) {
+  const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1;
   const uint32_t left = cur.rebase ? 0u : min(cur.act_end - cur.a, (uint32_t)BATH_SB);
   const uint32_t nseg = (left + BATH_SEG - 1) / BATH_SEG;
-  uint32_t m = cur.m, n_done = 0, rebase = 0, slow = 0;
   const uint4 wa = s.win[0], wb = s.win[1];
   const uint32_t win[BATH_SEGS] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-  for (uint32_t g0 = 0; g0 < nseg;) {
-    // the chain over the segments from g0 on (a start outside the window
-    // finds the sentinel); lane g keeps segment g's start
-    uint32_t my_m = 0, my_w = 0, P = m;
+  // a start outside a segment's window finds the sentinel, and so does, from
+  // there on, every later segment
+  uint32_t st[BATH_SEGS + 1], undec = 0;
+  st[0] = cur.m;
 #pragma unroll
-    for (uint32_t g = 0; g < BATH_SEGS; g++) {
-      const uint32_t e = win[g] + s.end[g][min(P - win[g], (uint32_t)BATH_NC)];
-      my_m = lane == g ? P : my_m;
-      my_w = lane == g ? win[g] : my_w;
-      P = g >= g0 && g < nseg ? e : P;
-    }
-    const bool mine = lane >= g0 && lane < nseg;
-    const uint32_t my_o = min(my_m - my_w, (uint32_t)BATH_NC), my_e = mine ? s.end[lane][my_o] : 0u;
-    const uint32_t g1 = min((uint32_t)__ffs(__ballot_sync(0xffffffffu, my_e >= BATH_NOT_YET)) - 1u, nseg);
-    if (mine && lane < g1) {
-      s.e_start[par][lane] = my_m;
-      s.e_pack[par][lane] = s.pack[lane][my_o];
-    }
-    n_done = min(g1 * BATH_SEG, left);
-    if (g1 == nseg) {
-      m = P;
-      break;
-    }
-    m = __shfl_sync(0xffffffffu, my_m, g1);
-    if (__shfl_sync(0xffffffffu, my_e, g1) == BATH_NOT_YET) break;
-    slow |= 1u << g1;
-    const uint32_t n_end = min(n_done + BATH_SEG, left);
-    bool stop = false;
-    while (n_done < n_end && !stop) {
+  for (uint32_t g = 0; g < BATH_SEGS; g++) {
+    const uint32_t e = s.end[g][min(st[g] - win[g], (uint32_t)BATH_NC)];
+    undec |= (uint32_t)(e >= BATH_NOT_YET) << g;
+    st[g + 1] = win[g] + e;
+  }
+  const uint32_t stop_g = min((uint32_t)__ffs(undec) - 1u, nseg);
+  uint32_t m = st[0], my_m = st[0];
+#pragma unroll
+  for (uint32_t g = 1; g <= BATH_SEGS; g++) {
+    if (g == stop_g) m = st[g];
+    if (g == w) my_m = st[g];
+  }
+  if (w < stop_g && lane == 0) {
+    s.e_start[par][w] = my_m;
+    s.e_pack[par][w] = s.pack[w][my_m - reinterpret_cast<const uint32_t *>(s.win)[w]];
+  }
+  if (w) return;
+  uint32_t n_done = min(stop_g * BATH_SEG, left), rebase = 0, slow = 0;
+  if (stop_g < nseg && s.end[stop_g][min(m - reinterpret_cast<const uint32_t *>(s.win)[stop_g], (uint32_t)BATH_NC)] == BATH_UNDECIDED) {
+    slow = 1u << stop_g;
+    const uint32_t n_end = min(n_done + BATH_SEG, left), lim = cur.conv_end;
+    while (n_done < n_end && !rebase) {
       const uint32_t a = (cur.a + n_done) & A, mx = s.a_b[a].w, lo = s.a_b[a].x;
-      if (m + max(33u, mx + 1) > lim) {   // its pairs are not converted yet
-        stop = true;
-        break;
-      }
+      if (m + max(33u, mx + 1) > lim) break;   // its pairs are not converted yet
       uint32_t c = 0;
       const uint32_t F = s.q[(m + 1 + lane) & M] - s.q[m & M];
       const uint32_t mm = __popc(__ballot_sync(0xffffffffu, F < lo));
@@ -1623,7 +1627,6 @@ __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const Bath
         } while (v < T1 && c < mx);
         if (v < T1) {
           rebase = bath_singles(d, s, cur.base + 2 * (m + c), cur.raw_end, inv, T1, v);
-          stop = true;
           if (!rebase) break;   // draws not generated yet
         }
       }
@@ -1634,8 +1637,6 @@ __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const Bath
       m += c;
       n_done++;
     }
-    if (stop) break;
-    g0 = g1 + 1;
   }
   const uint32_t a = cur.a + n_done;
   if (lane == 0) {
@@ -1674,14 +1675,16 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
   const uint32_t ev_base = (uint32_t)d.bath_rank_base[h];
   // draws of this launch are numbered from BATH_HIST; the ones before are the
   // rank's kept history
-  for (uint32_t n = tid; n < BATH_HIST; n += BATH_THREADS) s.raw[n] = d.bath_hist[(size_t)h * BATH_HIST + n];
+  const uint32_t kept = d.bath_kept[h];
+  for (uint32_t n = tid; n < kept; n += BATH_THREADS) s.raw[n] = d.bath_hist[(size_t)h * BATH_KEEP + n];
   for (uint32_t r = tid; r < 256; r += BATH_THREADS) s.near[r] = d.fix_near[r];
   for (uint32_t r = tid; r < LOG_TAB_N; r += BATH_THREADS) s.log_tab[r] = d.log_tab[r];
   if (tid == 0) {
     s.q[0] = s.q[BATH_PAIRS] = 0;
     s.a_t[0] = 0;
     BathCtl c = {};
-    c.raw_end = c.base = BATH_HIST;
+    c.base = BATH_HIST;
+    c.raw_end = kept;
     s.ctl[0] = c;
   }
   // the preparers' next neurons, loaded an iteration ahead
@@ -1708,7 +1711,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
     if (warp < BATH_SEGS) {
       bath_map(s, cur, warp, lane);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the mappers
-      if (warp == 0) bath_compose(d, s, cur, nxt, r & 1, T1, lane);
+      bath_compose(d, s, cur, nxt, r & 1, T1, warp, lane);
     } else if (warp == 15) {
       // x[n] = x[n-55] - x[n-24] mod 1e9, applied four times over: x[n] = x[n-96] - 4 x[n-127] + 6 x[n-158]
       // - 4 x[n-189] + x[n-220], so that 96 draws follow from the ones before them at once; keeping BATH_HIST
@@ -1773,7 +1776,9 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           const uint32_t k = (e + pw * n0 + __popc(bal & ((1u << lane) - 1))) & A;
           s.a_nb[k] = nb;
           s.a_inv[k] = inv;
-          s.a_b[k] = make_uint4(lo, hi1 - lo, min(mx, 16u), mx);
+          const uint4 ab = make_uint4(lo, hi1 - lo, mx < 16 ? 0x80000000u : hi1 - lo, mx);
+          s.a_b[k] = ab;
+          if (k < BATH_SEG) s.a_b[k + BATH_ACT] = ab;
           s.a_id[k] = i | (sub << 25);
           s.a_t[k] = p_t + pw * t0 + incl - tv;
         } else if (i < locN) {
@@ -1865,10 +1870,13 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
     return;
   }
   // the history of the next launch: the draws before the first unused one
-  const uint32_t pos = fin.base + 2 * fin.m;
-  for (uint32_t n = tid; n < BATH_HIST; n += BATH_THREADS)
-    d.bath_hist[(size_t)h * BATH_HIST + n] = s.raw[(pos - BATH_HIST + n) % BATH_RAW];
-  if (tid == 0) d.bath_t[h] = t + 1;
+  const uint32_t pos = fin.base + 2 * fin.m, keep = BATH_HIST + min(fin.raw_end - pos, (uint32_t)(BATH_KEEP - BATH_HIST));
+  for (uint32_t n = tid; n < keep; n += BATH_THREADS)
+    d.bath_hist[(size_t)h * BATH_KEEP + n] = s.raw[(pos - BATH_HIST + n) % BATH_RAW];
+  if (tid == 0) {
+    d.bath_kept[h] = keep;
+    d.bath_t[h] = t + 1;
+  }
 }
 
 // LIFCADynamic, non-PerseoDyn branch (DPSNN_neuron_sim.c:664-824): lifca_pre
@@ -3649,7 +3657,7 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     d.bath_at = e->bath_at2[0];
     // dynamics streams: SetRandomSeed(loc_h) (DPSNN_localNet_init.c:283).
     // Rank 0 continues its generation stream; others re-initialise.
-    std::vector<uint32_t> hist((size_t)P * BATH_HIST);
+    std::vector<uint32_t> hist((size_t)P * BATH_KEEP), kept(P, BATH_HIST);
     for (uint32_t h = 0; h < P; h++) {
       uint32_t h55[55];
       if (h == 0) {
@@ -3681,13 +3689,15 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
       // h55 is x[-55..-1].  The neurons' draws start at x[1]: the history is
       // x[1-BATH_HIST..0], x[0] = x[-55] - x[-24] and the older ones by the
       // recurrence backwards, x[k] = x[k+55] + x[k+31] (mod MBIG)
-      uint32_t *x = &hist[(size_t)h * BATH_HIST] + BATH_HIST - 1;   // x[0]
+      uint32_t *x = &hist[(size_t)h * BATH_KEEP] + BATH_HIST - 1;   // x[0]
       for (int k = 0; k < 55; k++) x[k - 55] = h55[k];
       x[0] = x[-55] >= x[-24] ? x[-55] - x[-24] : x[-55] + MBIG - x[-24];
       for (int k = -56; k > -BATH_HIST; k--) x[k] = (uint32_t)(((uint64_t)x[k + 55] + x[k + 31]) % MBIG);
     }
-    DALLOC(d.bath_hist, (size_t)P * BATH_HIST);
-    CK(cudaMemcpyAsync(d.bath_hist, hist.data(), 4ull * P * BATH_HIST, cudaMemcpyHostToDevice, e->stream));
+    DALLOC(d.bath_hist, (size_t)P * BATH_KEEP);
+    DALLOC(d.bath_kept, P);
+    CK(cudaMemcpyAsync(d.bath_hist, hist.data(), 4ull * P * BATH_KEEP, cudaMemcpyHostToDevice, e->stream));
+    CK(cudaMemcpyAsync(d.bath_kept, kept.data(), 4ull * P, cudaMemcpyHostToDevice, e->stream));
     CK(cudaStreamSynchronize(e->stream));
   }
   int rc = load_logf_fixup(e);
