@@ -2640,6 +2640,11 @@ __global__ void __launch_bounds__(HEAVY_THREADS) huge_kernel(Dev d) {
 
 // A block of WARPS warps per 32 neurons: warp 0 runs the light ones while the
 // others (and then it too) sort the heavier ones, which then run a lane each.
+// Light: up to SMALL_LIGHT events.  A thread's insertion sort and merge of 16
+// take its warp 40 000 cycles, a warp's sort of as many 4000 and their run by
+// lanes half of the former (16 000 busy neurons: 60 us per step against 67 with
+// the line at 16; 3 and 9 are within 2 us of 6).
+#define SMALL_LIGHT 6
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) neuron_small_kernel(Dev d) {
   __shared__ HeavySortWarp s_ws[WARPS];
@@ -2658,7 +2663,7 @@ __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) neuron_small_kernel(De
       cnt = d.ev_cnt[i];
       if (cnt) d.ev_cnt[i] = 0;
     }
-    light = i < N && cnt <= net->light_max;
+    light = i < N && cnt <= min(net->light_max, (uint32_t)SMALL_LIGHT);
     const bool heavy = !light && cnt && cnt <= warp_path_max(net);
     const uint32_t bal = __ballot_sync(0xffffffffu, heavy);
     if (heavy) {
