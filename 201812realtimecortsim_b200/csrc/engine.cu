@@ -4331,16 +4331,14 @@ extern "C" int dpsnn_bath_params(dpsnn_engine *e, double *inv_nu_ext, uint32_t *
   return 0;
 }
 
-// Host-side view of the connectome for the reference-order backward list.
+// Host-side view of the connectome.
 struct HostCsr {
   std::vector<uint64_t> row;
   std::vector<uint16_t> so;
   std::vector<uint32_t> post;
   std::vector<int16_t> w;
-  std::vector<float> td;
-  std::vector<uint8_t> sub;
 };
-static int fetch_csr(dpsnn_engine *e, HostCsr &h, bool with_td) {
+static int fetch_csr(dpsnn_engine *e, HostCsr &h) {
   int rc = dpsnn_sync(e);
   if (rc) return rc;
   const uint32_t N = e->hnet.N, D = e->hnet.D;
@@ -4348,54 +4346,247 @@ static int fetch_csr(dpsnn_engine *e, HostCsr &h, bool with_td) {
   h.so.resize((size_t)N * (D + 1));
   h.post.resize(e->S);
   h.w.resize(e->S);
-  h.sub.resize(N);
   CK(cudaMemcpy(h.row.data(), e->d.row_ptr, 8ull * (N + 1), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.so.data(), e->d.sub_off, 2ull * N * (D + 1), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.post.data(), e->d.post, 4ull * e->S, cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(h.w.data(), e->d.w16, 2ull * e->S, cudaMemcpyDeviceToHost));
-  CK(cudaMemcpy(h.sub.data(), e->d.sub, N, cudaMemcpyDeviceToHost));
-  if (with_td && e->d.tderiv) {
-    h.td.resize(e->S);
-    CK(cudaMemcpy(h.td.data(), e->d.tderiv, 4ull * e->S, cudaMemcpyDeviceToHost));
-  }
   return 0;
+}
+
+// ------------------------------------------------------------------ a rank's synapse list
+// The reference's order (inflateIntermToBackwardSynList): delay, then
+// presynaptic neuron, then generation order, of the synapses aimed at one
+// rank.  On the device: the list's segments, one per (delay, presynaptic
+// neuron), are counted, summed and written in place, and only the rank's list
+// crosses to the host.  (The host walked a copy of the whole connectome, twice
+// with the count: 6 ms of a small network's dump, seconds of a large one's.)
+#define LIST_SCAN_THREADS 256
+#define LIST_SCAN_ITEMS 8
+#define LIST_SCAN_TILE (LIST_SCAN_THREADS * LIST_SCAN_ITEMS)
+// seg[dl * N + P]: synapses of the segment (P, dl) in the rank's neurons
+// [lo, hi), a warp per presynaptic neuron.
+__global__ void list_count_kernel(Dev d, uint32_t lo, uint32_t hi, uint32_t *__restrict__ seg) {
+  const uint32_t N = d.net->N, D = d.net->D, lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t P = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; P < N; P += nw) {
+    const uint64_t row = d.row_ptr[P];
+    const uint16_t *so = d.sub_off + (size_t)P * (D + 1);
+    for (uint32_t dl = 0; dl < D; dl++) {
+      const uint32_t b = so[dl], e = so[dl + 1];
+      uint32_t c = 0;
+      for (uint32_t k = b + lane; k < e; k += 32) {
+        const uint32_t j = d.post[row + k];
+        c += j >= lo && j < hi;
+      }
+      c = __reduce_add_sync(0xffffffffu, c);
+      if (lane == 0) seg[(size_t)dl * N + P] = c;
+    }
+  }
+}
+// Sums of tiles of LIST_SCAN_TILE segments, then each tile's base.
+__global__ void __launch_bounds__(LIST_SCAN_THREADS) list_sum_kernel(const uint32_t *__restrict__ seg, uint64_t n,
+                                                                     uint64_t *__restrict__ tile) {
+  __shared__ uint64_t s[LIST_SCAN_THREADS / 32];
+  uint64_t c = 0;
+  for (uint32_t k = threadIdx.x; k < LIST_SCAN_TILE; k += LIST_SCAN_THREADS) {
+    const uint64_t i = (uint64_t)blockIdx.x * LIST_SCAN_TILE + k;
+    if (i < n) c += seg[i];
+  }
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t w = 1; w < LIST_SCAN_THREADS / 32; w++) c += s[w];
+    tile[blockIdx.x] = c;
+  }
+}
+__global__ void list_base_kernel(uint64_t *tile, uint32_t n) {   // one warp: exclusive sums; the total at tile[n]
+  uint64_t acc = 0;
+  for (uint32_t i0 = 0; i0 < n; i0 += 32) {
+    const uint32_t i = i0 + threadIdx.x;
+    const uint64_t c = i < n ? tile[i] : 0;
+    uint64_t incl = c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (threadIdx.x >= (uint32_t)o) incl += y;
+    }
+    if (i < n) tile[i] = acc + incl - c;
+    acc += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  if (threadIdx.x == 0) tile[n] = acc;
+}
+// at[i]: first place of segment i.
+__global__ void __launch_bounds__(LIST_SCAN_THREADS) list_place_kernel(const uint32_t *__restrict__ seg, uint64_t n,
+                                                                       const uint64_t *__restrict__ tile,
+                                                                       uint64_t *__restrict__ at) {
+  __shared__ uint32_t s[LIST_SCAN_THREADS / 32];
+  const uint64_t i0 = (uint64_t)blockIdx.x * LIST_SCAN_TILE + threadIdx.x * LIST_SCAN_ITEMS;
+  uint32_t c[LIST_SCAN_ITEMS], sum = 0;
+  for (int k = 0; k < LIST_SCAN_ITEMS; k++) {
+    c[k] = i0 + k < n ? seg[i0 + k] : 0u;
+    sum += c[k];   // a tile holds below 2^32 synapses (2048 segments of at most 7500)
+  }
+  uint32_t incl = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((threadIdx.x & 31) >= (uint32_t)o) incl += y;
+  }
+  if ((threadIdx.x & 31) == 31) s[threadIdx.x >> 5] = incl;
+  __syncthreads();
+  uint64_t acc = tile[blockIdx.x] + incl - sum;
+  for (uint32_t w = 0; w < (threadIdx.x >> 5); w++) acc += s[w];
+  for (int k = 0; k < LIST_SCAN_ITEMS; k++)
+    if (i0 + k < n) {
+      at[i0 + k] = acc;
+      acc += c[k];
+    }
+}
+struct SynapseList {   // device arrays of one rank's list; null: not wanted
+  uint32_t *pre, *post;
+  uint8_t *delay, *kind;
+  int16_t *weight;
+  float *tderiv;
+};
+__global__ void list_fill_kernel(Dev d, uint32_t lo, uint32_t hi, const uint64_t *__restrict__ at, SynapseList l) {
+  const uint32_t N = d.net->N, D = d.net->D, lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t P = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; P < N; P += nw) {
+    const uint64_t row = d.row_ptr[P];
+    const uint16_t *so = d.sub_off + (size_t)P * (D + 1);
+    const uint8_t kind = d.sub[P];
+    for (uint32_t dl = 0; dl < D; dl++) {
+      const uint32_t b = so[dl], e = so[dl + 1];
+      uint64_t o0 = at[(size_t)dl * N + P];
+      for (uint32_t k0 = b; k0 < e; k0 += 32) {
+        const uint32_t k = k0 + lane, j = k < e ? d.post[row + k] : 0xFFFFFFFFu;
+        const bool in = k < e && j >= lo && j < hi;
+        const uint32_t bal = __ballot_sync(0xffffffffu, in);
+        if (in) {
+          const uint64_t o = o0 + __popc(bal & ((1u << lane) - 1));
+          if (l.pre) l.pre[o] = P;
+          if (l.post) l.post[o] = j;
+          if (l.delay) l.delay[o] = (uint8_t)dl;
+          if (l.kind) l.kind[o] = kind;
+          if (l.weight) l.weight[o] = d.w16[row + k];
+          if (l.tderiv) l.tderiv[o] = d.tderiv ? d.tderiv[row + k] : 0.0f;
+        }
+        o0 += __popc(bal);
+      }
+    }
+  }
+}
+
+// Stream-ordered scratch of one call.
+struct CallScratch {
+  dpsnn_engine *e;
+  std::vector<void *> held;
+  explicit CallScratch(dpsnn_engine *eng) : e(eng) {}
+  ~CallScratch() {
+    for (void *q : held) cudaFreeAsync(q, e->stream);
+  }
+  template <typename T>
+  int get(T **p, size_t n) {
+    void *q = nullptr;
+    const cudaError_t err = cudaMallocAsync(&q, std::max<size_t>(n * sizeof(T), 16), e->stream);
+    if (err != cudaSuccess) return dpsnn_fail(DPSNN_E_NOMEM, "cudaMallocAsync: %s", cudaGetErrorString(err));
+    held.push_back(q);
+    *p = (T *)q;
+    return 0;
+  }
+};
+
+// Rank h's list: its length, and with `out` its arrays (host; null: not
+// wanted).  DPSNN_E_NOMEM where the device has no room for the scratch (12
+// bytes per neuron and delay, and the list).
+static int rank_list_device(dpsnn_engine *e, uint32_t h, uint64_t *count, const SynapseList *out) {
+  int rc = 0;
+  const uint32_t N = e->hnet.N, D = e->hnet.D, lo = h * e->hnet.locN, hi = lo + e->hnet.locN;
+  const uint64_t nseg = (uint64_t)N * D;
+  const uint32_t tiles = (uint32_t)((nseg + LIST_SCAN_TILE - 1) / LIST_SCAN_TILE);
+  const uint32_t grid = std::min<uint32_t>((uint32_t)e->sms * 8, (N + 7) / 8);
+  CallScratch m(e);
+  uint32_t *seg;
+  uint64_t *tile, *at, n = 0;
+  if ((rc = m.get(&seg, nseg)) || (rc = m.get(&tile, tiles + 1))) return rc;
+  list_count_kernel<<<grid, 256, 0, e->stream>>>(e->d, lo, hi, seg);
+  list_sum_kernel<<<tiles, LIST_SCAN_THREADS, 0, e->stream>>>(seg, nseg, tile);
+  list_base_kernel<<<1, 32, 0, e->stream>>>(tile, tiles);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(&n, tile + tiles, 8, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  if (count) *count = n;
+  if (!out || !n) return 0;
+  SynapseList l = {};
+  if ((rc = m.get(&at, nseg))) return rc;
+  if (out->pre && (rc = m.get(&l.pre, n))) return rc;
+  if (out->post && (rc = m.get(&l.post, n))) return rc;
+  if (out->delay && (rc = m.get(&l.delay, n))) return rc;
+  if (out->kind && (rc = m.get(&l.kind, n))) return rc;
+  if (out->weight && (rc = m.get(&l.weight, n))) return rc;
+  if (out->tderiv && (rc = m.get(&l.tderiv, n))) return rc;
+  list_place_kernel<<<tiles, LIST_SCAN_THREADS, 0, e->stream>>>(seg, nseg, tile, at);
+  list_fill_kernel<<<grid, 256, 0, e->stream>>>(e->d, lo, hi, at, l);
+  CK(cudaGetLastError());
+  if (out->pre) CK(cudaMemcpyAsync(out->pre, l.pre, 4 * n, cudaMemcpyDeviceToHost, e->stream));
+  if (out->post) CK(cudaMemcpyAsync(out->post, l.post, 4 * n, cudaMemcpyDeviceToHost, e->stream));
+  if (out->delay) CK(cudaMemcpyAsync(out->delay, l.delay, n, cudaMemcpyDeviceToHost, e->stream));
+  if (out->kind) CK(cudaMemcpyAsync(out->kind, l.kind, n, cudaMemcpyDeviceToHost, e->stream));
+  if (out->weight) CK(cudaMemcpyAsync(out->weight, l.weight, 2 * n, cudaMemcpyDeviceToHost, e->stream));
+  if (out->tderiv) CK(cudaMemcpyAsync(out->tderiv, l.tderiv, 4 * n, cudaMemcpyDeviceToHost, e->stream));
+  CK(cudaStreamSynchronize(e->stream));
+  return 0;
+}
+
+// The same on the host, from a copy of the connectome.
+static int rank_list_host(dpsnn_engine *e, uint32_t h, uint64_t *count, const SynapseList *out) {
+  HostCsr c;
+  int rc = fetch_csr(e, c);
+  if (rc) return rc;
+  const uint32_t N = e->hnet.N, D = e->hnet.D, locN = e->hnet.locN;
+  std::vector<float> td;
+  std::vector<uint8_t> sub(N);
+  CK(cudaMemcpy(sub.data(), e->d.sub, N, cudaMemcpyDeviceToHost));
+  if (out && out->tderiv && e->d.tderiv) {
+    td.resize(e->S);
+    CK(cudaMemcpy(td.data(), e->d.tderiv, 4ull * e->S, cudaMemcpyDeviceToHost));
+  }
+  uint64_t o = 0;
+  for (uint32_t dl = 0; dl < D; dl++)
+    for (uint32_t P = 0; P < N; P++) {
+      const uint64_t b = c.row[P] + c.so[(size_t)P * (D + 1) + dl], en = c.row[P] + c.so[(size_t)P * (D + 1) + dl + 1];
+      for (uint64_t k = b; k < en; k++) {
+        if (c.post[k] / locN != h) continue;
+        if (out && out->pre) out->pre[o] = P;
+        if (out && out->post) out->post[o] = c.post[k];
+        if (out && out->delay) out->delay[o] = (uint8_t)dl;
+        if (out && out->kind) out->kind[o] = sub[P];
+        if (out && out->weight) out->weight[o] = c.w[k];
+        if (out && out->tderiv) out->tderiv[o] = td.empty() ? 0.0f : td[k];
+        o++;
+      }
+    }
+  if (count) *count = o;
+  return 0;
+}
+static int rank_list(dpsnn_engine *e, uint32_t h, uint64_t *count, const SynapseList *out) {
+  int rc = dpsnn_sync(e);
+  if (!rc) rc = rank_list_device(e, h, count, out);
+  if (rc != DPSNN_E_NOMEM) return rc;
+  cudaGetLastError();
+  return rank_list_host(e, h, count, out);
 }
 
 extern "C" uint64_t dpsnn_rank_synapse_count(dpsnn_engine *e, uint32_t h) {
   if (!e || h >= e->hnet.P) return 0;
-  HostCsr c;
-  if (fetch_csr(e, c, false)) return 0;
+  if (e->hnet.P == 1) return dpsnn_sync(e) ? 0 : e->S;
   uint64_t n = 0;
-  for (uint64_t k = 0; k < e->S; k++) n += (c.post[k] / e->hnet.locN == h);
-  return n;
+  return rank_list(e, h, &n, nullptr) ? 0 : n;
 }
 
 extern "C" int dpsnn_backward_synapses(dpsnn_engine *e, uint32_t h, uint32_t *pre, uint32_t *post, uint8_t *delay,
                                        uint8_t *kind, int16_t *weight, float *tderiv) {
   if (!e) return dpsnn_fail(DPSNN_E_PARAM, "null engine");
   if (h >= e->hnet.P) return dpsnn_fail(DPSNN_E_PARAM, "rank %u out of range", h);
-  HostCsr c;
-  int rc = fetch_csr(e, c, tderiv != nullptr);
-  if (rc) return rc;
-  // reference order (inflateIntermToBackwardSynList): delay, then source
-  // rank / presynaptic index, then generation order
-  const uint32_t N = e->hnet.N, D = e->hnet.D, locN = e->hnet.locN;
-  uint64_t o = 0;
-  for (uint32_t dl = 0; dl < D; dl++)
-    for (uint32_t P = 0; P < N; P++) {
-      uint64_t b = c.row[P] + c.so[(size_t)P * (D + 1) + dl], en = c.row[P] + c.so[(size_t)P * (D + 1) + dl + 1];
-      for (uint64_t k = b; k < en; k++) {
-        if (c.post[k] / locN != h) continue;
-        if (pre) pre[o] = P;
-        if (post) post[o] = c.post[k];
-        if (delay) delay[o] = (uint8_t)dl;
-        if (kind) kind[o] = c.sub[P];
-        if (weight) weight[o] = c.w[k];
-        if (tderiv) tderiv[o] = c.td.empty() ? 0.0f : c.td[k];
-        o++;
-      }
-    }
-  return 0;
+  const SynapseList out = {pre, post, delay, kind, weight, tderiv};
+  return rank_list(e, h, nullptr, &out);
 }
 
 extern "C" int dpsnn_enable_ltp_probe(dpsnn_engine *e) {
@@ -4417,7 +4608,7 @@ extern "C" int dpsnn_ltp_probe(dpsnn_engine *e, uint32_t h, uint32_t *t_ms, int1
   if (!e->d.probe_w) return dpsnn_fail(DPSNN_E_PARAM, "the LTP probe is not enabled");
   if (e->probe_t == UINT32_MAX) return dpsnn_fail(DPSNN_E_PARAM, "no plasticity update has run yet");
   HostCsr c;
-  int rc = fetch_csr(e, c, false);   // synchronises: the probe and the weights are final
+  int rc = fetch_csr(e, c);   // synchronises: the probe and the weights are final
   if (rc) return rc;
   std::vector<int16_t> pw(e->S);
   std::vector<float> pt(e->S), pm(e->S);
@@ -4451,7 +4642,7 @@ extern "C" int dpsnn_enable_stdp_events(dpsnn_engine *e) {
   if (e->t_host) return dpsnn_fail(DPSNN_E_PARAM, "the STDP event log is enabled before the first step");
   cudaSetDevice(e->device);
   HostCsr c;
-  int rc = fetch_csr(e, c, false);
+  int rc = fetch_csr(e, c);
   if (rc) return rc;
   e->h_row = std::move(c.row);
   e->h_so = std::move(c.so);
