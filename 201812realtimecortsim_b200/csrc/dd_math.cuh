@@ -186,12 +186,6 @@ DD_HD double log_cr(double x) {
 // floats are keys[bucket[b] .. bucket[b+1]).
 #define LOGF_FIX_BASE (0x30000000u >> 12)
 #define LOGF_FIX_NBUCKET ((0x3F800000u >> 12) - LOGF_FIX_BASE + 2)
-typedef struct {
-  const uint32_t *keys;
-  const float *vals;
-  const uint32_t *bucket;
-  uint32_t n;
-} logf_fixup_t;
 
 // Correctly rounded float log, from a double log with at most one ulp of
 // error when the rounding is unambiguous, else from log_cr.

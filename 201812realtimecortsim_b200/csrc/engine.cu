@@ -1307,8 +1307,8 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
 //   mappers     (warps 0-7) decide up to 128 neurons, 16 each: a mapper walks
 //               its 16 neurons from each of 32 candidate starts around the
 //               predicted one, a candidate per lane (bath_map).  The chain is
-//               then eight lookups (bath_compose, warp 0): each segment's
-//               end for its actual start.  A start outside a segment's window
+//               then eight lookups (bath_compose, by every mapper for
+//               itself): each segment's end for its actual start.  A start outside a segment's window
 //               ends the round there;
 //   preparers   (8, 13) read the next neurons, turn each one's budget (t+1 -
 //               nextBath)/invNuExt into integer bounds, and queue those with
@@ -1333,11 +1333,12 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
 // about 3000 cycles beside its steps, and at more neurons per segment the last
 // windows miss too often.  Measured per step (one B200), against the form
 // before, in which ten warps built tables of 64 candidate starts for every
-// neuron and every draw of both parities was converted: 62 us from 173 for one
-// rank of 1600 neurons, 99 from 300 for 11 ranks of 2743, 194 from 679 for 192
-// ranks of 3750, 16 from 67 for one of 100.  One warp deciding neuron by
-// neuron (a shared read, a vote and a count each) took 85 cycles per neuron
-// alone and 215 beside the other warps; this takes about 75.
+// neuron and every draw of both parities was converted: 53 us from 173 for one
+// rank of 1600 neurons, 87 from 300 for 11 ranks of 2743, 207 from 679 for 192
+// ranks of 3750 beside the update (44 of the 148 SMs hold two ranks), 16 from
+// 67 for one of 100.  One warp deciding neuron by neuron (a shared read, a vote
+// and a count each) took 85 cycles per neuron alone and 215 beside the other
+// warps; this takes about 60.
 #define BATH_THREADS 512       // 16 warps: roles above
 #define BATH_SEG 16            // neurons per mapper
 #define BATH_SEGS 8            // mappers
@@ -1943,9 +1944,8 @@ __device__ static inline void lifca_coeff(const Par &p, double deltaT, double &d
   poly = 1 - rc + rc * rc / 2;
 }
 
-// The calcium decay over the refractory period: once per spike, so out of
-// line (inlined, its double-double arithmetic takes the registers of the
-// neuron kernels).
+// The calcium decay over the refractory period: once per spike.  Out of line
+// it is no faster.
 __device__ __forceinline__ static double exp_cr_call(double x) { return exp_cr(x); }
 
 // LIFCADynamic with the coefficients of this event computed ahead; the branch
@@ -2661,7 +2661,7 @@ __global__ void __launch_bounds__(HEAVY_THREADS) huge_kernel(Dev d) {
 // Here a step is three kernels (and the bath): deliver_small_kernel with the
 // compaction, neuron_small_kernel with the warp path's sorts and runs, and
 // tail_small_kernel, each brought up while the one before it ends.  Measured
-// per step: 19 us from 45 for 100 neurons, 23 from 54 for 1155 in 5 ranks, 67
+// per step: 19 us from 45 for 100 neurons, 23 from 54 for 1155 in 5 ranks, 60
 // from 113 for 16 000 busy ones (8 events per neuron); what is left is the
 // update's chain of events, and the bath where a rank is long.
 
