@@ -1758,7 +1758,9 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           x_mx = d.max_ext[i0 + i + 64];
           x_sub = d.sub[i0 + i + 64];
         }
-        const bool act = i < locN && inv > 0 && nb < T1;
+        // a bath of rate zero (invNuExt infinite) asks for an event and has no slot for one
+        const bool due = i < locN && inv > 0 && nb < T1, act = due && mx > 0;
+        if (due && !act) atomicOr(d.flags, F_BATH_DRAWS);
         const uint32_t bal = __ballot_sync(0xffffffffu, act);
         uint32_t lo = 0, hi1 = 0;
         if (act) bath_bounds(T1, nb, inv, lo, hi1);

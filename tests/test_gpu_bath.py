@@ -36,3 +36,19 @@ def test_next_bath_and_raster_match_oracle(n_exc, n_inh, ranks, rate):
     for k in st:
         np.testing.assert_array_equal(st[k], so[k], err_msg=k)
     eng.close()
+
+
+# a rate of zero makes the interval infinite and the cap 0: the reference's loop
+# still makes one event, which has no slot; refused, as a cap that is exceeded is
+def test_rate_of_zero_is_refused():
+    cfg = nc.cortical_grid(1, 1, n_exc_a=20, n_exc_b=20, n_inh=10, p1=0.2, mu=0.6, total_ms=10, seed=5)
+    cfg.subpops[2].NuExt = 0.0
+    eng = E.Engine(cfg)
+    inv, cap = eng.bath_params()
+    assert np.isinf(inv[40:]).all() and not cap[40:].any() and cap[:40].all()
+    eng.step(2)
+    with pytest.raises(E.EngineError, match="bath"):
+        eng.sync()
+    with pytest.raises(E.EngineError, match="bath"):
+        eng.spikes(1)
+    eng.close()
