@@ -3520,7 +3520,10 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     n.light_max = lm ? (uint32_t)atoi(lm) : LOCAL_EVENTS;
     if (n.light_max < 1 || n.light_max > LOCAL_EVENTS) n.light_max = LOCAL_EVENTS;
   }
-  if (n.ev_cap > 4096) n.ev_cap = 4096;
+  // at least what the thread-per-neuron path reads of a bucket, and even: the
+  // sorted streams of two doubles per event start at a multiple of 16 bytes
+  n.ev_cap = std::min(4096u, std::max<uint32_t>(LOCAL_EVENTS, n.ev_cap));
+  n.ev_cap += n.ev_cap & 1;
   if (!(o && o->events_per_neuron)) {   // default: at most 16 GiB of event slots
     while (n.ev_cap > 64 && 8ull * n.ev_cap * n.N > (16ull << 30)) n.ev_cap >>= 1;
   }

@@ -93,7 +93,8 @@ typedef struct {
 typedef struct {
   uint32_t events_per_neuron;     /* per-target event slots per step (default
                                      1024, halved while they would exceed
-                                     16 GiB; at most 4096) */
+                                     16 GiB; at most 4096, at least 16,
+                                     and even: others are rounded) */
   uint32_t overflow_events;       /* events beyond that, per step (default 1<<22) */
   int device;                     /* CUDA device ordinal (default current) */
 } dpsnn_options;

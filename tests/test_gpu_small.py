@@ -64,3 +64,26 @@ def test_forms_match_oracle(cfx, cfy, ranks):
     for k in st:
         np.testing.assert_array_equal(st[k], so[k], err_msg=k)
     eng.close()
+
+
+# requests below the smallest bucket (16) and odd ones are rounded; the burst in
+# the small form, and the other form at its smallest network
+@pytest.mark.parametrize("cap, slots", [(1, 16), (7, 16), (65, 66)])
+@pytest.mark.parametrize("form", ["small", "large"])
+def test_rounded_buckets_match_oracle(form, cap, slots):
+    small = form == "small"
+    cfg = CASES["burst"][0]() if small else grid(32, 17, 32, 8, mu=0.8, g_c=0.5)
+    eng, even = E.Engine(cfg, events_per_neuron=cap), E.Engine(cfg, events_per_neuron=slots)
+    assert eng.device_bytes == even.device_bytes
+    even.close()
+    orc = O.OracleNet(cfg, 1)
+    for t in range(40 if small else 30):
+        eng.step(1)
+        ids, te = eng.spikes(t)
+        oi, ot = orc.step()
+        np.testing.assert_array_equal(ids, oi)
+        np.testing.assert_array_equal(te, ot)
+    st, so = eng.state(), orc.state()
+    for k in st:
+        np.testing.assert_array_equal(st[k], so[k], err_msg=k)
+    eng.close()
