@@ -1336,7 +1336,10 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
 // neuron and every draw of both parities was converted: 53 us from 173 for one
 // rank of 1600 neurons, 87 from 300 for 11 ranks of 2743, 207 from 679 for 192
 // ranks of 3750 beside the update (44 of the 148 SMs hold two ranks), 16 from
-// 67 for one of 100.  One warp deciding neuron by neuron (a shared read, a vote
+// 67 for one of 100.  At lower rates a step of 1600 neurons takes 24, 31, 31, 31
+// and 32 us for 0.01, 0.06, 0.25, 0.5 and 0.7 events per neuron and ms; with the
+// caps below 16 that go with them left to the walk it took 29, 45, 126, 217 and
+// 275.  One warp deciding neuron by neuron (a shared read, a vote
 // and a count each) took 85 cycles per neuron alone and 215 beside the other
 // warps; this takes about 60.
 #define BATH_THREADS 512       // 16 warps: roles above
@@ -1385,7 +1388,7 @@ struct BathSmem {
   float lap[BATH_PAIRS];
   uint8_t idx[BATH_PAIRS];
   double a_nb[BATH_ACT], a_inv[BATH_ACT];   // queued neuron a at a % BATH_ACT
-  uint4 a_b[BATH_ACT + BATH_SEG];   // bounds lo and hi - lo, the latter for the mappers, cap; mirrored at the end
+  uint4 a_b[BATH_ACT + BATH_SEG];   // bounds lo and hi - lo, cap; mirrored at the end
   uint32_t a_id[BATH_ACT];          // neuron of the rank, its sub-population in the top bits
   uint32_t a_t[BATH_ACT];           // expected q advance of the queued neurons before a (2^-20 units)
   uint2 pack[BATH_SEGS][BATH_NC];   // a segment's counts less one, a nibble per neuron, by candidate
@@ -1525,9 +1528,10 @@ __device__ __forceinline__ uint32_t bath_count(const BathSmem &s, const uint4 &k
   const uint32_t e = x + (y1 >> 31) + (y2 >> 31) + (y3 >> 31) + (y4 >> 31), c = e - p;
   // the first sum not below lo, less lo: the negative ones are large unsigned
   const uint32_t over = min(min(y1, y2), min(y3, y4));
-  // undecided, in bad's top bit: the sum lies between lo and hi, or none of
-  // the sixteen reaches lo (k.z: hi - lo, or 2^31 where the cap is below 16)
-  bad |= over - k.z;
+  // undecided, in bad's top bit: the sum lies between lo and hi, none of the
+  // sixteen reaches lo (over is then a negative number), or the count is past
+  // the neuron's cap (k.z)
+  bad |= (over - k.y) | ~(c - k.z);
   qm = T + over;
   p = e + 1;
   return c;
@@ -1613,7 +1617,7 @@ __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const Bath
     slow = 1u << stop_g;
     const uint32_t n_end = min(n_done + BATH_SEG, left), lim = cur.conv_end;
     while (n_done < n_end && !rebase) {
-      const uint32_t a = (cur.a + n_done) & A, mx = s.a_b[a].w, lo = s.a_b[a].x;
+      const uint32_t a = (cur.a + n_done) & A, mx = s.a_b[a].z, lo = s.a_b[a].x;
       if (m + max(33u, mx + 1) > lim) break;   // its pairs are not converted yet
       uint32_t c = 0;
       const uint32_t F = s.q[(m + 1 + lane) & M] - s.q[m & M];
@@ -1779,7 +1783,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           const uint32_t k = (e + pw * n0 + __popc(bal & ((1u << lane) - 1))) & A;
           s.a_nb[k] = nb;
           s.a_inv[k] = inv;
-          const uint4 ab = make_uint4(lo, hi1 - lo, mx < 16 ? 0x80000000u : hi1 - lo, mx);
+          const uint4 ab = make_uint4(lo, hi1 - lo, mx, 0u);
           s.a_b[k] = ab;
           if (k < BATH_SEG) s.a_b[k + BATH_ACT] = ab;
           s.a_id[k] = i | (sub << 25);

@@ -38,6 +38,31 @@ def test_next_bath_and_raster_match_oracle(n_exc, n_inh, ranks, rate):
     eng.close()
 
 
+# caps below the sixteen events a mapper counts (rates below 0.75) are decided by
+# the mappers too: fewer events take no longer, where a walk neuron by neuron took
+# five times as long
+def test_low_rates_cost_no_more():
+    def bath_seconds(rate):
+        cfg = nc.cortical_grid(1, 1, n_exc_a=640, n_exc_b=640, n_inh=320, p1=0.01, p_intra=0.02, mu=0.001,
+                               nu_ext_hz=rate, total_ms=1000, seed=7)
+        eng = E.Engine(cfg)
+        eng.step(50)
+        eng.sync()
+        eng.set_timing(True)
+        best = np.inf
+        for _ in range(5):
+            before = eng.kernel_times()[0][2]
+            eng.step(50)
+            eng.sync()
+            best = min(best, eng.kernel_times()[0][2] - before)
+        eng.close()
+        return best
+
+    at_3 = bath_seconds(3.0)
+    for rate in (0.06, 0.25, 0.7):
+        assert bath_seconds(rate) < 1.3 * at_3
+
+
 # a rate of zero makes the interval infinite and the cap 0: the reference's loop
 # still makes one event, which has no slot; refused, as a cap that is exceeded is
 def test_rate_of_zero_is_refused():
