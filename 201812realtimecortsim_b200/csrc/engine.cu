@@ -3750,8 +3750,11 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   // a block per 32 neurons: in a burst, or under a fast bath, tens of a small
   // network's neurons have more than 256 events in a step.  With one per 256,
   // 80 steps of 32 networks of 1250 to 20 000 neurons took 258 ms against 146
-  // around their onset, and 65 against 45 later.
-  e->grid_tail = std::min<uint32_t>((uint32_t)sms, (N + 31) / 32);
+  // around their onset, and 65 against 45 later.  Smaller buckets than the
+  // default's send neurons of fewer events there, and each searches the overflow
+  // list: a block per SM (the burst of 1250 neurons with 64 and 512 slots: 1.38
+  // and 0.39 ms per step, 4.5 and 1.09 with a block per 32 neurons).
+  e->grid_tail = n.ev_cap < DEFAULT_EVENT_CAP ? (uint32_t)sms : std::min<uint32_t>((uint32_t)sms, (N + 31) / 32);
   e->grid_huge = (uint32_t)sms;
   free_temps(e);   // after their last use on this stream
   CK(cudaStreamSynchronize(e->stream));

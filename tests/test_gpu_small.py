@@ -3,6 +3,8 @@ sorts, tail) where its branches change, against the CPU restatement: light,
 sorted, block-sorted and overflowing neurons (the bucket size moves the lines
 between them), networks whose size is no multiple of a warp, with and without
 plasticity, and the sizes on either side of the form's limits."""
+import time
+
 import numpy as np
 import pytest
 
@@ -87,3 +89,23 @@ def test_rounded_buckets_match_oracle(form, cap, slots):
     for k in st:
         np.testing.assert_array_equal(st[k], so[k], err_msg=k)
     eng.close()
+
+
+# small buckets send most of a burst's neurons to the blocks' sort (with an
+# overflow list to search): 5 times the default's time, 17 when it had a block
+# per 32 neurons there too
+def test_small_buckets_in_a_burst():
+    def seconds(cap):
+        best = np.inf
+        for _ in range(3):
+            eng = E.Engine(CASES["burst"][0](), events_per_neuron=cap)
+            eng.step(1)
+            eng.sync()
+            t = time.perf_counter()
+            eng.step(39)
+            eng.sync()
+            best = min(best, time.perf_counter() - t)
+            eng.close()
+        return best
+
+    assert seconds(64) < 11 * seconds(0)
