@@ -3747,14 +3747,20 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
   e->sms = sms;
   default_grids(e, 0, 0, 0);
-  // a block per 32 neurons: in a burst, or under a fast bath, tens of a small
-  // network's neurons have more than 256 events in a step.  With one per 256,
-  // 80 steps of 32 networks of 1250 to 20 000 neurons took 258 ms against 146
-  // around their onset, and 65 against 45 later.  Smaller buckets than the
-  // default's send neurons of fewer events there, and each searches the overflow
-  // list: a block per SM (the burst of 1250 neurons with 64 and 512 slots: 1.38
-  // and 0.39 ms per step, 4.5 and 1.09 with a block per 32 neurons).
-  e->grid_tail = n.ev_cap < DEFAULT_EVENT_CAP ? (uint32_t)sms : std::min<uint32_t>((uint32_t)sms, (N + 31) / 32);
+  // The tail's blocks.  A block per 32 neurons where few neurons can have more
+  // than 256 events in a step (one per incoming synapse at most): with one per
+  // 256, 80 steps of 32 networks of 1250 to 20 000 neurons took 258 ms against
+  // 146 around their onset, and 65 against 45 later; a graph of 16 networks of
+  // 120 to 1920 neurons with 150 synapses each takes 3.6 ms, 3.9 with one per 8.
+  // One per 8 where a burst brings most neurons more: a step of 2000 neurons with
+  // 1900 synapses each in their burst 1.84 ms from 3.92, of 1250 with 1125 0.27
+  // from 0.44.  Smaller buckets than the default's send neurons of fewer events
+  // there, and each searches the overflow list: a block per SM (the burst of 1250
+  // neurons with 64 and 512 slots: 1.38 and 0.39 ms per step, 4.5 and 1.09 with a
+  // block per 32 neurons).
+  const uint32_t per_block = e->S > 2ull * HEAVY_WARP_MAX * N ? 8 : 32;
+  e->grid_tail = n.ev_cap < DEFAULT_EVENT_CAP ? (uint32_t)sms
+                                              : std::min<uint32_t>((uint32_t)sms, (N + per_block - 1) / per_block);
   e->grid_huge = (uint32_t)sms;
   free_temps(e);   // after their last use on this stream
   CK(cudaStreamSynchronize(e->stream));

@@ -91,21 +91,30 @@ def test_rounded_buckets_match_oracle(form, cap, slots):
     eng.close()
 
 
+def burst_seconds(cfg, steps, cap):
+    best = np.inf
+    for _ in range(3):
+        eng = E.Engine(cfg, events_per_neuron=cap)
+        eng.step(1)
+        eng.sync()
+        t = time.perf_counter()
+        eng.step(steps)
+        eng.sync()
+        best = min(best, time.perf_counter() - t)
+        eng.close()
+    return best
+
+
 # small buckets send most of a burst's neurons to the blocks' sort (with an
 # overflow list to search): 5 times the default's time, 17 when it had a block
 # per 32 neurons there too
 def test_small_buckets_in_a_burst():
-    def seconds(cap):
-        best = np.inf
-        for _ in range(3):
-            eng = E.Engine(CASES["burst"][0](), events_per_neuron=cap)
-            eng.step(1)
-            eng.sync()
-            t = time.perf_counter()
-            eng.step(39)
-            eng.sync()
-            best = min(best, time.perf_counter() - t)
-            eng.close()
-        return best
+    cfg = CASES["burst"][0]()
+    assert burst_seconds(cfg, 39, 64) < 11 * burst_seconds(cfg, 39, 0)
 
-    assert seconds(64) < 11 * seconds(0)
+
+# so does a large in-degree with the default's buckets: as many blocks as buckets
+# of nearly that size have, where a block per 32 neurons took twice the time
+def test_large_in_degree_in_a_burst():
+    cfg = grid(1, 1, 2000, 1, mu=0.3, g_c=0.2, p_intra=0.95)
+    assert burst_seconds(cfg, 49, 0) < 1.5 * burst_seconds(cfg, 49, 1022)
