@@ -2997,6 +2997,7 @@ struct dpsnn_engine {
   uint32_t *h_pin = nullptr;          // pinned {flags, spike count} of dpsnn_rank_spikes_noalloc
   SpikeRead *h_read = nullptr;        // pinned, mapped: what read_pack_kernel writes, h_read_cap spikes
   uint32_t h_read_cap = 0;
+  std::mutex read_mu;                 // held from that kernel's launch until its lists are copied out
   // spike lists are read on their own stream as soon as the compaction of
   // their step is done, while the rest of that step (and later ones) run
   cudaStream_t read_stream = nullptr;
@@ -4285,14 +4286,14 @@ extern "C" uint64_t dpsnn_events_delivered(const dpsnn_engine *e) {
 // The lists of steps t0 .. t0+n-1 (1 <= n <= RING_SLOTS) after the compaction
 // of the last of them (steps complete in order on the engine stream; the rest
 // of that step and later ones may still run): the error flags, the counts, and
-// whether the lists fitted the read buffer.
+// whether the lists fitted, in the read buffer, which the caller holds (read_mu).
 static int read_lists(dpsnn_engine *e, uint32_t t0, uint32_t n, bool &packed) {
   CK(cudaStreamWaitEvent(e->read_stream, e->ev_slot[(t0 + n - 1) % RING_SLOTS], 0));
   read_pack_kernel<<<n == 1 ? 2 : 16, READ_PACK_THREADS, 0, e->read_stream>>>(e->d, t0, n, e->h_read_cap, e->h_read);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(e->read_stream));
   packed = e->h_read->total <= e->h_read_cap;
-  return flags_error(e->h_read->flags);
+  return 0;
 }
 static const uint32_t *read_ids(const dpsnn_engine *e) {
   return reinterpret_cast<const uint32_t *>(spike_read_te(e->h_read) + e->h_read_cap);
@@ -4304,8 +4305,10 @@ extern "C" int dpsnn_spikes(dpsnn_engine *e, uint32_t t_ms, uint32_t *ids, doubl
   if (t_ms >= e->t_host || t_ms + RING_SLOTS < e->t_host)
     return dpsnn_fail(DPSNN_E_STATE, "step %u is not among the last %d completed steps", t_ms, RING_SLOTS);
   cudaSetDevice(e->device);
+  std::lock_guard<std::mutex> lock(e->read_mu);
   bool packed;
   int rc = read_lists(e, t_ms, 1, packed);
+  if (!rc) rc = flags_error(e->h_read->flags);
   if (rc) return rc;
   const uint32_t cnt = e->h_read->total, k = std::min(cnt, cap);
   *count = cnt;
@@ -4329,9 +4332,12 @@ extern "C" int dpsnn_spikes_range(dpsnn_engine *e, uint32_t t0, uint32_t n, uint
     return dpsnn_fail(DPSNN_E_STATE, "steps %u..%u are not among the last %d completed steps", t0, t0 + n - 1,
                       RING_SLOTS);
   cudaSetDevice(e->device);
+  std::lock_guard<std::mutex> lock(e->read_mu);
   bool packed;
   int rc = read_lists(e, t0, n, packed);
+  if (rc) return rc;
   memcpy(counts, e->h_read->counts, 4ull * n);
+  rc = flags_error(e->h_read->flags);
   if (rc) return rc;
   uint64_t off = e->h_read->total;
   if (off > cap) return dpsnn_fail(DPSNN_E_CAPACITY, "%llu spikes in steps %u..%u exceed the buffers (%llu)",
