@@ -1401,6 +1401,7 @@ struct BathSmem {
   double near[256];                 // Dev::fix_near
   double2 log_tab[LOG_TAB_N];       // Dev::log_tab
   uint32_t conv_tot[3];             // converters: lapse sums of the warps' pairs
+  uint32_t slots;                   // the rank's event slots (bath_slots)
   BathCtl ctl[2];
 };
 
@@ -1687,6 +1688,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
   if (tid == 0) {
     s.q[0] = s.q[BATH_PAIRS] = 0;
     s.a_t[0] = 0;
+    s.slots = (uint32_t)(d.bath_rank_base[h + 1] - d.bath_rank_base[h]);
     BathCtl c = {};
     c.base = BATH_HIST;
     c.raw_end = kept;
@@ -1854,6 +1856,10 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           const uint32_t word = jj < 8 ? pk.x : pk.y, sh = 4 * (jj & 7);
           m0 = s.e_start[par][g] + jj + nibble_sum(word & ((1u << sh) - 1)) + (jj < 8 ? 0u : nibble_sum(pk.x));
           cnt = ((word >> sh) & 15u) + 1;
+        }
+        if (cur.out + m0 + cnt > s.slots) {
+          atomicOr(d.flags, F_BATH_DRAWS);
+          continue;
         }
         const uint32_t id = s.a_id[a], i = i0 + (id & ((1u << 25) - 1)), at = ev_base + cur.out + m0;
         const double *lut = d.lut + 256 * (id >> 25);
@@ -2983,6 +2989,7 @@ struct dpsnn_engine {
   std::vector<uint16_t> h_so;      // (for the STDP event log's order)
   std::vector<void *> allocs;
   std::vector<void *> temps;       // build scratch, released when the build ends
+  std::vector<void *> spare;       // scratch that the build is done with, released then too, or when memory runs out
   uint64_t bytes = 0;              // device memory held (allocs)
   uint32_t grid_neuron = 0, grid_deliver = 0, grid_heavy = 0, grid_heavy_run = 0, grid_huge = 0, grid_tail = 0;
   int sms = 148;                   // the device's SMs (default grids)
@@ -3030,12 +3037,29 @@ static void default_grids(dpsnn_engine *e, uint32_t deliver, uint32_t heavy_sort
 // device's memory pool): unlike cudaMalloc/cudaFree they do not synchronise
 // the device, so engines built from several host threads, or while other
 // engines step, do not wait for each other.  `temp` allocations (the
-// connectome build's scratch) are released at the end of the build.
+// connectome build's scratch) are released at the end of the build: earlier,
+// the pool would unmap and map the same memory again (24x24: 30 of 200 ms).
+// Where memory runs out before, the finished generation's, hundreds of bytes
+// per neuron, goes first.
+static void free_list(dpsnn_engine *e, std::vector<void *> &v) {
+  for (void *q : v) cudaFreeAsync(q, e->stream);
+  v.clear();
+}
+static void free_temps(dpsnn_engine *e) {
+  free_list(e, e->spare);
+  free_list(e, e->temps);
+}
 template <typename T>
 static int dalloc(dpsnn_engine *e, T **p, size_t n, bool temp = false) {
   void *q = nullptr;
   size_t bytes = std::max<size_t>(n * sizeof(T), 16);
   cudaError_t err = cudaMallocAsync(&q, bytes, e->stream);
+  if (err == cudaErrorMemoryAllocation && !e->spare.empty()) {
+    cudaGetLastError();
+    free_list(e, e->spare);
+    CK(cudaStreamSynchronize(e->stream));
+    err = cudaMallocAsync(&q, bytes, e->stream);
+  }
   if (err != cudaSuccess)
     return dpsnn_fail(DPSNN_E_NOMEM, "cudaMallocAsync(%zu bytes): %s", bytes, cudaGetErrorString(err));
   (temp ? e->temps : e->allocs).push_back(q);
@@ -3055,11 +3079,6 @@ static int dalloc(dpsnn_engine *e, T **p, size_t n, bool temp = false) {
     int rc_ = dalloc(e, &(ptr), (size_t)(n), true);   \
     if (rc_) return rc_;                              \
   } while (0)
-
-static void free_temps(dpsnn_engine *e) {
-  for (void *q : e->temps) cudaFreeAsync(q, e->stream);
-  e->temps.clear();
-}
 
 // The fix-up table on the device: a bit per float that has one, and per result
 // binade the fix-up inputs' least distance from the float their logarithm
@@ -3438,6 +3457,23 @@ static int generate_by_threads(dpsnn_engine *e, const std::vector<float> &prob, 
   return 0;
 }
 
+// A rank's bath event slots.  A neuron has 1/invNuExt events per step on
+// average, Poisson distributed, one more at step 0 (nextBath = 0), and at most
+// its cap, 20 times the mean.  The rank's mean and 32 deviations (passed with a
+// probability below 1e-100; the emitters check), and no more than its caps: an
+// event takes 16 bytes, in two buffers, and all the caps of the 24x24 network
+// 1.1 GB.
+static uint64_t bath_slots(const uint32_t *max_ext, const double *inv_nu, uint32_t neurons) {
+  uint64_t caps = 0;
+  double mean = 0;
+  for (uint32_t i = 0; i < neurons; i++) {
+    if (!(inv_nu[i] > 0)) continue;
+    caps += max_ext[i];
+    mean += std::min((double)max_ext[i], 1.0 + 1.0 / inv_nu[i]);
+  }
+  return std::min(caps, (uint64_t)(mean + 32.0 * sqrt(mean)) + 64);
+}
+
 static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_options *o) {
   NetConst &n = e->hnet;
   memset(&n, 0, sizeof n);
@@ -3596,6 +3632,7 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     const bool warp_form = gen_plan(n, prob, plan);
     int rc = warp_form ? generate_by_warps(e, plan, bath_tmpl, hist0) : generate_by_threads(e, prob, bath_tmpl, hist0);
     if (rc) return rc;
+    e->spare.swap(e->temps);
   }
   // ---- run-over-group-end check (see DPSNN_synapse.c:211-265): the reference's
   // search continues past a (delay, source rank) group while the next entry has
@@ -3674,16 +3711,14 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
   init_neurons_kernel<<<(N + 255) / 256, 256, 0, e->stream>>>(d);
   CK(cudaGetLastError());
   {
-    // per-rank bath event capacity = sum of maxExternCurrentCount
     std::vector<uint32_t> mx(N);
+    std::vector<double> inv(N);
     CK(cudaMemcpyAsync(mx.data(), d.max_ext, 4ull * N, cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaMemcpyAsync(inv.data(), d.inv_nu, 8ull * N, cudaMemcpyDeviceToHost, e->stream));
     CK(cudaStreamSynchronize(e->stream));
     std::vector<uint64_t> base(P + 1, 0);
-    for (uint32_t h = 0; h < P; h++) {
-      uint64_t s = 0;
-      for (uint32_t i = h * n.locN; i < (h + 1) * n.locN; i++) s += mx[i];
-      base[h + 1] = base[h] + s;
-    }
+    for (uint32_t h = 0; h < P; h++)
+      base[h + 1] = base[h] + bath_slots(&mx[(size_t)h * n.locN], &inv[(size_t)h * n.locN], n.locN);
     uint32_t mx_max = 0;
     for (uint32_t i = 0; i < N; i++) mx_max = std::max(mx_max, mx[i]);
     if (mx_max > BATH_MAX_EXT)

@@ -77,3 +77,17 @@ def test_rate_of_zero_is_refused():
     with pytest.raises(E.EngineError, match="bath"):
         eng.spikes(1)
     eng.close()
+
+
+# a network's bath events hold no more memory than 9 bytes per event slot in two
+# buffers did, a slot for every event that the neurons' caps allow
+def test_events_hold_what_a_step_needs():
+    def held(rate):
+        cfg = nc.cortical_grid(4, 4, total_ms=10, seed=5, glob_h=16, p1=0.01, p_intra=0.02, nu_ext_hz=rate)
+        eng = E.Engine(cfg)
+        b, caps = eng.device_bytes, int(eng.bath_params()[1].astype(np.int64).sum())
+        eng.close()
+        return b, caps
+
+    (low, low_caps), (high, high_caps) = held(0.5), held(5.0)
+    assert high - low < 2 * 9 * (high_caps - low_caps)
