@@ -68,8 +68,43 @@ def expected_synapses(cfg: nc.NetConfig) -> float:
     return tot
 
 
+def _longest_row(cfg: nc.NetConfig) -> float:
+    """Most synapses to expect of one neuron: its expected number, in the
+    module that has the most, and six deviations."""
+    S, longest = cfg.stencil_dim, 0.0
+    near = lambda c, size: [d for d in range(-(S - 1), S) if 0 <= c + d < size]
+    # a module S - 1 from the border sees as many as any further in
+    cells = {(tuple(near(cx, cfg.cfx)), tuple(near(cy, cfg.cfy)))
+             for cx in range(min(cfg.cfx, S)) for cy in range(min(cfg.cfy, S))}
+    for s, p in enumerate(cfg.subpops):
+        if p.count == 0:
+            continue
+        for xs, ys in cells:
+            row = sum(probs[abs(dy) * S + abs(dx)] * cfg.subpops[t].count
+                      for (u, t), (_, _, _, _, probs) in cfg.conn.items() if u == s for dx in xs for dy in ys)
+            longest = max(longest, row)
+    return longest + 6 * math.sqrt(longest)
+
+
+def _build_scratch(cfg: nc.NetConfig) -> int:
+    """Device memory that the connectome's generation needs beside what the
+    engine keeps."""
+    N = cfg.glob_n
+    # a weight may be drawn again, or a probability is refused: one thread per
+    # module (the engine's rule between the two forms)
+    by_threads = any(max(probs) > 0 and (8.97 * abs(np.float32(dj)) > 0.999 or
+                                         any(0 < np.float32(q) <= np.float32(1e-5) for q in probs))
+                     for _, dj, _, _, probs in cfg.conn.values())
+    if by_threads:   # each thread's target list, and a neuron's synapses per delay, under two hypotheses
+        return cfg.n_modules * 61_000 + N * (4 * cfg.D + 4)
+    # where each neuron's synapses start in its module's stream, under one or
+    # two hypotheses for NormDev's cache; lists longer than 1536 per warp
+    fill = 4 * min(-(-N // 4), 592) * 52_500 if _longest_row(cfg) > 1536 else 0
+    return cfg.n_modules * 600 + N * (1 if cfg.glob_h == cfg.n_modules else 2) * 236 + fill
+
+
 def estimate_device_bytes(cfg: nc.NetConfig, events_per_neuron: int = 1024) -> int:
-    """Device memory an engine of this network holds, from its size (the
+    """Device memory an engine of this network takes, from its size (the
     engine's layout: state, ring, event buckets, bath buffers, build scratch,
     6 B per synapse and 12 more with plasticity), with a 10 % margin on the
     synapse count."""
@@ -77,18 +112,20 @@ def estimate_device_bytes(cfg: nc.NetConfig, events_per_neuron: int = 1024) -> i
     cap = events_per_neuron
     while cap > 64 and 8 * cap * N > (16 << 30):
         cap //= 2
-    max_ext = 0
+    # bath events per step: a module's mean and caps, a rank's slots
+    mean = caps = 0.0
     for p in cfg.subpops:
         if p.count and p.NuExt > 0:
-            inv = 1000.0 / (p.NuExt * cfg.bath_cext)
-            max_ext = max(max_ext, math.ceil(20 / inv))
-    # the build's scratch: where each neuron's synapses start in its module's
-    # stream, under one or two hypotheses for NormDev's cache
-    starts = (1 if cfg.glob_h == cfg.n_modules else 2) * 236
-    per_neuron = 66 + 2 * (cfg.D + 1) + 8 + 80 * 12 + 8 * cap + 20 + 12 + 2 * (16 * max_ext + 8) + starts + 4
+            rate = p.NuExt * cfg.bath_cext / 1000.0
+            caps += p.count * math.ceil(20 * rate)
+            mean += p.count * min(math.ceil(20 * rate), 1 + rate)
+    per_rank = cfg.n_modules // cfg.glob_h
+    slots = min(per_rank * caps, per_rank * mean + 32 * math.sqrt(per_rank * mean) + 64)
+    per_neuron = 66 + 2 * (cfg.D + 1) + 8 + 80 * 12 + 8 * cap + 20 + 12 + 2 * 8 + 4
     per_syn = 6 + (12 if cfg.stdp is not None else 0)
-    fixed = (116 << 20) + cfg.glob_h * 1_100 + cfg.n_modules * 600
-    return int(N * per_neuron + 1.1 * expected_synapses(cfg) * per_syn + fixed)
+    fixed = (116 << 20) + cfg.glob_h * (1_100 + 8 * cfg.D)
+    return int(N * per_neuron + 1.1 * expected_synapses(cfg) * per_syn + cfg.glob_h * 32 * slots + fixed +
+               _build_scratch(cfg))
 
 
 @dataclasses.dataclass

@@ -38,3 +38,39 @@ def test_each_result_is_the_same_alone_and_in_the_mix():
     dones = sorted(j.t_done for j in served)
     assert starts[-1] >= dones[0]
     assert any(x.t_start < y.t_done and y.t_start < x.t_done for x in served for y in served if x is not y)
+
+
+def network(name):
+    if name == "by_warps":
+        return nc.cortical_grid(4, 4, glob_h=4, p1=0.01)
+    if name == "plastic":
+        return nc.cortical_grid(3, 3, glob_h=9, p1=0.02, stdp=True, start_plasticity_ms=0)
+    if name == "fast_bath":
+        return nc.cortical_grid(4, 4, n_exc_a=400, n_exc_b=400, n_inh=200, glob_h=1, p1=0.005, nu_ext_hz=6.0)
+    if name == "long_rows":
+        return nc.cortical_grid(1, 1, n_exc_a=700, n_exc_b=700, n_inh=500, p_intra=0.95)
+    cfg = nc.cortical_grid(16, 16, n_exc_a=10, n_exc_b=10, n_inh=5, glob_h=256, p1=0.1)   # by_threads
+    cfg.conn = {k: (J, 0.2, lo, hi, probs) for k, (J, _, lo, hi, probs) in cfg.conn.items()}
+    return cfg
+
+
+@pytest.mark.parametrize("name", ["by_warps", "by_threads", "plastic", "fast_bath", "long_rows"])
+def test_footprint_covers_the_build(name):
+    """What the device's pool held at its highest while the engine was built."""
+    from cuda.bindings import driver, runtime
+    E = importlib.import_module(package().__name__ + ".engine")
+    cfg = network(name)
+    E.Engine(nc.cortical_grid(1, 1, n_exc_a=10, n_exc_b=10, n_inh=5, p1=0.1), device=0).close()   # the device is set up
+    err, pool = runtime.cudaDeviceGetDefaultMemPool(0)
+    assert int(err) == 0
+    high = runtime.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    err, = runtime.cudaMemPoolSetAttribute(pool, high, driver.cuuint64_t(0))
+    assert int(err) == 0
+    eng = E.Engine(cfg, device=0)
+    err, used = runtime.cudaMemPoolGetAttribute(pool, high)
+    assert int(err) == 0
+    held = eng.device_bytes
+    eng.close()
+    estimate = S.estimate_device_bytes(cfg)
+    assert held <= int(used) <= estimate
+    assert estimate < 1.3 * int(used)

@@ -140,3 +140,20 @@ def test_footprint_estimate_grows_with_the_network():
     assert 0 < a < b < c
     # ~5.6 M synapses at 2x2 (mean in-degree ~1125)
     assert 5.0e6 < S.expected_synapses(nc.cortical_grid(2, 2)) < 6.2e6
+
+
+def with_spread(cfg, dj):
+    cfg.conn = {k: (J, dj, lo, hi, probs) for k, (J, _, lo, hi, probs) in cfg.conn.items()}
+    return cfg
+
+
+def test_footprint_estimate_holds_the_build_scratch():
+    small = dict(n_exc_a=10, n_exc_b=10, n_inh=5, p1=0.1, delay_range_subpop=True)
+    cfg = nc.cortical_grid(16, 16, **small)
+    by_warps, by_threads = (S.estimate_device_bytes(with_spread(cfg, dj)) for dj in (0.1, 0.2))
+    # a target list of 7500 per module and hypothesis, counts per delay for each neuron and hypothesis
+    assert by_threads - by_warps > 256 * (2 * 4 * 7500 - 600) + 6400 * (4 * cfg.D - 472)
+    # rows longer than the lists in shared memory: 52.5 KB for each of 4 warps in up to 592 blocks
+    short, long_rows = (S.estimate_device_bytes(nc.cortical_grid(1, 1, n_exc_a=n, n_exc_b=n, n_inh=n, p_intra=0.95))
+                        for n in (400, 600))
+    assert long_rows - short > 1800 // 4 * 4 * 52_500
