@@ -3247,8 +3247,9 @@ struct GenPlan {
 
 // The warp form's plan; false where the thread form has to do: a weight may
 // be rejected (NormDev's values are below sqrt(-2 ln 4e-18) = 8.96, so with
-// sigma under 1/8.97 of the mean none is), a probability that the reference
-// does not take, or more distinct probabilities than tables.
+// sigma under 1/8.97 of the mean none is; near the denormal floats their
+// rounding moves sigma and the weights too far), a probability that the
+// reference does not take, or more distinct probabilities than tables.
 static bool gen_plan(const NetConst &n, const std::vector<float> &prob, GenPlan &g) {
   const uint32_t st = n.stencil, M = n.max_mod;
   g.row_off.push_back(0);
@@ -3258,7 +3259,10 @@ static bool gen_plan(const NetConst &n, const std::vector<float> &prob, GenPlan 
         for (uint32_t y = 0; y < st; y++) {
           const float pf = prob[(((size_t)s * DPSNN_MAX_SUBPOP + t) * st + x) * st + y];
           if (!(pf > 0)) continue;
-          if (!(pf > 0.00001f) || !(8.97 * fabs(n.DJ[s * DPSNN_MAX_SUBPOP + t]) <= 0.999)) return false;
+          const double mean = n.J[s * DPSNN_MAX_SUBPOP + t];
+          if (!(pf > 0.00001f) || !(8.97 * fabs(n.DJ[s * DPSNN_MAX_SUBPOP + t]) <= 0.999) ||
+              (mean != 0 && !(fabs(mean) > 1e-30)))
+            return false;
           uint32_t k = 0;
           while (k < g.tabs.size() && g.tabs[k].pf != pf) k++;
           if (k == g.tabs.size()) {

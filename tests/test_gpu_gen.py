@@ -12,12 +12,14 @@ E = engine_module()
 nc = netconfig()
 
 
-def grid(cfx, cfy, a, b, i, ranks=1, dj=None, **kw):
+def grid(cfx, cfy, a, b, i, ranks=1, dj=None, mean=None, **kw):
     kw.setdefault("mu", 0.3)
     cfg = nc.cortical_grid(cfx, cfy, n_exc_a=a, n_exc_b=b, n_inh=i, glob_h=ranks, total_ms=10, seed=9,
                            delay_range_subpop=True, **kw)
     if dj is not None:
         cfg.conn = {k: (J, dj, d0, d1, p) for k, (J, _, d0, d1, p) in cfg.conn.items()}
+    if mean is not None:
+        cfg.conn = {k: (mean, d, d0, d1, p) for k, (_, d, d0, d1, p) in cfg.conn.items()}
     return cfg
 
 
@@ -33,6 +35,9 @@ CASES = {
     "long_rows": lambda: grid(1, 1, 700, 700, 500, p_intra=0.95),
     # weights far from their mean are drawn again: the thread form
     "rejected_weights": lambda: grid(2, 2, 40, 37, 20, ranks=2, p1=0.2, dj=0.6, mu=0.2),
+    # means of five denormal units: a spread of 0.111 rounds to one unit, 0.2 of
+    # the mean, and some weights are drawn again (all of them are stored as 0)
+    "denormal_mean": lambda: grid(1, 1, 500, 500, 250, p_intra=0.95, dj=0.111, mean=7e-45),
     # one value per weight
     "no_spread": lambda: grid(2, 1, 40, 37, 20, ranks=1, p1=0.2, dj=0.0),
 }
