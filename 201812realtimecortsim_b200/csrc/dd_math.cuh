@@ -1,5 +1,5 @@
 // dd_math.cuh -- correctly rounded exp/log in double-double arithmetic, and
-// a logf bit-identical to the host C library's.
+// the correctly rounded float log.
 //
 // The reference calls the C library's exp (LIFCA calcium decay,
 // DPSNN_neuron_sim.c:705), log (NormDev, randdev.c:599) and logf (bath
@@ -15,10 +15,9 @@
 //    The C library's exp/log differ from the correctly rounded value in about
 //    0.08% of arguments by one ulp; the raster is bit-identical to the
 //    reference until such a difference first changes a threshold decision.
-//  * logf_ref(x) equals the C library's logf for every float in (0,1]: the
-//    correctly rounded float logarithm, except at the inputs listed in a
-//    fix-up table built on the host from the C library itself
-//    (logf_fixup.c), where the C library's value is returned.
+//  * the C library's logf on (0,1] is the correctly rounded float logarithm
+//    (logf_cr_from), except at the inputs listed in a fix-up table built on the
+//    host from the C library itself (logf_fixup.c).
 #pragma once
 #include <stdint.h>
 #include <math.h>
@@ -179,13 +178,6 @@ DD_HD double log_cr(double x) {
   if (lo == hi) return lo;
   return log_cr_dd(x);
 }
-
-// Fix-up table of the C library's logf on (0,1]: sorted input bit patterns
-// keys[] with the library's results vals[]; bucket[b] is the first entry
-// whose key>>12 is >= b + LOGF_FIX_BASE, so the keys of one block of 4096
-// floats are keys[bucket[b] .. bucket[b+1]).
-#define LOGF_FIX_BASE (0x30000000u >> 12)
-#define LOGF_FIX_NBUCKET ((0x3F800000u >> 12) - LOGF_FIX_BASE + 2)
 
 // Correctly rounded float log, from a double log with at most one ulp of
 // error when the rounding is unambiguous, else from log_cr.

@@ -1406,8 +1406,8 @@ struct BathSmem {
 };
 
 // The correctly rounded float log in the rare case that the double one does
-// not decide it; out of line, since inlined it takes the registers of the
-// whole kernel.
+// not decide it.  Inlined: out of line the kernel spills more (68 bytes from
+// 52), and one rank of 1600 neurons takes 55.9 us per step against 53.1.
 __device__ __forceinline__ static float logf_cr_undecided(float x) { return (float)log_cr((double)x); }
 
 // The double of a normal float's bits (no conversion instruction: those have a
@@ -1429,7 +1429,8 @@ __device__ __forceinline__ double double_of_bits(uint32_t fb) {
 //    when the table is loaded; a search of the table here took up to eight
 //    dependent loads, in half of a warp's conversions).
 // Each step is done for all K draws before the next, so that their loads are
-// in flight together.
+// in flight together.  Run over all 10^9 draws, its lapses are the C library's,
+// bit for bit.
 template <int K>
 __device__ static inline void bath_lapse(const Dev &d, const BathSmem &s, const uint32_t (&mj)[K], float (&lap)[K]) {
   uint32_t fb[K], key[K], bw[K];
@@ -1937,7 +1938,9 @@ struct LifcaRegs {
 // r (a - b q) rounds to the quotient rounded to nearest; the first correction
 // brings q = a r within an ulp).  Five operations and no branch, where a
 // division's code has both; r = 0: b is out of the range in which nothing
-// overflows or underflows on the way, and is divided by.
+// overflows or underflows on the way, and is divided by.  The same bits as a / b
+// for 12 G pairs (a of 2^-60 to 2^30, b of 2^-40 to 2^40, an eighth of them with
+// a float's or an almost full mantissa).
 __device__ static inline double div_by(double a, double b, double r) {
   if (r == 0.0) return a / b;
   double q = a * r;
@@ -3013,11 +3016,16 @@ struct dpsnn_engine {
 
 static void collect_timings(dpsnn_engine *e);
 
-// The rule between a step's two forms.  The small one is faster at every size
-// its fired bits allow (per step, settled: 16 000 neurons in 64 ranks 34 us
-// against 53, 30 173 in 143 ranks 39 against 63, 100 in one 19 against 45),
-// except for a network that waits for long ranks' baths anyway and whose update
-// is large enough to slow them beside it (30 173 in 11 ranks: 102 against 97).
+// The rule between a step's two forms, in us per step at rest / busy (8 events
+// per neuron and ms), small form against large.  Up to 16 384 neurons the small
+// one is as fast or faster: 16 000 in 1 rank 426 / 432 against 430 / 433, in 8
+// ranks 67 / 74 against 68 / 97, in 64 ranks 32 / 61 against 47 / 104; 100 in one
+// 19 against 45.  Beyond, it is with short ranks (32 400 in 120: 37 / 101 against
+// 54 / 115, in 40: 46 / 102 against 50 / 122); with long ones both wait for the
+// baths, which the small one's update slows (in 4 ranks 229 / 239 against 227 /
+// 232, in 10 ranks 106 / 120 against 101 / 114).  Near the line one is ahead at
+// rest and the other busy (15 ranks of 2160: 80 / 98 against 73 / 110; 20 of 1620:
+// 66 / 101 against 59 / 111).
 static bool small_form(uint64_t neurons, uint64_t rank_neurons) {
   return neurons <= SMALL_N && (neurons <= SMALL_N / 2 || rank_neurons <= 2048);
 }
@@ -3114,10 +3122,9 @@ static int load_logf_fixup(dpsnn_engine *e) {
   if (!f) return dpsnn_fail(DPSNN_E_PARAM, "cannot open %s (built with the engine)", path.c_str());
   uint32_t n = 0;
   bool ok = fread(&n, 4, 1, f) == 1;
-  std::vector<uint32_t> keys(n), vals(n), bucket(LOGF_FIX_NBUCKET);
+  std::vector<uint32_t> keys(n), vals(n);
   ok = ok && fread(keys.data(), 4, n, f) == n;
   ok = ok && fread(vals.data(), 4, n, f) == n;
-  ok = ok && fread(bucket.data(), 4, LOGF_FIX_NBUCKET, f) == LOGF_FIX_NBUCKET;
   fclose(f);
   if (!ok) return dpsnn_fail(DPSNN_E_PARAM, "truncated %s", path.c_str());
   {
