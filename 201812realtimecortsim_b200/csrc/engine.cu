@@ -103,6 +103,8 @@ struct NetConst {
   uint32_t light_max;   // neurons with more synaptic events take the heavy path
   uint32_t delay_exp;  // getRandomDelay_EXP instead of _UNI
   float inv_log_tn;    // (float)(1.0 / log(0.05)), the EXP tail constant
+  const uint32_t *fix_keys, *fix_vals;   // the logf fix-up table, where bath_kernel<true> searches it
+  uint32_t fix_n;
 };
 
 // ------------------------------------------------------------------ ran3
@@ -1425,13 +1427,14 @@ __device__ __forceinline__ double double_of_bits(uint32_t fb) {
 //  - Inputs where the C library differs from the correctly rounded float all
 //    have a logarithm close to a rounding midpoint: nearer than the furthest
 //    of them in the result's binade (near) a bit per float says whether x is
-//    one.  Its value is then the float on the midpoint's other side (checked
-//    when the table is loaded; a search of the table here took up to eight
-//    dependent loads, in half of a warp's conversions).
+//    one.  Its value is then the float on the midpoint's other side, as that of
+//    any library with an error below one ulp is (a search of the table here took
+//    up to eight dependent loads, in half of a warp's conversions); where the
+//    table loaded has another value, SEARCH finds it.
 // Each step is done for all K draws before the next, so that their loads are
 // in flight together.  Run over all 10^9 draws, its lapses are the C library's,
 // bit for bit.
-template <int K>
+template <int K, bool SEARCH>
 __device__ static inline void bath_lapse(const Dev &d, const BathSmem &s, const uint32_t (&mj)[K], float (&lap)[K]) {
   uint32_t fb[K], key[K], bw[K];
   double r[K];
@@ -1475,8 +1478,19 @@ __device__ static inline void bath_lapse(const Dev &d, const BathSmem &s, const 
         fb[i] = __float_as_uint(f);
       }
     }
-    // f < 0: the next float below has the next bit pattern
-    if ((bw[i] >> ((key[i] - 0x30000000u) & 31)) & 1u) fb[i] += r[i] < 0 ? 1u : 0xFFFFFFFFu;
+    if ((bw[i] >> ((key[i] - 0x30000000u) & 31)) & 1u) {
+      if (SEARCH) {
+        const NetConst *net = d.net;
+        uint32_t lo = 0, hi = net->fix_n - 1;   // the key is listed
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (net->fix_keys[mid] < key[i]) lo = mid + 1; else hi = mid;
+        }
+        fb[i] = net->fix_vals[lo];
+      } else {
+        fb[i] += r[i] < 0 ? 1u : 0xFFFFFFFFu;   // f < 0: the next float below has the next bit pattern
+      }
+    }
     lap[i] = -__uint_as_float(fb[i]);
   }
 }
@@ -1505,13 +1519,14 @@ __device__ static inline void bath_bounds(double T1, double nb, double inv, uint
 // Draws past a neuron's cap, single ones (rare): from draw n on, until
 // nextBath reaches T1; returns the position after them, 0 when a draw that
 // is not generated yet is needed.
+template <bool SEARCH>
 __device__ static inline uint32_t bath_singles(const Dev &d, const BathSmem &s, uint32_t n, uint32_t raw_end,
                                                double inv, double T1, double &v) {
   do {
     if (n >= raw_end) return 0;
     const uint32_t mj[1] = {s.raw[n % BATH_RAW]};
     float lp[1];
-    bath_lapse<1>(d, s, mj, lp);
+    bath_lapse<1, SEARCH>(d, s, mj, lp);
     v += (double)lp[0] * inv;
     n++;
   } while (v < T1);
@@ -1585,6 +1600,7 @@ __device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t
 // round's start.  A segment with no decided entry at its start runs neuron
 // by neuron (warp 0) and ends the round: the sums of 1..32 lapses by lane and
 // a vote, or the reference's loop.
+template <bool SEARCH>
 __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const BathCtl &cur, BathCtl &nxt, uint32_t par,
                                            double T1, uint32_t w, uint32_t lane) {
   const uint32_t M = BATH_PAIRS - 1, A = BATH_ACT - 1;
@@ -1633,7 +1649,7 @@ __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const Bath
           c++;
         } while (v < T1 && c < mx);
         if (v < T1) {
-          rebase = bath_singles(d, s, cur.base + 2 * (m + c), cur.raw_end, inv, T1, v);
+          rebase = bath_singles<SEARCH>(d, s, cur.base + 2 * (m + c), cur.raw_end, inv, T1, v);
           if (!rebase) break;   // draws not generated yet
         }
       }
@@ -1671,6 +1687,7 @@ __device__ static inline uint32_t nibble_sum(uint32_t x) {
   return (((x & 0x0F0F0F0Fu) + ((x >> 4) & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
 }
 
+template <bool SEARCH>
 __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
   extern __shared__ __align__(16) unsigned char bath_smem_raw[];
   BathSmem &s = *reinterpret_cast<BathSmem *>(bath_smem_raw);
@@ -1719,7 +1736,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
     if (warp < BATH_SEGS) {
       bath_map(s, cur, warp, lane);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the mappers
-      bath_compose(d, s, cur, nxt, r & 1, T1, warp, lane);
+      bath_compose<SEARCH>(d, s, cur, nxt, r & 1, T1, warp, lane);
     } else if (warp == 15) {
       // x[n] = x[n-55] - x[n-24] mod 1e9, applied four times over: x[n] = x[n-96] - 4 x[n-127] + 6 x[n-158]
       // - 4 x[n-189] + x[n-220], so that 96 draws follow from the ones before them at once; keeping BATH_HIST
@@ -1819,7 +1836,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
         const uint32_t mi0 = s.raw[n % BATH_RAW], mi1 = s.raw[(n + 2) % BATH_RAW];
         const uint32_t mj[2] = {s.raw[(n + 1) % BATH_RAW], s.raw[(n + 3) % BATH_RAW]};
         float lp[2];
-        bath_lapse<2>(d, s, mj, lp);
+        bath_lapse<2, SEARCH>(d, s, mj, lp);
         const uint32_t f0 = lap_fixed(lp[0]), f1 = lap_fixed(lp[1]);
         uint32_t incl = f0 + f1;
         for (int o = 1; o < 32; o <<= 1) {
@@ -1871,7 +1888,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           ev[c] = make_double2(v, __ldg(&lut[s.idx[(m0 + c) & M]]));
           v += (double)s.lap[(m0 + c) & M] * inv;
         }
-        if (v < T1) bath_singles(d, s, cur.base + 2 * (m0 + cnt), cur.raw_end, inv, T1, v);
+        if (v < T1) bath_singles<SEARCH>(d, s, cur.base + 2 * (m0 + cnt), cur.raw_end, inv, T1, v);
         d.nb[i] = v;
         d.bath_at[i] = make_uint2(at, cnt);
       }
@@ -3096,7 +3113,7 @@ static int dalloc(dpsnn_engine *e, T **p, size_t n, bool temp = false) {
 // a small network's build.
 __global__ void fix_clear_kernel(double *near) { near[threadIdx.x] = INFINITY; }
 __global__ void fix_table_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint32_t n,
-                                 uint32_t *bitmap, double *near, uint32_t *err) {
+                                 uint32_t *bitmap, double *near, uint32_t *other) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t key = keys[i];
@@ -3106,12 +3123,11 @@ __global__ void fix_table_kernel(const uint32_t *__restrict__ keys, const uint32
   const double y = log((double)x);
   const float f = logf_cr_from(x, y);
   const uint32_t fb = __float_as_uint(f), E = (fb >> 23) & 0xFFu;
-  // bath_lapse takes a fix-up to be the float on the other side of the
-  // midpoint, as it is for any log with an error below one ulp
-  if (vals[i] != fb + (y < (double)f ? 1u : 0xFFFFFFFFu)) atomicMax(err, key);
+  // a fix-up that is not the float on the other side of the midpoint
+  if (vals[i] != fb + (y < (double)f ? 1u : 0xFFFFFFFFu)) *other = 1;
   if ((fb & 0x7FFFFFu) == 0) return;   // always looked up
-  const double dist = fabs(y - (double)f) - ldexp(1e-3, (int)E - 150);
-  atomicMin((unsigned long long *)&near[E], (unsigned long long)__double_as_longlong(dist));   // positive doubles
+  const double dist = fmax(fabs(y - (double)f) - ldexp(1e-3, (int)E - 150), 0.0);
+  atomicMin((unsigned long long *)&near[E], (unsigned long long)__double_as_longlong(dist));   // no negative doubles
 }
 
 static int load_logf_fixup(dpsnn_engine *e) {
@@ -3129,19 +3145,19 @@ static int load_logf_fixup(dpsnn_engine *e) {
   if (!ok) return dpsnn_fail(DPSNN_E_PARAM, "truncated %s", path.c_str());
   {
     const size_t words = ((size_t)(0x3F800000u - 0x30000000u) + 1 + 31) / 32;
-    uint32_t *dbm, *dkeys, *dvals, *derr, herr = 0;
+    uint32_t *dbm, *dkeys, *dvals, *dother, other = 0;
     double *dnear;
     DALLOC(dbm, words);
     DALLOC(dnear, 256);
     TALLOC(dkeys, n);
     TALLOC(dvals, n);
-    TALLOC(derr, 1);
+    TALLOC(dother, 1);
     CK(cudaMemcpyAsync(dkeys, keys.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
     CK(cudaMemcpyAsync(dvals, vals.data(), 4ull * n, cudaMemcpyHostToDevice, e->stream));
     fix_clear_kernel<<<1, 256, 0, e->stream>>>(dnear);
-    fix_table_kernel<<<(n + 255) / 256 + 1, 256, 0, e->stream>>>(dkeys, dvals, n, dbm, dnear, derr);
+    fix_table_kernel<<<(n + 255) / 256 + 1, 256, 0, e->stream>>>(dkeys, dvals, n, dbm, dnear, dother);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, e->stream));
+    CK(cudaMemcpyAsync(&other, dother, 4, cudaMemcpyDeviceToHost, e->stream));
     std::vector<double2> tab(LOG_TAB_N);
     for (int k = 0; k < LOG_TAB_N; k++) {   // the logarithm that goes with the rounded 64/i
       const double c = 64.0 / (LOG_TAB_0 + k);
@@ -3151,8 +3167,18 @@ static int load_logf_fixup(dpsnn_engine *e) {
     DALLOC(dtab, LOG_TAB_N);
     CK(cudaMemcpyAsync(dtab, tab.data(), sizeof(double2) * LOG_TAB_N, cudaMemcpyHostToDevice, e->stream));
     CK(cudaStreamSynchronize(e->stream));
-    if (herr)
-      return dpsnn_fail(DPSNN_E_PARAM, "%s: logf is off by more than one ulp at 0x%08x", path.c_str(), herr);
+    if (other) {   // the table's values are searched: it stays on the device
+      uint32_t *k, *v;
+      DALLOC(k, n);
+      DALLOC(v, n);
+      CK(cudaMemcpyAsync(k, dkeys, 4ull * n, cudaMemcpyDeviceToDevice, e->stream));
+      CK(cudaMemcpyAsync(v, dvals, 4ull * n, cudaMemcpyDeviceToDevice, e->stream));
+      e->hnet.fix_keys = k;
+      e->hnet.fix_vals = v;
+      e->hnet.fix_n = n;
+      CK(cudaMemcpyAsync(e->d.net, &e->hnet, sizeof e->hnet, cudaMemcpyHostToDevice, e->stream));
+      CK(cudaStreamSynchronize(e->stream));
+    }
     e->d.fix_bitmap = dbm;
     e->d.fix_near = dnear;
     e->d.log_tab = dtab;
@@ -3224,12 +3250,13 @@ static int set_kernel_attributes(int device) {
   CK(cudaFuncSetAttribute(gen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GEN_SMEM));
   CK(cudaFuncSetAttribute(gen_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)(GEN_FILL_WARPS * sizeof(GenFillWarp))));
-  CK(cudaFuncSetAttribute(bath_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BathSmem)));
   // the bath's blocks stay resident for most of a step: with the largest
   // shared-memory carveout, the SMs that hold two of them still have room for
   // a block of the main stream's kernels that use shared memory
-  CK(cudaFuncSetAttribute(bath_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                          (int)cudaSharedmemCarveoutMaxShared));
+  for (auto bath : {bath_kernel<false>, bath_kernel<true>}) {
+    CK(cudaFuncSetAttribute(bath, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BathSmem)));
+    CK(cudaFuncSetAttribute(bath, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  }
   done[device] = 1;
   return 0;
 }
@@ -3970,7 +3997,7 @@ static void enqueue_bath(dpsnn_engine *e, uint32_t t) {
   cudaStreamWaitEvent(e->bath_stream, e->ev_neuron[b], 0);
   timed_launch_begin(e, 2, e->bath_stream);
   // each rank's block keeps its step in d.bath_t (baths are launched in step order)
-  bath_kernel<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
+  (e->hnet.fix_n ? bath_kernel<true> : bath_kernel<false>)<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
   e->launches++;
   timed_launch_end(e, 2);
   cudaEventRecord(e->ev_bath[b], e->bath_stream);

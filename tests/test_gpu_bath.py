@@ -1,6 +1,8 @@
 """The Poisson bath kernel at the sizes and rates where its rounds, segments
 and caps have edges, against the CPU restatement: nextBath (the sum of every
 lapse drawn) and the raster must be the same bits."""
+import os
+
 import numpy as np
 import pytest
 
@@ -91,3 +93,35 @@ def test_events_hold_what_a_step_needs():
 
     (low, low_caps), (high, high_caps) = held(0.5), held(5.0)
     assert high - low < 2 * 9 * (high_caps - low_caps)
+
+
+def fixup_table():
+    raw = np.fromfile(os.path.join(E.HERE, "logf_fixup.bin"), np.uint32)
+    return raw[1:1 + raw[0]], raw[1 + raw[0]:1 + 2 * raw[0]]
+
+
+# a table may hold any value: one that is not a neighbouring float (here of an
+# input below 1e-9, which no draw makes) has the kernel search the table, with
+# the same results; values moved by three floats are the ones that it uses
+@pytest.mark.parametrize("moved", [False, True])
+def test_fixup_table_of_another_library(moved, tmp_path, monkeypatch):
+    keys, vals = fixup_table()
+    vals = vals + np.uint32(3) if moved else vals
+    first = np.array([0x30000001], np.uint32)
+    path = tmp_path / "logf_fixup.bin"
+    np.concatenate([np.array([len(keys) + 1], np.uint32), first, keys, np.array([0xC1A00000], np.uint32),
+                    vals]).tofile(path)
+    monkeypatch.setenv("DPSNN_LOGF_FIXUP", str(path))
+    cfg = nc.cortical_grid(2, 2, n_exc_a=130, n_exc_b=130, n_inh=41, p1=0.02, p_intra=0.02, mu=0.001, nu_ext_hz=3.0,
+                           total_ms=60, seed=5)
+    eng, orc = E.Engine(cfg), O.OracleNet(cfg, 1)
+    eng.step(60)
+    for _ in range(60):
+        orc.step()
+    got, want = eng.state()["nb"], orc.state()["nb"]
+    eng.close()
+    if moved:
+        assert np.any(got != want)
+        np.testing.assert_allclose(got, want, rtol=1e-7)   # three floats of a few lapses
+    else:
+        np.testing.assert_array_equal(got, want)
