@@ -1665,6 +1665,10 @@ __device__ static inline void bath_compose(const Dev &d, BathSmem &s, const Bath
   if (lane == 0) {
     nxt.sb_a = cur.a;
     nxt.sb_n = a - cur.a;
+    if (cur.out + m > s.slots) {   // pairs and events have the same count: no room for this round's
+      atomicOr(d.flags, F_BATH_DRAWS);
+      nxt.sb_n = 0;
+    }
     nxt.slow = slow;
     nxt.a = a;
     nxt.rebase = rebase;
@@ -1874,10 +1878,6 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
           const uint32_t word = jj < 8 ? pk.x : pk.y, sh = 4 * (jj & 7);
           m0 = s.e_start[par][g] + jj + nibble_sum(word & ((1u << sh) - 1)) + (jj < 8 ? 0u : nibble_sum(pk.x));
           cnt = ((word >> sh) & 15u) + 1;
-        }
-        if (cur.out + m0 + cnt > s.slots) {
-          atomicOr(d.flags, F_BATH_DRAWS);
-          continue;
         }
         const uint32_t id = s.a_id[a], i = i0 + (id & ((1u << 25) - 1)), at = ev_base + cur.out + m0;
         const double *lut = d.lut + 256 * (id >> 25);
@@ -3498,9 +3498,11 @@ static int generate_by_threads(dpsnn_engine *e, const std::vector<float> &prob, 
 // A rank's bath event slots.  A neuron has 1/invNuExt events per step on
 // average, Poisson distributed, one more at step 0 (nextBath = 0), and at most
 // its cap, 20 times the mean.  The rank's mean and 32 deviations (passed with a
-// probability below 1e-100; the emitters check), and no more than its caps: an
-// event takes 16 bytes, in two buffers, and all the caps of the 24x24 network
-// 1.1 GB.
+// probability below 1e-100; checked once a round), no more than its caps, and a
+// quarter of them at least: an event takes 16 bytes, in two buffers, and all the
+// caps of the 24x24 network 1.1 GB, a quarter 0.3.  The ranks' rows closer
+// together are slower by where they lie (a quiet 24x24 step 217 us, 213 with a
+// quarter, 215 with all).
 static uint64_t bath_slots(const uint32_t *max_ext, const double *inv_nu, uint32_t neurons) {
   uint64_t caps = 0;
   double mean = 0;
@@ -3509,7 +3511,7 @@ static uint64_t bath_slots(const uint32_t *max_ext, const double *inv_nu, uint32
     caps += max_ext[i];
     mean += std::min((double)max_ext[i], 1.0 + 1.0 / inv_nu[i]);
   }
-  return std::min(caps, (uint64_t)(mean + 32.0 * sqrt(mean)) + 64);
+  return std::min(caps, std::max(caps / 4, (uint64_t)(mean + 32.0 * sqrt(mean)) + 64));
 }
 
 static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_options *o) {

@@ -120,7 +120,7 @@ def estimate_device_bytes(cfg: nc.NetConfig, events_per_neuron: int = 1024) -> i
             caps += p.count * math.ceil(20 * rate)
             mean += p.count * min(math.ceil(20 * rate), 1 + rate)
     per_rank = cfg.n_modules // cfg.glob_h
-    slots = min(per_rank * caps, per_rank * mean + 32 * math.sqrt(per_rank * mean) + 64)
+    slots = min(per_rank * caps, max(per_rank * caps / 4, per_rank * mean + 32 * math.sqrt(per_rank * mean) + 64))
     per_neuron = 66 + 2 * (cfg.D + 1) + 8 + 80 * 12 + 8 * cap + 20 + 12 + 2 * 8 + 4
     per_syn = 6 + (12 if cfg.stdp is not None else 0)
     fixed = (116 << 20) + cfg.glob_h * (1_100 + 8 * cfg.D)
