@@ -103,7 +103,7 @@ struct NetConst {
   uint32_t light_max;   // neurons with more synaptic events take the heavy path
   uint32_t delay_exp;  // getRandomDelay_EXP instead of _UNI
   float inv_log_tn;    // (float)(1.0 / log(0.05)), the EXP tail constant
-  const uint32_t *fix_keys, *fix_vals;   // the logf fix-up table, where bath_kernel<true> searches it
+  const uint32_t *fix_keys, *fix_vals;   // the logf fix-up table, where the bath searches it
   uint32_t fix_n;
 };
 
@@ -1535,7 +1535,9 @@ __device__ static inline uint32_t bath_singles(const Dev &d, const BathSmem &s, 
 
 // One neuron of a mapper's segment from its lane's candidate (pair p, whose
 // q is qm): 1 + the number of sums of 1..16 lapses below lo, by fours, then
-// within the four.  Returns the count less one.
+// within the four.  Returns the count less one.  LOW: a neuron's cap may be below
+// sixteen.
+template <bool LOW>
 __device__ __forceinline__ uint32_t bath_count(const BathSmem &s, const uint4 &k, uint32_t &p, uint32_t &qm,
                                                uint32_t &bad) {
   const uint32_t T = qm + k.x;
@@ -1548,13 +1550,15 @@ __device__ __forceinline__ uint32_t bath_count(const BathSmem &s, const uint4 &k
   // undecided, in bad's top bit: the sum lies between lo and hi, none of the
   // sixteen reaches lo (over is then a negative number), or the count is past
   // the neuron's cap (k.z)
-  bad |= (over - k.y) | ~(c - k.z);
+  bad |= over - k.y;
+  if (LOW) bad |= ~(c - k.z);
   qm = T + over;
   p = e + 1;
   return c;
 }
 
 // Mapper w: its segment's end and counts from every candidate start.
+template <bool LOW>
 __device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t w, uint32_t lane) {
   const uint32_t A = BATH_ACT - 1, a0 = cur.a + BATH_SEG * w;
   if (a0 >= cur.act_end || cur.rebase) return;
@@ -1575,13 +1579,13 @@ __device__ static inline void bath_map(BathSmem &s, const BathCtl &cur, uint32_t
   const uint4 *k = &s.a_b[a0 & A];   // mirrored past the ring's end
   if (n == BATH_SEG) {
 #pragma unroll
-    for (int j = 0; j < 8; j++) pk.x += bath_count(s, k[j], p, qm, bad) << (4 * j);
+    for (int j = 0; j < 8; j++) pk.x += bath_count<LOW>(s, k[j], p, qm, bad) << (4 * j);
 #pragma unroll
-    for (int j = 0; j < 8; j++) pk.y += bath_count(s, k[8 + j], p, qm, bad) << (4 * j);
+    for (int j = 0; j < 8; j++) pk.y += bath_count<LOW>(s, k[8 + j], p, qm, bad) << (4 * j);
   } else {
 #pragma unroll 1
     for (uint32_t j = 0; j < n; j++) {
-      const uint32_t c = bath_count(s, k[j], p, qm, bad) << (4 * (j & 7));
+      const uint32_t c = bath_count<LOW>(s, k[j], p, qm, bad) << (4 * (j & 7));
       if (j < 8) pk.x += c; else pk.y += c;
     }
   }
@@ -1691,7 +1695,10 @@ __device__ static inline uint32_t nibble_sum(uint32_t x) {
   return (((x & 0x0F0F0F0Fu) + ((x >> 4) & 0x0F0F0F0Fu)) * 0x01010101u) >> 24;
 }
 
-template <bool SEARCH>
+// SEARCH: the logf table has values to search for (bath_lapse).  LOW: a neuron's
+// cap is below sixteen (rates below 0.75); the comparison that goes with it makes
+// 24x24 steps of 6 events per neuron 1.2 % longer, so that others go without.
+template <bool SEARCH, bool LOW>
 __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
   extern __shared__ __align__(16) unsigned char bath_smem_raw[];
   BathSmem &s = *reinterpret_cast<BathSmem *>(bath_smem_raw);
@@ -1738,7 +1745,7 @@ __global__ void __launch_bounds__(BATH_THREADS, 2) bath_kernel(Dev d) {
     BathCtl &nxt = s.ctl[(r + 1) & 1];
     if (cur.done || r == max_rounds) break;
     if (warp < BATH_SEGS) {
-      bath_map(s, cur, warp, lane);
+      bath_map<LOW>(s, cur, warp, lane);
       asm volatile("bar.sync 1, 256;" ::: "memory");   // the mappers
       bath_compose<SEARCH>(d, s, cur, nxt, r & 1, T1, warp, lane);
     } else if (warp == 15) {
@@ -3002,6 +3009,7 @@ struct dpsnn_engine {
   uint2 *bath_at2[2] = {nullptr, nullptr};
   int device = 0;
   uint64_t S = 0;
+  bool low_caps = false;   // some neuron's maxExternCurrentCount is below 16 (bath_kernel)
   uint32_t t_host = 0;   // steps enqueued
   uint32_t probe_t = UINT32_MAX;   // step of the last LTP probe taken
   uint32_t stdp_log_t = UINT32_MAX;   // step the STDP event log holds
@@ -3237,6 +3245,9 @@ static void h_gaussian_lut(double mu, double sigma, double xmin, double xmax, do
   }
 }
 
+static void (*const BATH_KERNELS[4])(Dev) = {bath_kernel<false, false>, bath_kernel<false, true>,
+                                             bath_kernel<true, false>, bath_kernel<true, true>};
+
 // The kernels' shared-memory attributes, set once per device and process,
 // before the device's first build: setting an attribute waits for the
 // kernel's running instances, which would serialise the builds of engines
@@ -3253,7 +3264,7 @@ static int set_kernel_attributes(int device) {
   // the bath's blocks stay resident for most of a step: with the largest
   // shared-memory carveout, the SMs that hold two of them still have room for
   // a block of the main stream's kernels that use shared memory
-  for (auto bath : {bath_kernel<false>, bath_kernel<true>}) {
+  for (auto bath : BATH_KERNELS) {
     CK(cudaFuncSetAttribute(bath, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BathSmem)));
     CK(cudaFuncSetAttribute(bath, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
   }
@@ -3760,7 +3771,10 @@ static int engine_build(dpsnn_engine *e, const dpsnn_params *p, const dpsnn_opti
     for (uint32_t h = 0; h < P; h++)
       base[h + 1] = base[h] + bath_slots(&mx[(size_t)h * n.locN], &inv[(size_t)h * n.locN], n.locN);
     uint32_t mx_max = 0;
-    for (uint32_t i = 0; i < N; i++) mx_max = std::max(mx_max, mx[i]);
+    for (uint32_t i = 0; i < N; i++) {
+      mx_max = std::max(mx_max, mx[i]);
+      e->low_caps |= inv[i] > 0 && mx[i] < 16;
+    }
     if (mx_max > BATH_MAX_EXT)
       return dpsnn_fail(DPSNN_E_CAPACITY, "maxExternCurrentCount %u exceeds what the bath ring holds (%d)", mx_max,
                         BATH_MAX_EXT);
@@ -3999,7 +4013,8 @@ static void enqueue_bath(dpsnn_engine *e, uint32_t t) {
   cudaStreamWaitEvent(e->bath_stream, e->ev_neuron[b], 0);
   timed_launch_begin(e, 2, e->bath_stream);
   // each rank's block keeps its step in d.bath_t (baths are launched in step order)
-  (e->hnet.fix_n ? bath_kernel<true> : bath_kernel<false>)<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
+  const auto kernel = BATH_KERNELS[2 * (e->hnet.fix_n != 0) + e->low_caps];
+  kernel<<<e->hnet.P, BATH_THREADS, sizeof(BathSmem), e->bath_stream>>>(db);
   e->launches++;
   timed_launch_end(e, 2);
   cudaEventRecord(e->ev_bath[b], e->bath_stream);
