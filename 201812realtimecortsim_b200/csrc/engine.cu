@@ -1331,7 +1331,7 @@ __global__ void __launch_bounds__(DELIVER_THREADS) deliver_small_kernel(Dev d) {
 // neuron's maxExternCurrentCount cap are single; after one the pairs start
 // afresh at the new position), so only every other draw becomes a lapse.
 // What bounds it: the latency of a round (a mapper's 16 dependent steps, then
-// the chain), not issue slots (a third used).  Segments of 16: a round costs
+// the chain), not issue slots (less than half used).  Segments of 16: a round costs
 // about 3000 cycles beside its steps, and at more neurons per segment the last
 // windows miss too often.  Measured per step (one B200), against the form
 // before, in which ten warps built tables of 64 candidate starts for every
@@ -2136,9 +2136,9 @@ __device__ static inline uint32_t warp_path_max(const NetConst *net);
 // coalesced, and each thread reads its own from there.  A warp that spans two
 // ranks, or whose neurons have more than NEURON_STAGE events, reads global
 // memory.  What bounds it: the latency of a warp's chain, events one after
-// another in 16 lanes of 32 on average (at 24x24, 720 000 neurons without
-// synaptic events: 80 us alone, DRAM at 7 %, an instruction every 4 cycles
-// per scheduler).  A step of 24x24 takes 228 us with the staged pairs and
+// another in 16 lanes of 32 on average (720 000 neurons without synaptic
+// events: 80 us alone; 180 000: 32 us, DRAM at 6.5 %, an instruction every 5
+// cycles per scheduler).  A step of 24x24 takes 228 us with the staged pairs and
 // div_by against 239 with three dependent loads per event and two divisions.
 #define NEURON_STAGE 192
 

@@ -142,9 +142,9 @@ void dpsnn_graph_destroy(dpsnn_graph *g);
 /* Grid sizes (blocks) of the delivery, warp-sort and heavy-run kernels; 0
  * restores the default (8, 8 and 16 blocks per SM, sized for a network that
  * fills the GPU; the delivery of a smaller one a block per 32 neurons; a
- * network of up to 32768 neurons has no separate sort and run kernels).  Every kernel loops over its work, so the results do not
- * depend on them; a small network stepped beside others runs faster on
- * smaller grids.  Takes effect for steps queued (or graphs recorded) after
+ * network of up to 32768 neurons has no separate sort and run kernels).
+ * Every kernel loops over its work, so the results do not depend on them; a
+ * small network stepped beside others runs faster on smaller grids.  Takes effect for steps queued (or graphs recorded) after
  * the call.  No counterpart in the reference. */
 int dpsnn_set_launch_shape(dpsnn_engine *e, uint32_t deliver_blocks, uint32_t heavy_sort_blocks,
                            uint32_t heavy_run_blocks);
